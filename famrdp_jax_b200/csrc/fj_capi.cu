@@ -253,14 +253,29 @@ int step_body(fj_ctx* ctx, const fj_block* blocks, double* const* q0p, double* c
   int s;
   const bool persist = ctx->pipeline == FJ_PIPELINE_SPLIT && o.persist && p->precision == FJ_PREC_F32FLUX && kmet;
   const bool fused_fill = ctx->pipeline == FJ_PIPELINE_SPLIT && o.fill && p->precision == FJ_PREC_F32FLUX && kmet;
-  // the copy and the halo fill as one kernel where the step is not in place
-  // (its sources are then the untouched input states); the persistent and
-  // fused-fill paths fill the halo themselves
+  // the copy, the halo fill and the stage-1 primitives as one kernel where the
+  // step is not in place (its sources are then the untouched input states);
+  // the persistent and fused-fill paths fill the halo themselves
+  const bool split_run = ctx->pipeline == FJ_PIPELINE_SPLIT && !persist &&
+                         !(o.tile && p->precision == FJ_PREC_F32FLUX && kmet);
+  std::vector<SplitBlock> sb;
+  if (split_run) {
+    sb.resize(nblocks);
+    for (int b = 0; b < nblocks; ++b) {
+      const fj_block& B = out[b];
+      sb[b] = split_block(q0p[b], q0p[b], q1s[b], B.kxyz, kmet ? kmet[b] : nullptr, B.vol, B.ni, B.nj, B.nk,
+                          mu0_b ? mu0_b[b] : p->mu0, dt_b ? dt_b[b] : dt);
+    }
+    split_assign_scratch(p->precision, sb.data(), nblocks, tail);
+  }
+  std::vector<void*> prim(sb.size());
+  for (size_t b = 0; b < sb.size(); ++b) prim[b] = sb[b].prim;
+  const PrimsOut prims{p->precision, prim.data(), p->gamma - 1.0, p->R, kmet ? o.p_ref : 0.0};
   bool filled = false;
   bool apart = nlinks > 0 && !persist && !fused_fill;
   for (int b = 0; b < nblocks && apart; ++b) apart = q0p[b] != blocks[b].q;
   if (apart) {
-    s = copy_fill(ctx, blocks, q0p, nblocks, links, nlinks, p->ghost, st, &filled);
+    s = copy_fill(ctx, blocks, q0p, nblocks, links, nlinks, p->ghost, st, &filled, split_run ? &prims : nullptr);
     if (s != FJ_OK) return s;
   }
   for (int b = 0; b < nblocks; ++b) out[b].q = q0p[b];
@@ -294,22 +309,14 @@ int step_body(fj_ctx* ctx, const fj_block* blocks, double* const* q0p, double* c
       s = halo_exchange(ctx, out.data(), nblocks, links, nlinks, p->ghost, (double*)tail, tail_b, st);
       if (s != FJ_OK) return s;
     }
-    s = apply_bc(ctx, out.data(), nblocks, bcs, nbcs, p, st);
+    s = apply_bc(ctx, out.data(), nblocks, bcs, nbcs, p, st, filled && split_run ? &prims : nullptr);
   }
   if (s != FJ_OK) return s;
   const int flags = kRhsInvscd | kRhsViscous;
   if (ctx->pipeline == FJ_PIPELINE_SPLIT && o.tile && p->precision == FJ_PREC_F32FLUX && kmet)
     return tile_step(ctx, out, q1s, q2s, q_out, p, dt, kmet, st, o);
-  if (ctx->pipeline == FJ_PIPELINE_SPLIT) {
+  if (split_run) {
     // all blocks per launch; the tail holds the intermediates of every block
-    std::vector<SplitBlock> sb(nblocks);
-    for (int b = 0; b < nblocks; ++b) {
-      const fj_block& B = out[b];
-      sb[b] = split_block(B.q, B.q, q1s[b], B.kxyz,
-                          kmet ? kmet[b] : nullptr, B.vol, B.ni,
-                          B.nj, B.nk, mu0_b ? mu0_b[b] : p->mu0, dt_b ? dt_b[b] : dt);
-    }
-    split_assign_scratch(p->precision, sb.data(), nblocks, tail);
     Phys ph = make_phys(p);
     ph.p_ref = o.p_ref;
     // the blocks of each stream group; one group unless two streams are set up
@@ -343,8 +350,9 @@ int step_body(fj_ctx* ctx, const fj_block* blocks, double* const* q0p, double* c
       }
       if (v.empty()) return FJ_OK;
       // the assembly of stages 1 and 2 also writes the next stage's primitives
-      // (the fused ghost fill writes stage 1's)
-      return split_stage(ctx, v.data(), (int)v.size(), ph, flags, stage, p->precision, gs, stage > 1 || fused_fill,
+      // (the fill of the start state writes stage 1's)
+      return split_stage(ctx, v.data(), (int)v.size(), ph, flags, stage, p->precision, gs,
+                         stage > 1 || fused_fill || filled,
                          stage < 3, variant, after_fluxes);
     };
     if (two) {

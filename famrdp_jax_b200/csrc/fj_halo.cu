@@ -30,6 +30,7 @@
 #include "fj_common.cuh"
 #include "fj_halo_dev.cuh"
 #include "fj_rhs.cuh"
+#include "fj_split_dev.cuh"
 
 namespace fj {
 
@@ -47,9 +48,18 @@ struct HaloTable {
 
 struct BcTable {
   int n;
-  double gamma, R;
+  double gamma, R, p_ref;
   BcDesc d[kMaxBcPerLaunch];
+  void* prim[kMaxBcPerLaunch];  // the face's block's primitive records (k_bc<4>, <8>)
 };
+
+// Primitive records of conserved values q: PR = bytes of a record's values (4:
+// FP32, 8: FP64, 0: none).
+template <int PR>
+__device__ __forceinline__ void put_prims(void* prim, size_t c, const double q[5], double gm1, double R, double p_ref) {
+  if constexpr (PR == 4) sd::store_prim_record<float>(prim, c, q, gm1, R, 1.0 / R, p_ref);
+  if constexpr (PR == 8) sd::store_prim_record<double>(prim, c, q, gm1, R, 1.0 / R, p_ref);
+}
 
 __global__ void k_halo_gather(const HaloTable tab, double* __restrict__ scratch) {
   grid_dep_wait();
@@ -86,6 +96,7 @@ __global__ void k_halo_scatter(const HaloTable tab, const double* __restrict__ s
   }
 }
 
+template <int PR>
 __global__ void k_bc(const BcTable tab, int g) {
   grid_dep_wait();
   const BcDesc& d = tab.d[blockIdx.y];
@@ -98,6 +109,15 @@ __global__ void k_bc(const BcTable tab, int g) {
     const int x = (int)((r / d.n[ob]) % d.n[oa]);
     const int o = (int)(r / ((int64_t)d.n[ob] * d.n[oa]));
     bc_cell(d, d.q, ax, oa, ob, o, x, y, g, tab.gamma, tab.R);
+    if constexpr (PR != 0) {
+      int at[3], inner;
+      bc_layers(d.face, d.n[ax], g, o, at[ax], inner);
+      at[oa] = x;
+      at[ob] = y;
+      const int64_t c = cell_index(d.n, at[0], at[1], at[2]), N = (int64_t)d.n[0] * d.n[1] * d.n[2];
+      const double q[5] = {d.q[c], d.q[N + c], d.q[2 * N + c], d.q[3 * N + c], d.q[4 * N + c]};
+      put_prims<PR>(tab.prim[blockIdx.y], (size_t)c, q, tab.gamma - 1.0, tab.R, tab.p_ref);
+    }
   }
 }
 
@@ -297,59 +317,83 @@ namespace {
 // Block b owns the CTAs [cta_begin[b], cta_begin[b+1]), `cells` cells each
 // (CTAs in proportion to the block's cells): one per thread for tables that
 // would not give every SM 16 CTAs so (their time is the per-thread latency),
-// else four.
-constexpr int kMaxFillBlocks = 64;
+// else kFillCells.
+constexpr int kMaxFillBlocks = 64, kFillCells = 4;
 struct CopyFillTable {
   int nb, ghost, cells;
+  double gm1, R, p_ref;
   const double* src[kMaxFillBlocks];
   double* dst[kMaxFillBlocks];
+  void* prim[kMaxFillBlocks];
   int n[kMaxFillBlocks][3];
+  sd::FastDiv dk[kMaxFillBlocks], dj[kMaxFillBlocks];
   int cta_begin[kMaxFillBlocks + 1];
   short first[kMaxFillBlocks], count[kMaxFillBlocks];
   short order[kMaxLinksPerLaunch];
 };
-static_assert(sizeof(HaloTable) + sizeof(CopyFillTable) <= 32000, "kernel parameter space");
+static_assert(sizeof(HaloTable) + sizeof(CopyFillTable) <= 32764, "kernel parameter space");
 
 // dst[b] := src[b] cell by cell, except the ghost cells a link of block b
 // covers: those take the source cell of the LAST such link (list order), read
 // from the source block's src, i.e. from the pre-exchange states (src is
 // never written here).  The same values as a copy followed by the gather and
-// the ordered scatter.
-__global__ void k_copy_fill(const HaloTable tab, const CopyFillTable ct) {
+// the ordered scatter.  With PR, the cells' primitive records too, from the
+// values in registers (a separate kernel read the 40 bytes a cell again).
+// Bound by memory: a thread's U cells are all loaded before the first store.
+// 4.0 M cells: 70 us with FP32 records, 86 us with FP64 ones (4.9 TB/s); the copy
+// alone took 77 us cell by cell and the primitive kernel after it 40 and 59 us.
+template <int PR, int U>
+__global__ void __launch_bounds__(kThreads) k_copy_fill(const HaloTable tab, const CopyFillTable ct) {
   grid_dep_wait();
-  int b = 0;
-  while (b + 1 < ct.nb && ct.cta_begin[b + 1] <= (int)blockIdx.x) ++b;
+  int b = 0, hi = ct.nb - 1;
+  while (b < hi) {
+    const int mid = (b + hi + 1) >> 1;
+    if (ct.cta_begin[mid] <= (int)blockIdx.x) b = mid;
+    else hi = mid - 1;
+  }
   const int ni = ct.n[b][0], nj = ct.n[b][1], nk = ct.n[b][2], g = ct.ghost;
   const uint32_t N = (uint32_t)ni * nj * nk;  // < 2^31, checked on the host
   const double* __restrict__ s = ct.src[b];
   double* __restrict__ d = ct.dst[b];
   const int e0 = ct.first[b], e1 = ct.first[b] + ct.count[b];
-  const uint32_t c0 = (uint32_t)(blockIdx.x - ct.cta_begin[b]) * (uint32_t)ct.cells;
-  for (uint32_t c = c0 + threadIdx.x; c < N && c < c0 + (uint32_t)ct.cells; c += kThreads) {
-    const uint32_t t = c / (uint32_t)nk;
+  const uint32_t c0 = (uint32_t)(blockIdx.x - ct.cta_begin[b]) * (uint32_t)ct.cells + threadIdx.x;
+  double q[U][5];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const uint32_t c = c0 + u * kThreads;
+    if (c >= N) break;
+    const uint32_t t = ct.dk[b].div(c);
     const int k = (int)(c - t * (uint32_t)nk);
-    const int i = (int)(t / (uint32_t)nj), j = (int)(t - (uint32_t)i * (uint32_t)nj);
-    int L = -1;
-    if (i < g || i >= ni - g || j < g || j >= nj - g || k < g || k >= nk - g)
+    const int i = (int)ct.dj[b].div(t), j = (int)(t - (uint32_t)i * (uint32_t)nj);
+    const double* from = s + c;
+    int64_t NS = N;
+    if (i < g || i >= ni - g || j < g || j >= nj - g || k < g || k >= nk - g) {
+      int L = -1;
       for (int e = e1 - 1; e >= e0 && L < 0; --e)
         if (slab_covers(tab.d[ct.order[e]], i, j, k)) L = ct.order[e];
-    if (L < 0) {
-#pragma unroll
-      for (int v = 0; v < 5; ++v) d[(size_t)v * N + c] = s[(size_t)v * N + c];
-    } else {
-      const HaloDesc& h = tab.d[L];
-      const int64_t NS = (int64_t)h.sn[0] * h.sn[1] * h.sn[2];
-      const int64_t si = h.s0 + (i - h.tlo[0]) * h.sstr[0] + (j - h.tlo[1]) * h.sstr[1] + (k - h.tlo[2]) * h.sstr[2];
-#pragma unroll
-      for (int v = 0; v < 5; ++v) d[(size_t)v * N + c] = h.src[v * NS + si];
+      if (L >= 0) {
+        const HaloDesc& h = tab.d[L];
+        NS = (int64_t)h.sn[0] * h.sn[1] * h.sn[2];
+        from = h.src + (h.s0 + (i - h.tlo[0]) * h.sstr[0] + (j - h.tlo[1]) * h.sstr[1] + (k - h.tlo[2]) * h.sstr[2]);
+      }
     }
+#pragma unroll
+    for (int v = 0; v < 5; ++v) q[u][v] = __ldg(from + v * NS);
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const uint32_t c = c0 + u * kThreads;
+    if (c >= N) break;
+#pragma unroll
+    for (int v = 0; v < 5; ++v) d[(size_t)v * N + c] = q[u][v];
+    put_prims<PR>(ct.prim[b], c, q[u], ct.gm1, ct.R, ct.p_ref);
   }
 }
 
 }  // namespace
 
 int copy_fill(fj_ctx* ctx, const fj_block* blocks, double* const* dst, int nblocks, const fj_link* links, int nlinks,
-              int ghost, cudaStream_t st, bool* done) {
+              int ghost, cudaStream_t st, bool* done, const PrimsOut* prims) {
   *done = false;
   if (nblocks > kMaxFillBlocks || nlinks > kMaxLinksPerLaunch) return FJ_OK;  // the separate copy and fill
   for (int b = 0; b < nblocks; ++b)
@@ -367,10 +411,17 @@ int copy_fill(fj_ctx* ctx, const fj_block* blocks, double* const* dst, int nbloc
   int pos = 0;
   int64_t ctas = 0, narrow = 0;
   for (int b = 0; b < nblocks; ++b) narrow += ((int64_t)blocks[b].ni * blocks[b].nj * blocks[b].nk + kThreads - 1) / kThreads;
-  ct.cells = narrow < 16 * 148 ? kThreads : 4 * kThreads;
+  const bool wide = narrow >= 16 * 148;
+  ct.cells = wide ? kFillCells * kThreads : kThreads;
+  ct.gm1 = prims ? prims->gm1 : 0.0;
+  ct.R = prims ? prims->R : 1.0;
+  ct.p_ref = prims ? prims->p_ref : 0.0;
   for (int b = 0; b < nblocks; ++b) {
     ct.src[b] = blocks[b].q;
     ct.dst[b] = dst[b];
+    ct.prim[b] = prims ? prims->prim[b] : nullptr;
+    ct.dk[b].init((uint32_t)blocks[b].nk);
+    ct.dj[b].init((uint32_t)blocks[b].nj);
     ct.n[b][0] = blocks[b].ni;
     ct.n[b][1] = blocks[b].nj;
     ct.n[b][2] = blocks[b].nk;
@@ -383,7 +434,11 @@ int copy_fill(fj_ctx* ctx, const fj_block* blocks, double* const* dst, int nbloc
   }
   ct.cta_begin[nblocks] = (int)ctas;
   if (ctas == 0) return FJ_OK;
-  pdl_launch(k_copy_fill, dim3((unsigned)ctas), kThreads, 0, st, tab, ct);
+  const int pr = !prims ? 0 : (prims->precision == FJ_PREC_F32FLUX ? 4 : 8);
+  auto kern = pr == 4   ? (wide ? k_copy_fill<4, kFillCells> : k_copy_fill<4, 1>)
+              : pr == 8 ? (wide ? k_copy_fill<8, kFillCells> : k_copy_fill<8, 1>)
+                        : (wide ? k_copy_fill<0, kFillCells> : k_copy_fill<0, 1>);
+  pdl_launch(kern, dim3((unsigned)ctas), kThreads, 0, st, tab, ct);
   ctx->launches += 1;
   s = launch_status(ctx, "copy-fill launch");
   if (s == FJ_OK) *done = true;
@@ -391,7 +446,7 @@ int copy_fill(fj_ctx* ctx, const fj_block* blocks, double* const* dst, int nbloc
 }
 
 int apply_bc(fj_ctx* ctx, const fj_block* blocks, int nblocks, const fj_bc* bcs, int nbcs,
-             const fj_params* p, cudaStream_t st) {
+             const fj_params* p, cudaStream_t st, const PrimsOut* prims) {
   for (int b = 0; b < nbcs; ++b) {
     const fj_bc& e = bcs[b];
     if (e.block < 0 || e.block >= nblocks)
@@ -403,10 +458,12 @@ int apply_bc(fj_ctx* ctx, const fj_block* blocks, int nblocks, const fj_bc* bcs,
   }
   for (int face = 0; face < 6; ++face) {
     std::vector<BcDesc> ds;
+    std::vector<void*> rec;
     for (int b = 0; b < nbcs; ++b) {
       const fj_bc& e = bcs[b];
       if (e.face != face) continue;
       const fj_block& blk = blocks[e.block];
+      rec.push_back(prims ? prims->prim[e.block] : nullptr);
       BcDesc d;
       d.q = blk.q;
       d.n[0] = blk.ni; d.n[1] = blk.nj; d.n[2] = blk.nk;
@@ -422,15 +479,18 @@ int apply_bc(fj_ctx* ctx, const fj_block* blocks, int nblocks, const fj_bc* bcs,
       tab.n = (int)std::min<size_t>(kMaxBcPerLaunch, ds.size() - base);
       tab.gamma = p->gamma;
       tab.R = p->R;
+      tab.p_ref = prims ? prims->p_ref : 0.0;
       int64_t vmax = 0;
       for (int t = 0; t < tab.n; ++t) {
         tab.d[t] = ds[base + t];
+        tab.prim[t] = rec[base + t];
         const int ax = face >> 1;
         int64_t area = (int64_t)tab.d[t].n[0] * tab.d[t].n[1] * tab.d[t].n[2] / tab.d[t].n[ax];
         vmax = std::max<int64_t>(vmax, area * p->ghost);
       }
       dim3 grid((unsigned)std::min<int64_t>(grid_for(vmax), 4096), tab.n);
-      pdl_launch(k_bc, grid, kThreads, 0, st, tab, p->ghost);
+      auto kern = !prims ? k_bc<0> : (prims->precision == FJ_PREC_F32FLUX ? k_bc<4> : k_bc<8>);
+      pdl_launch(kern, grid, kThreads, 0, st, tab, p->ghost);
       ctx->launches += 1;
       int s = launch_status(ctx, "bc launch");
       if (s != FJ_OK) return s;

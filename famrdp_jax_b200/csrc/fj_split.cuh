@@ -34,6 +34,7 @@ struct SplitBlock {
   void* Fk;              // FP32 only: the k face c | c+1 of each cell, 5 per cell (written and read only
                          // by the kernels of tables too small to fill the GPU; zero where no face exists)
   double mu0;            // viscosity scale of this block (per-instance ensembles)
+  float mu0_f;           // and in FP32
   double dt;             // time step of this block (stages 1..3)
   int ni, nj, nk;
   int cta_begin;         // filled by the launcher

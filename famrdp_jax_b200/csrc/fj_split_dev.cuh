@@ -85,6 +85,12 @@ struct TablePtrs {
   __device__ __forceinline__ void* prim_next() const { return B.prim_next; }
 };
 
+template <typename T>
+__device__ __forceinline__ T block_mu0(const SplitBlock& B) {
+  if constexpr (sizeof(T) == 4) return B.mu0_f;
+  else return B.mu0;
+}
+
 // Coordinates of cell c of block d; false past the block's end.
 __device__ __forceinline__ bool decode_cell(const Dev& d, int64_t c, Cell& x) {
   const SplitBlock& B = d.blk;
@@ -350,8 +356,8 @@ __device__ __forceinline__ void face_from_cells(const Cell6<T>& a0, const Cell6<
                                                 const Phys& ph, T* F, T p_ref) {
   Prim<T> cell[4] = {{a0.r, a0.u, a0.v, a0.w, a0.p}, {a1.r, a1.u, a1.v, a1.w, a1.p},
                      {a2.r, a2.u, a2.v, a2.w, a2.p}, {a3.r, a3.u, a3.v, a3.w, a3.p}};
-  invscd_face_fast<T, POFF>(cell, kl[0], kl[1], kl[2], kr[0], kr[1], kr[2], (T)ph.gm1, (T)ph.inv_gm1,
-                            (T)ph.eps_entropy, ph.limiter, F, p_ref);
+  invscd_face_fast<T, POFF>(cell, kl[0], kl[1], kl[2], kr[0], kr[1], kr[2], num<T>(ph).gm1, num<T>(ph).inv_gm1,
+                            num<T>(ph).eps_entropy, ph.limiter, F, p_ref);
 }
 
 // With next_prims, also writes the primitives of the stage result (the next
@@ -513,7 +519,7 @@ __device__ __forceinline__ void k_face_left(const SplitBlock& B, const void* pri
                  a3 = load_cell<T, NC>(P, c + 1);
   T kl[3];
   metric_row<T, K_AOS>(B, N, 2, c - 1, kl);
-  face_from_cells<T, K_AOS>(a0, a1, a2, a3, kl, kr, ph, F, K_AOS ? (T)ph.p_ref : T(0));
+  face_from_cells<T, K_AOS>(a0, a1, a2, a3, kl, kr, ph, F, K_AOS ? num<T>(ph).p_ref : T(0));
 }
 
 // Cells per assembly CTA: each warp assembles 31 consecutive cells; its 32nd
@@ -586,12 +592,12 @@ __device__ __forceinline__ void flux_cell(const SplitBlock& B, const void* prim,
     for (int s = 0; s < 4; ++s)
 #pragma unroll
       for (int m = 0; m < 3; ++m) g[s][m] = d[s][0] * kk[m] + d[s][1] * kk[3 + m] + d[s][2] * kk[6 + m];
-    T mu = (T)B.mu0;
+    T mu = block_mu0<T>(B);
     if (ph.visc_law == 0) {  // Sutherland (physics/eos.py:24-25)
-      const T r = C0.t * (T)ph.inv_T0;
-      mu = (T)B.mu0 * (r * M::sqrt_pos(r)) * (T)ph.sfac * M::rcp(C0.t + (T)ph.Ts);
+      const T r = C0.t * num<T>(ph).inv_T0;
+      mu = block_mu0<T>(B) * (r * M::sqrt_pos(r)) * num<T>(ph).sfac * M::rcp(C0.t + num<T>(ph).Ts);
     }
-    const T kappa = (T)ph.kap_fac * mu;
+    const T kappa = num<T>(ph).kap_fac * mu;
     const T third = (T)(1.0 / 3.0);
     const T div_u = g[0][0] + g[1][1] + g[2][2];
     const T t00 = T(2) * mu * (g[0][0] - div_u * third);
@@ -616,7 +622,7 @@ __device__ __forceinline__ void flux_cell(const SplitBlock& B, const void* prim,
     T kn[3];
     // with metric records the primitives carry p' = p - p_ref and the FP64
     // correction of the momentum fluxes is in the records
-    const T p_ref = K_AOS ? (T)ph.p_ref : T(0);
+    const T p_ref = K_AOS ? num<T>(ph).p_ref : T(0);
     if (x.i >= 1 && x.i <= x.ni - 3) {
       const Cell6<T> I2 = load_cell<T, NC>(P, c + 2 * si);
       metric_row<T, K_AOS>(B, N, 0, c + si, kn);
@@ -667,12 +673,12 @@ __device__ __forceinline__ void flux_visc_part(const SplitBlock& B, const void* 
   for (int s = 0; s < 4; ++s)
 #pragma unroll
     for (int m = 0; m < 3; ++m) g[s][m] = d[s][0] * kk[m] + d[s][1] * kk[3 + m] + d[s][2] * kk[6 + m];
-  T mu = (T)B.mu0;
+  T mu = block_mu0<T>(B);
   if (ph.visc_law == 0) {  // Sutherland (physics/eos.py:24-25)
-    const T r = C0.t * (T)ph.inv_T0;
-    mu = (T)B.mu0 * (r * M::sqrt_pos(r)) * (T)ph.sfac * M::rcp(C0.t + (T)ph.Ts);
+    const T r = C0.t * num<T>(ph).inv_T0;
+    mu = block_mu0<T>(B) * (r * M::sqrt_pos(r)) * num<T>(ph).sfac * M::rcp(C0.t + num<T>(ph).Ts);
   }
-  const T kappa = (T)ph.kap_fac * mu;
+  const T kappa = num<T>(ph).kap_fac * mu;
   const T third = (T)(1.0 / 3.0);
   const T div_u = g[0][0] + g[1][1] + g[2][2];
   const T t00 = T(2) * mu * (g[0][0] - div_u * third);
@@ -706,7 +712,7 @@ __device__ __forceinline__ void flux_face_part(const SplitBlock& B, const void* 
     T kc[3], kn[3];
     metric_row<T, K_AOS>(B, N, AXIS, c, kc);
     metric_row<T, K_AOS>(B, N, AXIS, c + sa, kn);
-    face_from_cells<T, K_AOS>(A0, A1, A2, A3, kc, kn, ph, F, K_AOS ? (T)ph.p_ref : T(0));
+    face_from_cells<T, K_AOS>(A0, A1, A2, A3, kc, kn, ph, F, K_AOS ? num<T>(ph).p_ref : T(0));
   }
   if (AXIS == 2) {
     T* fk = (T*)B.Fk + (size_t)c * 5;

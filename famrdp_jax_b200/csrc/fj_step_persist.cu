@@ -804,6 +804,7 @@ int persist_step(fj_ctx* ctx, const PersistPlan& pp, const fj_block* blocks, int
     e.kaos = kmet[b];
     e.vol = blocks[b].vol;
     e.mu0 = mu0_b ? mu0_b[b] : p->mu0;
+    e.mu0_f = (float)e.mu0;
     e.dt = dt_b ? dt_b[b] : dt;
     e.ni = blocks[b].ni;
     e.nj = blocks[b].nj;
@@ -824,7 +825,7 @@ int persist_step(fj_ctx* ctx, const PersistPlan& pp, const fj_block* blocks, int
     P.plane_base[b] = pp.plane_base[b];
   }
   P.ph = make_phys(p);
-  P.ph.p_ref = p_ref;
+  P.ph.set_p_ref(p_ref);
   P.gamma = p->gamma;
   P.gm1 = p->gamma - 1.0;
   P.R = p->R;

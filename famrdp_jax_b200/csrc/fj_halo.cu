@@ -41,10 +41,12 @@ constexpr int kMaxBcPerLaunch = 128;
 
 using namespace hd;
 
-struct HaloTable {
+template <int NL>
+struct HaloTableN {
   int n;
-  HaloDesc d[kMaxLinksPerLaunch];
+  HaloDesc d[NL];
 };
+using HaloTable = HaloTableN<kMaxLinksPerLaunch>;
 
 struct BcTable {
   int n;
@@ -319,18 +321,26 @@ namespace {
 // would not give every SM 16 CTAs so (their time is the per-thread latency),
 // else kFillCells.
 constexpr int kMaxFillBlocks = 64, kFillCells = 4;
-struct CopyFillTable {
+struct FillBlock {
+  const double* src;
+  double* dst;
+  void* prim;
+  int n[3];
+  sd::FastDiv dk, dj;
+  int cta_begin;
+  short first, count;
+};
+template <int NB, int NL>
+struct CopyFillTableN {
   int nb, ghost, cells;
   double gm1, R, p_ref;
-  const double* src[kMaxFillBlocks];
-  double* dst[kMaxFillBlocks];
-  void* prim[kMaxFillBlocks];
-  int n[kMaxFillBlocks][3];
-  sd::FastDiv dk[kMaxFillBlocks], dj[kMaxFillBlocks];
-  int cta_begin[kMaxFillBlocks + 1];
-  short first[kMaxFillBlocks], count[kMaxFillBlocks];
-  short order[kMaxLinksPerLaunch];
+  FillBlock b[NB];
+  short order[NL];
 };
+using CopyFillTable = CopyFillTableN<kMaxFillBlocks, kMaxLinksPerLaunch>;
+// one block with a link on each face at most: 0.9 KB of parameters instead of 26
+using HaloTable1 = HaloTableN<6>;
+using CopyFillTable1 = CopyFillTableN<1, 6>;
 static_assert(sizeof(HaloTable) + sizeof(CopyFillTable) <= 32764, "kernel parameter space");
 
 // dst[b] := src[b] cell by cell, except the ghost cells a link of block b
@@ -342,29 +352,33 @@ static_assert(sizeof(HaloTable) + sizeof(CopyFillTable) <= 32764, "kernel parame
 // Bound by memory: a thread's U cells are all loaded before the first store.
 // 4.0 M cells: 70 us with FP32 records, 86 us with FP64 ones (4.9 TB/s); the copy
 // alone took 77 us cell by cell and the primitive kernel after it 40 and 59 us.
-template <int PR, int U>
-__global__ void __launch_bounds__(kThreads) k_copy_fill(const HaloTable tab, const CopyFillTable ct) {
+template <int PR, int U, int NB, int NL>
+__global__ void __launch_bounds__(kThreads) k_copy_fill(const HaloTableN<NL> tab, const CopyFillTableN<NB, NL> ct) {
   grid_dep_wait();
-  int b = 0, hi = ct.nb - 1;
-  while (b < hi) {
-    const int mid = (b + hi + 1) >> 1;
-    if (ct.cta_begin[mid] <= (int)blockIdx.x) b = mid;
-    else hi = mid - 1;
+  int b = 0;
+  if constexpr (NB > 1) {
+    int hi = ct.nb - 1;
+    while (b < hi) {
+      const int mid = (b + hi + 1) >> 1;
+      if (ct.b[mid].cta_begin <= (int)blockIdx.x) b = mid;
+      else hi = mid - 1;
+    }
   }
-  const int ni = ct.n[b][0], nj = ct.n[b][1], nk = ct.n[b][2], g = ct.ghost;
+  const FillBlock& B = ct.b[b];
+  const int ni = B.n[0], nj = B.n[1], nk = B.n[2], g = ct.ghost;
   const uint32_t N = (uint32_t)ni * nj * nk;  // < 2^31, checked on the host
-  const double* __restrict__ s = ct.src[b];
-  double* __restrict__ d = ct.dst[b];
-  const int e0 = ct.first[b], e1 = ct.first[b] + ct.count[b];
-  const uint32_t c0 = (uint32_t)(blockIdx.x - ct.cta_begin[b]) * (uint32_t)ct.cells + threadIdx.x;
+  const double* __restrict__ s = B.src;
+  double* __restrict__ d = B.dst;
+  const int e0 = B.first, e1 = B.first + B.count;
+  const uint32_t c0 = (uint32_t)(blockIdx.x - B.cta_begin) * (uint32_t)ct.cells + threadIdx.x;
   double q[U][5];
 #pragma unroll
   for (int u = 0; u < U; ++u) {
     const uint32_t c = c0 + u * kThreads;
     if (c >= N) break;
-    const uint32_t t = ct.dk[b].div(c);
+    const uint32_t t = B.dk.div(c);
     const int k = (int)(c - t * (uint32_t)nk);
-    const int i = (int)ct.dj[b].div(t), j = (int)(t - (uint32_t)i * (uint32_t)nj);
+    const int i = (int)B.dj.div(t), j = (int)(t - (uint32_t)i * (uint32_t)nj);
     const double* from = s + c;
     int64_t NS = N;
     if (i < g || i >= ni - g || j < g || j >= nj - g || k < g || k >= nk - g) {
@@ -386,7 +400,7 @@ __global__ void __launch_bounds__(kThreads) k_copy_fill(const HaloTable tab, con
     if (c >= N) break;
 #pragma unroll
     for (int v = 0; v < 5; ++v) d[(size_t)v * N + c] = q[u][v];
-    put_prims<PR>(ct.prim[b], c, q[u], ct.gm1, ct.R, ct.p_ref);
+    put_prims<PR>(B.prim, c, q[u], ct.gm1, ct.R, ct.p_ref);
   }
 }
 
@@ -417,28 +431,43 @@ int copy_fill(fj_ctx* ctx, const fj_block* blocks, double* const* dst, int nbloc
   ct.R = prims ? prims->R : 1.0;
   ct.p_ref = prims ? prims->p_ref : 0.0;
   for (int b = 0; b < nblocks; ++b) {
-    ct.src[b] = blocks[b].q;
-    ct.dst[b] = dst[b];
-    ct.prim[b] = prims ? prims->prim[b] : nullptr;
-    ct.dk[b].init((uint32_t)blocks[b].nk);
-    ct.dj[b].init((uint32_t)blocks[b].nj);
-    ct.n[b][0] = blocks[b].ni;
-    ct.n[b][1] = blocks[b].nj;
-    ct.n[b][2] = blocks[b].nk;
-    ct.first[b] = (short)pos;
+    FillBlock& F = ct.b[b];
+    F.src = blocks[b].q;
+    F.dst = dst[b];
+    F.prim = prims ? prims->prim[b] : nullptr;
+    F.n[0] = blocks[b].ni;
+    F.n[1] = blocks[b].nj;
+    F.n[2] = blocks[b].nk;
+    F.dk.init((uint32_t)blocks[b].nk);
+    F.dj.init((uint32_t)blocks[b].nj);
+    F.first = (short)pos;
     for (int L = 0; L < tab.n; ++L)
       if (tab.d[L].tgt_block == b) ct.order[pos++] = (short)L;
-    ct.count[b] = (short)(pos - ct.first[b]);
-    ct.cta_begin[b] = (int)ctas;
+    F.count = (short)(pos - F.first);
+    F.cta_begin = (int)ctas;
     ctas += ((int64_t)blocks[b].ni * blocks[b].nj * blocks[b].nk + ct.cells - 1) / ct.cells;
   }
-  ct.cta_begin[nblocks] = (int)ctas;
   if (ctas == 0) return FJ_OK;
   const int pr = !prims ? 0 : (prims->precision == FJ_PREC_F32FLUX ? 4 : 8);
-  auto kern = pr == 4   ? (wide ? k_copy_fill<4, kFillCells> : k_copy_fill<4, 1>)
-              : pr == 8 ? (wide ? k_copy_fill<8, kFillCells> : k_copy_fill<8, 1>)
-                        : (wide ? k_copy_fill<0, kFillCells> : k_copy_fill<0, 1>);
-  pdl_launch(kern, dim3((unsigned)ctas), kThreads, 0, st, tab, ct);
+  auto launch = [&](auto nb, auto nl, const auto& ht, const auto& ft) {
+    constexpr int NB = decltype(nb)::value, NL = decltype(nl)::value, W = kFillCells;
+    auto kern = pr == 4   ? (wide ? k_copy_fill<4, W, NB, NL> : k_copy_fill<4, 1, NB, NL>)
+                : pr == 8 ? (wide ? k_copy_fill<8, W, NB, NL> : k_copy_fill<8, 1, NB, NL>)
+                          : (wide ? k_copy_fill<0, W, NB, NL> : k_copy_fill<0, 1, NB, NL>);
+    pdl_launch(kern, dim3((unsigned)ctas), kThreads, 0, st, ht, ft);
+  };
+  if (nblocks == 1 && tab.n <= 6) {
+    HaloTable1 h1;
+    h1.n = tab.n;
+    CopyFillTable1 f1{1, ct.ghost, ct.cells, ct.gm1, ct.R, ct.p_ref, {ct.b[0]}, {}};
+    for (int L = 0; L < tab.n; ++L) {
+      h1.d[L] = tab.d[L];
+      f1.order[L] = ct.order[L];
+    }
+    launch(std::integral_constant<int, 1>(), std::integral_constant<int, 6>(), h1, f1);
+  } else {
+    launch(std::integral_constant<int, kMaxFillBlocks>(), std::integral_constant<int, kMaxLinksPerLaunch>(), tab, ct);
+  }
   ctx->launches += 1;
   s = launch_status(ctx, "copy-fill launch");
   if (s == FJ_OK) *done = true;

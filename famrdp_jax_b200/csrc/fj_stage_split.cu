@@ -27,8 +27,8 @@
 // A plan also keeps the metrics as records (kRecK<T> T per cell: the nine
 // kxyz[l][m], l-major, then pad), converted once from the caller's FP64
 // field-major kxyz; without one the kernels read kxyz field by field.
-// Each launch covers every block of a table; a CTA handles 256 consecutive
-// cells of one block, and neighbours are read through L1/L2.
+// Each launch covers every block of a table; a CTA handles 128 (assembly: 124)
+// consecutive cells of one block, and neighbours are read through L1/L2.
 #include "fj_common.cuh"
 #include "fj_physics.cuh"
 #include "fj_rhs.cuh"
@@ -42,12 +42,11 @@ namespace {
 
 using namespace sd;
 
-// NW: warps per CTA.  8 normally; 2 for tables too small to give every SM two
-// 256-thread CTAs (the 32^3 block: 183 CTAs of 256 would leave a fifth of the
-// SMs with twice the work), whose flux and assembly work runs in
-// k_split_fluxes_roles and k_split_assemble_kmem over the same 64-cell ranges.
-template <typename T, int NW = 8>
-__global__ void __launch_bounds__(32 * NW) k_split_prims(const Table tab, const double gm1, const double R,
+// NW: warps per CTA.  4 normally; 2 for tables of less than two 256-cell ranges
+// per SM (the 32^3 block), whose flux and assembly work runs in
+// k_split_fluxes_roles and k_split_assemble_kmem over 64-cell ranges.
+template <typename T, int NW, class TB>
+__global__ void __launch_bounds__(32 * NW) k_split_prims(const TB tab, const double gm1, const double R,
                                                          const double iR, const double p_ref) {
   const int b = find_block(tab, blockIdx.x);
   if (threadIdx.x == 0) prefetch_state(tab.b[b], blockIdx.x, 32 * NW);
@@ -58,14 +57,13 @@ __global__ void __launch_bounds__(32 * NW) k_split_prims(const Table tab, const 
   prims_cell<T>(B, c, gm1, R, iR, p_ref);
 }
 
-template <typename T, bool K_AOS, int OCC = SplitOcc<T>::fluxes>
-__global__ void __launch_bounds__(kSplitThreads, OCC) k_split_fluxes(const Table tab, const Phys ph,
-                                                                     const int flags) {
+template <typename T, bool K_AOS, int OCC, int NT, class TB>
+__global__ void __launch_bounds__(NT, OCC) k_split_fluxes(const TB tab, const Phys ph, const int flags) {
   const int b = find_block(tab, blockIdx.x);
-  if (threadIdx.x == 0) prefetch_fluxes<T, K_AOS, false>(tab.b[b], blockIdx.x);
+  if (threadIdx.x == 0) prefetch_fluxes<T, K_AOS, false>(tab.b[b], blockIdx.x, NT);
   grid_dep_wait();
   Cell x;
-  if (!decode(tab.b[b], blockIdx.x, x)) return;
+  if (!decode_cell(tab.b[b], (int64_t)(blockIdx.x - tab.b[b].blk.cta_begin) * NT + threadIdx.x, x)) return;
   flux_cell<T, K_AOS, true>(tab.b[b].blk, tab.b[b].blk.prim, x, ph, flags);
 }
 
@@ -76,8 +74,8 @@ __global__ void __launch_bounds__(kSplitThreads, OCC) k_split_fluxes(const Table
 // evaluating them).  Each thread's dependency chain is about a third of
 // k_split_fluxes' (a small table leaves most of the GPU's warp slots free,
 // and its kernels' times are set by those chains).
-template <typename T, bool K_AOS>
-__global__ void __launch_bounds__(256, 4) k_split_fluxes_roles(const Table tab, const Phys ph, const int flags) {
+template <typename T, bool K_AOS, class TB>
+__global__ void __launch_bounds__(256, 4) k_split_fluxes_roles(const TB tab, const Phys ph, const int flags) {
   const int b = find_block(tab, blockIdx.x);
   if (threadIdx.x == 0) prefetch_fluxes<T, K_AOS, false>(tab.b[b], blockIdx.x, 64);
   grid_dep_wait();
@@ -99,8 +97,8 @@ __global__ void __launch_bounds__(256, 4) k_split_fluxes_roles(const Table tab, 
 // The assembly of small FP32 tables: asm_chunk with the k faces read from Fk
 // (2-warp CTAs of 62 cells; a small table puts about five of them on an SM,
 // so the register cap is loose).
-template <typename T, bool K_AOS>
-__global__ void __launch_bounds__(64, 8) k_split_assemble_kmem(const Table tab, const int flags, const int stage,
+template <typename T, bool K_AOS, class TB>
+__global__ void __launch_bounds__(64, 8) k_split_assemble_kmem(const TB tab, const int flags, const int stage,
                                                                  const int next_prims, const double gm1,
                                                                  const double R, const double iR, const Phys ph) {
   const int b = find_block_asm(tab, blockIdx.x);
@@ -112,17 +110,16 @@ __global__ void __launch_bounds__(64, 8) k_split_assemble_kmem(const Table tab, 
                            gm1, R, iR, ph);
 }
 
-template <typename T, bool K_AOS, int OCC = SplitOcc<T>::assemble>
-__global__ void __launch_bounds__(kSplitThreads, OCC) k_split_assemble(const Table tab, const int flags,
-                                                                       const int stage, const int next_prims,
-                                                                       const double gm1, const double R,
-                                                                       const double iR, const Phys ph) {
+template <typename T, bool K_AOS, int OCC, int NW, class TB>
+__global__ void __launch_bounds__(32 * NW, OCC) k_split_assemble(const TB tab, const int flags, const int stage,
+                                                                 const int next_prims, const double gm1,
+                                                                 const double R, const double iR, const Phys ph) {
   const int b = find_block_asm(tab, blockIdx.x);
   const Dev& d = tab.b[b];
   const SplitBlock& B = d.blk;
-  if (threadIdx.x == 0) prefetch_assembly<T, K_AOS, false>(d, blockIdx.x, flags, stage, kAsmCells, B.cta_begin_asm);
+  if (threadIdx.x == 0) prefetch_assembly<T, K_AOS, false>(d, blockIdx.x, flags, stage, 31 * NW, B.cta_begin_asm);
   grid_dep_wait();
-  asm_chunk<T, K_AOS, true>(d, TablePtrs{B}, (int64_t)(blockIdx.x - B.cta_begin_asm) * kAsmCells, flags, stage,
+  asm_chunk<T, K_AOS, true>(d, TablePtrs{B}, (int64_t)(blockIdx.x - B.cta_begin_asm) * (31 * NW), flags, stage,
                             next_prims, gm1, R, iR, ph);
 }
 
@@ -133,8 +130,8 @@ __global__ void __launch_bounds__(kSplitThreads, OCC) k_split_assemble(const Tab
 // lane) and padding bytes than the index arithmetic they save.
 namespace fm {
 
-template <typename T, int NW = 8>
-__global__ void __launch_bounds__(32 * NW) k_fm_prims(const Table tab, const double gm1,
+template <typename T, int NW, class TB>
+__global__ void __launch_bounds__(32 * NW) k_fm_prims(const TB tab, const double gm1,
                                                               const double R, const double iR) {
   const int b = find_block(tab, blockIdx.x);
   if (threadIdx.x == 0) prefetch_state(tab.b[b], blockIdx.x, 32 * NW);
@@ -159,12 +156,12 @@ struct Cell6 {
   T r, u, v, w, p, t;
 };
 
-template <typename T, bool WITH_T>
-__device__ __forceinline__ Cell6<T> load_cell(const T* __restrict__ P, int32_t N, int32_t c) {
-  (void)N;
+// (values a caller does not use are not loaded: the loads are whole 16-byte pairs)
+template <typename T>
+__device__ __forceinline__ Cell6<T> load_cell(const T* __restrict__ P, int32_t c) {
   T x[kRecP64];
   ld_rec<T, kRecP64>(P + (size_t)c * kRecP64, x);
-  return Cell6<T>{x[0], x[1], x[2], x[3], x[4], WITH_T ? x[5] : T(0)};
+  return Cell6<T>{x[4], x[0], x[1], x[2], x[5], x[3]};
 }
 
 // Roe face c | c+e_a from the primitives of c-e_a, c, c+e_a, c+2e_a and the
@@ -187,16 +184,16 @@ __device__ __forceinline__ void metric_row(const SplitBlock& B, int32_t N, int r
   k[2] = (T)__ldg(K + 2 * N + c);
 }
 
-template <typename T, int OCC = 2>
-__global__ void __launch_bounds__(kSplitThreads, OCC) k_fm_fluxes(const Table tab, const Phys ph,
+template <typename T, int OCC, int NT, class TB>
+__global__ void __launch_bounds__(NT, OCC) k_fm_fluxes(const TB tab, const Phys ph,
                                                                  const int flags) {
   using M = FastMath<T>;
   const int b = find_block(tab, blockIdx.x);
-  if (threadIdx.x == 0) prefetch_fluxes<T, false, true>(tab.b[b], blockIdx.x);
+  if (threadIdx.x == 0) prefetch_fluxes<T, false, true>(tab.b[b], blockIdx.x, NT);
   grid_dep_wait();
   Cell x;
-  if (!decode(tab.b[b], blockIdx.x, x)) return;
   const SplitBlock& B = tab.b[b].blk;
+  if (!decode_cell(tab.b[b], (int64_t)(blockIdx.x - B.cta_begin) * NT + threadIdx.x, x)) return;
   // 32-bit offsets: 15 N < 2^31 is checked on the host
   const int32_t N = (int32_t)x.N, c = (int32_t)x.c;
   const int32_t si = x.nj * x.nk, sj = x.nk;
@@ -212,18 +209,18 @@ __global__ void __launch_bounds__(kSplitThreads, OCC) k_fm_fluxes(const Table ta
   const int32_t kp = x.k + 1 == x.nk ? c - (x.nk - 1) : c + 1;
   const int32_t km = x.k == 0 ? c + (x.nk - 1) : c - 1;
 
-  const Cell6<T> C0 = load_cell<T, true>(P, N, c);
-  const Cell6<T> Im = load_cell<T, true>(P, N, im), Ip = load_cell<T, true>(P, N, ip);
-  const Cell6<T> Jm = load_cell<T, true>(P, N, jm), Jp = load_cell<T, true>(P, N, jp);
-  const Cell6<T> Km = load_cell<T, true>(P, N, km), Kp = load_cell<T, true>(P, N, kp);
+  const Cell6<T> C0 = load_cell<T>(P, c);
+  const Cell6<T> Im = load_cell<T>(P, im), Ip = load_cell<T>(P, ip);
+  const Cell6<T> Jm = load_cell<T>(P, jm), Jp = load_cell<T>(P, jp);
+  const Cell6<T> Km = load_cell<T>(P, km), Kp = load_cell<T>(P, kp);
 
   if (vis) {
     // viscous flux components at c (rhs/viscous.py:36-105)
-    const T h = T(0.5);
-    const T d[4][3] = {{h * (Ip.u - Im.u), h * (Jp.u - Jm.u), h * (Kp.u - Km.u)},
-                       {h * (Ip.v - Im.v), h * (Jp.v - Jm.v), h * (Kp.v - Km.v)},
-                       {h * (Ip.w - Im.w), h * (Jp.w - Jm.w), h * (Kp.w - Km.w)},
-                       {h * (Ip.t - Im.t), h * (Jp.t - Jm.t), h * (Kp.t - Km.t)}};
+    // the central differences' factor 1/2 is carried by mu and kappa (exact)
+    const T d[4][3] = {{Ip.u - Im.u, Jp.u - Jm.u, Kp.u - Km.u},
+                       {Ip.v - Im.v, Jp.v - Jm.v, Kp.v - Km.v},
+                       {Ip.w - Im.w, Jp.w - Jm.w, Kp.w - Km.w},
+                       {Ip.t - Im.t, Jp.t - Jm.t, Kp.t - Km.t}};
     T kk[9];
     metric_row<T>(B, N, 0, c, kk);
     metric_row<T>(B, N, 1, c, kk + 3);
@@ -238,15 +235,15 @@ __global__ void __launch_bounds__(kSplitThreads, OCC) k_fm_fluxes(const Table ta
       const T r = C0.t * (T)ph.inv_T0;
       mu = (T)B.mu0 * (r * M::sqrt_pos(r)) * (T)ph.sfac * M::rcp(C0.t + (T)ph.Ts);
     }
-    const T kappa = (T)ph.kap_fac * mu;
+    const T muh = T(0.5) * mu, kappa = (T)ph.kap_fac * muh;
     const T third = (T)(1.0 / 3.0);
     const T div_u = g[0][0] + g[1][1] + g[2][2];
-    const T t00 = T(2) * mu * (g[0][0] - div_u * third);
-    const T t01 = mu * (g[0][1] + g[1][0]);
-    const T t02 = mu * (g[0][2] + g[2][0]);
-    const T t11 = T(2) * mu * (g[1][1] - div_u * third);
-    const T t12 = mu * (g[1][2] + g[2][1]);
-    const T t22 = T(2) * mu * (g[2][2] - div_u * third);
+    const T t00 = mu * (g[0][0] - div_u * third);
+    const T t01 = muh * (g[0][1] + g[1][0]);
+    const T t02 = muh * (g[0][2] + g[2][0]);
+    const T t11 = mu * (g[1][1] - div_u * third);
+    const T t12 = muh * (g[1][2] + g[2][1]);
+    const T t22 = mu * (g[2][2] - div_u * third);
     T* __restrict__ G = (T*)B.G;
     G[c] = t00;
     G[N + c] = t01;
@@ -263,7 +260,7 @@ __global__ void __launch_bounds__(kSplitThreads, OCC) k_fm_fluxes(const Table ta
     T* __restrict__ F = (T*)B.F;
     T kc[3], kn[3], Fo[5];
     if (x.i >= 1 && x.i <= x.ni - 3) {
-      const Cell6<T> I2 = load_cell<T, false>(P, N, c + 2 * si);
+      const Cell6<T> I2 = load_cell<T>(P, c + 2 * si);
       metric_row<T>(B, N, 0, c, kc);
       metric_row<T>(B, N, 0, c + si, kn);
       face_from_cells<T>(Im, C0, Ip, I2, kc, kn, ph, Fo);
@@ -271,7 +268,7 @@ __global__ void __launch_bounds__(kSplitThreads, OCC) k_fm_fluxes(const Table ta
       for (int v = 0; v < 5; ++v) F[v * N + c] = Fo[v];
     }
     if (x.j >= 1 && x.j <= x.nj - 3) {
-      const Cell6<T> J2 = load_cell<T, false>(P, N, c + 2 * sj);
+      const Cell6<T> J2 = load_cell<T>(P, c + 2 * sj);
       metric_row<T>(B, N, 1, c, kc);
       metric_row<T>(B, N, 1, c + sj, kn);
       face_from_cells<T>(Jm, C0, Jp, J2, kc, kn, ph, Fo);
@@ -293,8 +290,8 @@ __device__ __forceinline__ void fm_face_role(const SplitBlock& B, const Cell& x,
   if (ia < 1 || ia > na - 3) return;
   const int32_t sa = AXIS == 0 ? x.nj * x.nk : x.nk;
   const T* __restrict__ P = (const T*)B.prim;
-  const Cell6<T> a0 = load_cell<T, false>(P, N, c - sa), a1 = load_cell<T, false>(P, N, c),
-                 a2 = load_cell<T, false>(P, N, c + sa), a3 = load_cell<T, false>(P, N, c + 2 * sa);
+  const Cell6<T> a0 = load_cell<T>(P, c - sa), a1 = load_cell<T>(P, c),
+                 a2 = load_cell<T>(P, c + sa), a3 = load_cell<T>(P, c + 2 * sa);
   T kc[3], kn[3], Fo[5];
   metric_row<T>(B, N, AXIS, c, kc);
   metric_row<T>(B, N, AXIS, c + sa, kn);
@@ -316,15 +313,15 @@ __device__ __forceinline__ void fm_visc_role(const SplitBlock& B, const Cell& x,
   const int32_t jm = x.j == 0 ? c + (x.nj - 1) * sj : c - sj;
   const int32_t kp = x.k + 1 == x.nk ? c - (x.nk - 1) : c + 1;
   const int32_t km = x.k == 0 ? c + (x.nk - 1) : c - 1;
-  const Cell6<T> C0 = load_cell<T, true>(P, N, c);
-  const Cell6<T> Im = load_cell<T, true>(P, N, im), Ip = load_cell<T, true>(P, N, ip);
-  const Cell6<T> Jm = load_cell<T, true>(P, N, jm), Jp = load_cell<T, true>(P, N, jp);
-  const Cell6<T> Km = load_cell<T, true>(P, N, km), Kp = load_cell<T, true>(P, N, kp);
-  const T h = T(0.5);
-  const T d[4][3] = {{h * (Ip.u - Im.u), h * (Jp.u - Jm.u), h * (Kp.u - Km.u)},
-                     {h * (Ip.v - Im.v), h * (Jp.v - Jm.v), h * (Kp.v - Km.v)},
-                     {h * (Ip.w - Im.w), h * (Jp.w - Jm.w), h * (Kp.w - Km.w)},
-                     {h * (Ip.t - Im.t), h * (Jp.t - Jm.t), h * (Kp.t - Km.t)}};
+  const Cell6<T> C0 = load_cell<T>(P, c);
+  const Cell6<T> Im = load_cell<T>(P, im), Ip = load_cell<T>(P, ip);
+  const Cell6<T> Jm = load_cell<T>(P, jm), Jp = load_cell<T>(P, jp);
+  const Cell6<T> Km = load_cell<T>(P, km), Kp = load_cell<T>(P, kp);
+  // the central differences' factor 1/2 is carried by mu and kappa (exact)
+  const T d[4][3] = {{Ip.u - Im.u, Jp.u - Jm.u, Kp.u - Km.u},
+                     {Ip.v - Im.v, Jp.v - Jm.v, Kp.v - Km.v},
+                     {Ip.w - Im.w, Jp.w - Jm.w, Kp.w - Km.w},
+                     {Ip.t - Im.t, Jp.t - Jm.t, Kp.t - Km.t}};
   T kk[9];
   metric_row<T>(B, N, 0, c, kk);
   metric_row<T>(B, N, 1, c, kk + 3);
@@ -339,15 +336,15 @@ __device__ __forceinline__ void fm_visc_role(const SplitBlock& B, const Cell& x,
     const T r = C0.t * (T)ph.inv_T0;
     mu = (T)B.mu0 * (r * M::sqrt_pos(r)) * (T)ph.sfac * M::rcp(C0.t + (T)ph.Ts);
   }
-  const T kappa = (T)ph.kap_fac * mu;
+  const T muh = T(0.5) * mu, kappa = (T)ph.kap_fac * muh;
   const T third = (T)(1.0 / 3.0);
   const T div_u = g[0][0] + g[1][1] + g[2][2];
-  const T t00 = T(2) * mu * (g[0][0] - div_u * third);
-  const T t01 = mu * (g[0][1] + g[1][0]);
-  const T t02 = mu * (g[0][2] + g[2][0]);
-  const T t11 = T(2) * mu * (g[1][1] - div_u * third);
-  const T t12 = mu * (g[1][2] + g[2][1]);
-  const T t22 = T(2) * mu * (g[2][2] - div_u * third);
+  const T t00 = mu * (g[0][0] - div_u * third);
+  const T t01 = muh * (g[0][1] + g[1][0]);
+  const T t02 = muh * (g[0][2] + g[2][0]);
+  const T t11 = mu * (g[1][1] - div_u * third);
+  const T t12 = muh * (g[1][2] + g[2][1]);
+  const T t22 = mu * (g[2][2] - div_u * third);
   T* __restrict__ G = (T*)B.G;
   G[c] = t00;
   G[N + c] = t01;
@@ -360,8 +357,8 @@ __device__ __forceinline__ void fm_visc_role(const SplitBlock& B, const Cell& x,
   G[8 * N + c] = C0.u * t02 + C0.v * t12 + C0.w * t22 + kappa * g[3][2];
 }
 
-template <typename T>
-__global__ void __launch_bounds__(192, 2) k_fm_fluxes_roles(const Table tab, const Phys ph, const int flags) {
+template <typename T, class TB>
+__global__ void __launch_bounds__(192, 2) k_fm_fluxes_roles(const TB tab, const Phys ph, const int flags) {
   const int b = find_block(tab, blockIdx.x);
   if (threadIdx.x == 0) prefetch_fluxes<T, false, true>(tab.b[b], blockIdx.x, 64);
   grid_dep_wait();
@@ -383,8 +380,8 @@ __global__ void __launch_bounds__(192, 2) k_fm_fluxes_roles(const Table tab, con
 template <typename T>
 __device__ __forceinline__ void fm_k_face_left(const SplitBlock& B, int32_t N, int32_t c, const Phys& ph, T F[5]) {
   const T* __restrict__ P = (const T*)B.prim;
-  const Cell6<T> a0 = load_cell<T, false>(P, N, c - 2), a1 = load_cell<T, false>(P, N, c - 1),
-                 a2 = load_cell<T, false>(P, N, c), a3 = load_cell<T, false>(P, N, c + 1);
+  const Cell6<T> a0 = load_cell<T>(P, c - 2), a1 = load_cell<T>(P, c - 1),
+                 a2 = load_cell<T>(P, c), a3 = load_cell<T>(P, c + 1);
   T kl[3], kr[3];
   metric_row<T>(B, N, 2, c - 1, kl);
   metric_row<T>(B, N, 2, c, kr);
@@ -395,10 +392,14 @@ __device__ __forceinline__ void fm_k_face_left(const SplitBlock& B, int32_t N, i
 // left of its cell and takes the one on its right from lane l+1 by shuffle
 // (lane 31's cell is the next warp's first, for which it only supplies the
 // face), as in the FP32 assembly.
-// NW: warps per CTA (8; 2 for the small tables of launch_tab, with a looser
+// NW: warps per CTA (4; 2 for the small tables of launch_tab, with a looser
 // register cap since such a table puts few CTAs on an SM).
-template <typename T, int OCC = 3, int NW = 8>
-__global__ void __launch_bounds__(32 * NW, NW == 8 ? OCC : 8) k_fm_assemble(const Table tab, const int flags,
+// Bound by the latency of its loads (about 100 values a cell, most from L2): what
+// counts is how many times a thread waits, so the faces are one batch of loads
+// and the viscous components one per axis, with nothing branched around (4.0 M
+// cells: 369 -> 330 us against a branch per face and equation).
+template <typename T, int OCC, int NW, class TB>
+__global__ void __launch_bounds__(32 * NW, OCC) k_fm_assemble(const TB tab, const int flags,
                                                                  const int stage, const int next_prims,
                                                                  const double gm1, const double R,
                                                                  const double iR, const Phys ph) {
@@ -428,78 +429,50 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? OCC : 8) k_fm_assemble(cons
 #pragma unroll
   for (int v = 0; v < 5; ++v) fr[v] = __shfl_down_sync(0xffffffffu, fl[v], 1);
   if (lane == 31 || !alive) return;
-  const int64_t N = x.N, c = x.c;
-  const int64_t si = (int64_t)x.nj * x.nk, sj = x.nk;
+  // 32-bit offsets: 15 N < 2^31 is checked on the host
+  const int32_t N = (int32_t)x.N, c = (int32_t)x.c;
+  const int32_t si = x.nj * x.nk, sj = x.nk;
   const int n[3] = {x.ni, x.nj, x.nk};
   const int idx[3] = {x.i, x.j, x.k};
-  const int64_t st[3] = {si, sj, 1};
+  const int32_t st[3] = {si, sj, 1};
   double r[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
   if (flags & kRhsInvscd) {
-    const T* F = (const T*)B.F;
-    const double ivd = __drcp_rn(B.vol[c] + 1e-300);
-    const bool on[3] = {idx[0] >= 2 && idx[0] <= n[0] - 3, idx[1] >= 2 && idx[1] <= n[1] - 3,
-                        idx[2] >= 2 && idx[2] <= n[2] - 3};
+    // every face value in one batch of loads: a face that does not count is read
+    // at the cell itself and left out of the sum, not branched around
+    const bool on_i = idx[0] >= 2 && idx[0] <= n[0] - 3, on_j = idx[1] >= 2 && idx[1] <= n[1] - 3,
+               on_k = idx[2] >= 2 && idx[2] <= n[2] - 3;
+    const double ivd = rcp_normal(__ldg(B.vol + c) + 1e-300);
+    const T* __restrict__ F = (const T*)B.F + c;
+    const T* __restrict__ Fi = F - (on_i ? si : 0);
+    const T* __restrict__ Fj = F - (on_j ? sj : 0);
+    T di[5], dj[5];
 #pragma unroll
     for (int v = 0; v < 5; ++v) {
-      double dsum;
-      if (sizeof(T) == sizeof(double)) {
-        dsum = 0.0;  // axis by axis like the reference
-#pragma unroll
-        for (int a = 0; a < 3; ++a)
-          if (on[a]) {
-            if (a == 2) {
-              dsum += (double)(fr[v] - fl[v]);
-            } else {
-              const T* Fa = F + (int64_t)(a * 5 + v) * N;
-              dsum += (double)(Fa[c] - Fa[c - st[a]]);
-            }
-          }
-      } else {
-        T s = T(0);
-#pragma unroll
-        for (int a = 0; a < 3; ++a)
-          if (on[a]) {
-            if (a == 2) {
-              s += fr[v] - fl[v];
-            } else {
-              const T* Fa = F + (int64_t)(a * 5 + v) * N;
-              s += Fa[c] - Fa[c - st[a]];
-            }
-          }
-        dsum = (double)s;
-      }
-      r[v] = -dsum * ivd;
+      di[v] = __ldg(F + v * N) - __ldg(Fi + v * N);
+      dj[v] = __ldg(F + (5 + v) * N) - __ldg(Fj + (5 + v) * N);
     }
+#pragma unroll
+    for (int v = 0; v < 5; ++v)  // axis by axis like the reference
+      r[v] = -((on_i ? di[v] : 0.0) + (on_j ? dj[v] : 0.0) + (on_k ? fr[v] - fl[v] : 0.0)) * ivd;
   }
   if (flags & kRhsViscous) {
-    const T* G = (const T*)B.G;
-    int64_t cp[3], cm[3];
+    // sum over l of 0.5 kxyz[l][jj] (G(c+e_l) - G(c-e_l)): the 18 components of
+    // an axis in one batch of loads
+    const T* __restrict__ G = (const T*)B.G;
+    const T* __restrict__ K = B.kxyz + c;
 #pragma unroll
     for (int l = 0; l < 3; ++l) {
-      cp[l] = idx[l] + 1 == n[l] ? c - (int64_t)(n[l] - 1) * st[l] : c + st[l];
-      cm[l] = idx[l] == 0 ? c + (int64_t)(n[l] - 1) * st[l] : c - st[l];
-    }
-    T kk[9];
+      const T* __restrict__ gp = G + (idx[l] + 1 == n[l] ? c - (n[l] - 1) * st[l] : c + st[l]);
+      const T* __restrict__ gm = G + (idx[l] == 0 ? c + (n[l] - 1) * st[l] : c - st[l]);
+      T g[9];
 #pragma unroll
-    for (int lm = 0; lm < 9; ++lm) kk[lm] = metric<T>(B, N, lm, c);
-    // D[comp][l] = 0.5 (G(c+e_l) - G(c-e_l))
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      T res = T(0);
-#pragma unroll
-      for (int jj = 0; jj < 3; ++jj) {
-        int comp;
-        if (e == 3) {
-          comp = 6 + jj;
-        } else {
-          const int lo = e < jj ? e : jj, hi = e < jj ? jj : e;
-          comp = lo == 0 ? hi : (lo == 1 ? 2 + hi : 5);
-        }
-        const T* Gc = G + (int64_t)comp * N;
-        res += T(0.5) * ((Gc[cp[0]] - Gc[cm[0]]) * kk[jj] + (Gc[cp[1]] - Gc[cm[1]]) * kk[3 + jj] +
-                         (Gc[cp[2]] - Gc[cm[2]]) * kk[6 + jj]);
-      }
-      r[e + 1] += (double)res;
+      for (int m = 0; m < 9; ++m) g[m] = __ldg(gp + m * N) - __ldg(gm + m * N);
+      const T k0 = T(0.5) * __ldg(K + (3 * l) * N), k1 = T(0.5) * __ldg(K + (3 * l + 1) * N),
+              k2 = T(0.5) * __ldg(K + (3 * l + 2) * N);
+      r[1] += g[0] * k0 + g[1] * k1 + g[2] * k2;
+      r[2] += g[1] * k0 + g[3] * k1 + g[4] * k2;
+      r[3] += g[2] * k0 + g[4] * k1 + g[5] * k2;
+      r[4] += g[6] * k0 + g[7] * k1 + g[8] * k2;
     }
   }
   if (stage == 0) {
@@ -511,7 +484,7 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? OCC : 8) k_fm_assemble(cons
     double qn[5];
 #pragma unroll
     for (int v = 0; v < 5; ++v) {
-      const int64_t o = v * N + c;
+      const int32_t o = v * N + c;
       const double t = B.q[o] + B.dt * r[v];
       qn[v] = stage == 1 ? t : ca * B.q0[o] + cb * t;
       B.out[o] = qn[v];
@@ -593,64 +566,71 @@ __global__ void k_fold_sum(const double* __restrict__ part, int n, double* __res
 
 // Launch shapes of the split kernels, selected per plan by the autotuner
 // (index 0 is the default): the minimum resident CTAs per SM of the flux and
-// assembly kernels, i.e. their register caps.  These are the FP32 record
-// kernels' shapes; kSplitVariants64 below are the FP64 kernels'.
+// assembly kernels, i.e. their register caps, for CTAs of 4 warps (8-warp CTAs
+// at the same registers leave an SM idler between CTAs: 1.057 against 1.049 ms
+// for an FP32 step of 4.0 M cells, 1.867 against 1.813 ms in FP64; 2-warp CTAs
+// 1.33 and 1.81).  These are the FP32 record kernels' shapes; kSplitVariants64
+// below are the FP64 kernels'.
 struct SplitShape {
   int flux_occ, asm_occ;
 };
-constexpr SplitShape kSplitVariants[] = {{4, 4}, {3, 4}, {3, 6}, {3, 5}, {4, 3}, {2, 4}};
+constexpr int kWarps32 = 4;  // warps per CTA
+constexpr SplitShape kSplitVariants[] = {{9, 8}, {8, 8}, {7, 8}, {6, 8}, {8, 6}, {4, 8}};
 static_assert(sizeof(kSplitVariants) / sizeof(kSplitVariants[0]) == FJ_NUM_SPLIT_VARIANTS, "variant table");
 
 // Launch shapes of the FP64 field-major kernels (the same variant index; FP64
 // face arithmetic needs more registers at the same occupancy).
-constexpr SplitShape kSplitVariants64[] = {{2, 3}, {2, 4}, {3, 3}, {2, 2}, {3, 4}, {3, 2}};
+constexpr int kWarps64 = 4;
+constexpr SplitShape kSplitVariants64[] = {{4, 5}, {4, 6}, {4, 4}, {5, 5}, {5, 6}, {3, 5}};
 static_assert(sizeof(kSplitVariants64) / sizeof(kSplitVariants64[0]) == FJ_NUM_SPLIT_VARIANTS, "variant table");
 
-template <int V>
-void launch_pair64(const Table& tab, int ctas, int asm_ctas, const Phys& ph, int flags, int stage, int np,
+template <int V, class TB>
+void launch_pair64(const TB& tab, int ctas, int asm_ctas, const Phys& ph, int flags, int stage, int np,
                    cudaStream_t st, cudaEvent_t after_fluxes) {
   constexpr SplitShape sh = kSplitVariants64[V];
-  pdl_launch(fm::k_fm_fluxes<double, sh.flux_occ>, ctas, kSplitThreads, 0, st, tab, ph, flags);
+  constexpr int nt = 32 * kWarps64;
+  pdl_launch(fm::k_fm_fluxes<double, sh.flux_occ, nt, TB>, ctas, nt, 0, st, tab, ph, flags);
   if (after_fluxes) cudaEventRecord(after_fluxes, st);
-  pdl_launch(fm::k_fm_assemble<double, sh.asm_occ>, asm_ctas, kSplitThreads, 0, st, tab, flags, stage, np, ph.gm1,
+  pdl_launch(fm::k_fm_assemble<double, sh.asm_occ, kWarps64, TB>, asm_ctas, nt, 0, st, tab, flags, stage, np, ph.gm1,
              ph.R, 1.0 / ph.R, ph);
 }
 
-template <typename T, bool K_AOS, int V>
-void launch_pair(const Table& tab, int ctas, int asm_ctas, const Phys& ph, int flags, int stage, int np,
+template <typename T, bool K_AOS, int V, class TB>
+void launch_pair(const TB& tab, int ctas, int asm_ctas, const Phys& ph, int flags, int stage, int np,
                  cudaStream_t st, cudaEvent_t after_fluxes) {
   constexpr SplitShape sh = kSplitVariants[V];
-  pdl_launch(k_split_fluxes<T, K_AOS, sh.flux_occ>, ctas, kSplitThreads, 0, st, tab, ph, flags);
+  constexpr int nt = 32 * kWarps32;
+  pdl_launch(k_split_fluxes<T, K_AOS, sh.flux_occ, nt, TB>, ctas, nt, 0, st, tab, ph, flags);
   if (after_fluxes) cudaEventRecord(after_fluxes, st);
-  pdl_launch(k_split_assemble<T, K_AOS, sh.asm_occ>, asm_ctas, kSplitThreads, 0, st, tab, flags, stage, np, ph.gm1,
+  pdl_launch(k_split_assemble<T, K_AOS, sh.asm_occ, kWarps32, TB>, asm_ctas, nt, 0, st, tab, flags, stage, np, ph.gm1,
              ph.R, 1.0 / ph.R, ph);
 }
 
-template <typename T, bool K_AOS>
-int launch_tab(const Table& tab, int ctas, int asm_ctas, const Phys& ph, int flags, int stage, bool prims_ready,
+template <typename T, bool K_AOS, class TB>
+int launch_tab(const TB& tab, int ctas, int asm_ctas, const Phys& ph, int flags, int stage, bool prims_ready,
                bool next_prims, int variant, cudaStream_t st, cudaEvent_t after_fluxes, int nw = 8) {
   const int np = next_prims ? 1 : 0;
   if constexpr (sizeof(T) == 4) {
     if (nw == 2) {  // a small table: the role-split flux kernel and 2-warp assembly CTAs
       if (!prims_ready)
-        pdl_launch(k_split_prims<T, 2>, ctas, 64, 0, st, tab, ph.gm1, ph.R, 1.0 / ph.R, K_AOS ? ph.p_ref : 0.0);
-      pdl_launch(k_split_fluxes_roles<T, K_AOS>, ctas, 256, 0, st, tab, ph, flags);
+        pdl_launch(k_split_prims<T, 2, TB>, ctas, 64, 0, st, tab, ph.gm1, ph.R, 1.0 / ph.R, K_AOS ? ph.p_ref : 0.0);
+      pdl_launch(k_split_fluxes_roles<T, K_AOS, TB>, ctas, 256, 0, st, tab, ph, flags);
       if (after_fluxes) cudaEventRecord(after_fluxes, st);
-      pdl_launch(k_split_assemble_kmem<T, K_AOS>, asm_ctas, 64, 0, st, tab, flags, stage, np, ph.gm1, ph.R,
+      pdl_launch(k_split_assemble_kmem<T, K_AOS, TB>, asm_ctas, 64, 0, st, tab, flags, stage, np, ph.gm1, ph.R,
                  1.0 / ph.R, ph);
       return prims_ready ? 2 : 3;
     }
   }
   if constexpr (sizeof(T) == 8) {
     if (nw == 2) {  // a small table: the role-split flux kernel and 2-warp CTAs
-      if (!prims_ready) pdl_launch(fm::k_fm_prims<double, 2>, ctas, 64, 0, st, tab, ph.gm1, ph.R, 1.0 / ph.R);
-      pdl_launch(fm::k_fm_fluxes_roles<double>, ctas, 192, 0, st, tab, ph, flags);
+      if (!prims_ready) pdl_launch(fm::k_fm_prims<double, 2, TB>, ctas, 64, 0, st, tab, ph.gm1, ph.R, 1.0 / ph.R);
+      pdl_launch(fm::k_fm_fluxes_roles<double, TB>, ctas, 192, 0, st, tab, ph, flags);
       if (after_fluxes) cudaEventRecord(after_fluxes, st);
-      pdl_launch(fm::k_fm_assemble<double, 3, 2>, asm_ctas, 64, 0, st, tab, flags, stage, np, ph.gm1, ph.R,
+      pdl_launch(fm::k_fm_assemble<double, 8, 2, TB>, asm_ctas, 64, 0, st, tab, flags, stage, np, ph.gm1, ph.R,
                  1.0 / ph.R, ph);
       return prims_ready ? 2 : 3;
     }
-    if (!prims_ready) pdl_launch(fm::k_fm_prims<double>, ctas, kSplitThreads, 0, st, tab, ph.gm1, ph.R, 1.0 / ph.R);
+    if (!prims_ready) pdl_launch(fm::k_fm_prims<double, kWarps64, TB>, ctas, 32 * kWarps64, 0, st, tab, ph.gm1, ph.R, 1.0 / ph.R);
     switch (variant) {
       case 1: launch_pair64<1>(tab, ctas, asm_ctas, ph, flags, stage, np, st, after_fluxes); break;
       case 2: launch_pair64<2>(tab, ctas, asm_ctas, ph, flags, stage, np, st, after_fluxes); break;
@@ -661,7 +641,7 @@ int launch_tab(const Table& tab, int ctas, int asm_ctas, const Phys& ph, int fla
     }
   } else {
     if (!prims_ready)
-      pdl_launch(k_split_prims<T>, ctas, kSplitThreads, 0, st, tab, ph.gm1, ph.R, 1.0 / ph.R, K_AOS ? ph.p_ref : 0.0);
+      pdl_launch(k_split_prims<T, kWarps32, TB>, ctas, 32 * kWarps32, 0, st, tab, ph.gm1, ph.R, 1.0 / ph.R, K_AOS ? ph.p_ref : 0.0);
     switch (K_AOS ? variant : 0) {
       case 1: launch_pair<T, K_AOS, 1>(tab, ctas, asm_ctas, ph, flags, stage, np, st, after_fluxes); break;
       case 2: launch_pair<T, K_AOS, 2>(tab, ctas, asm_ctas, ph, flags, stage, np, st, after_fluxes); break;
@@ -685,7 +665,7 @@ int launch_split(fj_ctx* ctx, const SplitBlock* blocks, int nblocks, const Phys&
     Table tab;
     tab.n = std::min(kMaxSplitBlocks, nblocks - base);
     // tables with fewer 256-thread flux CTAs than two per SM run 2-warp CTAs
-    int nw = 8;
+    int nw = sizeof(T) == 8 ? kWarps64 : kWarps32;
     {
       int64_t wide = 0;
       for (int t = 0; t < tab.n; ++t) {
@@ -717,10 +697,11 @@ int launch_split(fj_ctx* ctx, const SplitBlock* blocks, int nblocks, const Phys&
       return set_err(ctx, FJ_ERR_INVALID_ARGUMENT, "the FP64 split path reads kxyz directly");
     // the event marks the first chunk's flux launch
     cudaEvent_t ev = base == 0 ? after_fluxes : nullptr;
-    ctx->launches += k_aos ? launch_tab<T, true>(tab, ctas, asm_ctas, ph, flags, stage, prims_ready, next_prims,
-                                                 variant, st, ev, nw)
-                           : launch_tab<T, false>(tab, ctas, asm_ctas, ph, flags, stage, prims_ready, next_prims,
-                                                  variant, st, ev, nw);
+    auto launch = [&](const auto& t) {
+      return k_aos ? launch_tab<T, true>(t, ctas, asm_ctas, ph, flags, stage, prims_ready, next_prims, variant, st, ev, nw)
+                   : launch_tab<T, false>(t, ctas, asm_ctas, ph, flags, stage, prims_ready, next_prims, variant, st, ev, nw);
+    };
+    ctx->launches += tab.n == 1 ? launch(TableN<1>{1, {tab.b[0]}}) : launch(tab);
     int s = launch_status(ctx, "split stage launch");
     if (s != FJ_OK) return s;
   }

@@ -29,6 +29,7 @@
 #include "fj_adjoint.cuh"
 #include "fj_common.cuh"
 #include "fj_rhs.cuh"
+#include "fj_split_dev.cuh"
 
 namespace fj {
 
@@ -38,13 +39,14 @@ constexpr int kAT = 256;
 
 struct ADims {
   int ni, nj, nk;
+  sd::FastDiv dk, dj;  // n / nk, n / nj
 };
 
 __device__ __forceinline__ void dec(int c, const ADims& d, int& i, int& j, int& k) {
-  k = c % d.nk;
-  const int t = c / d.nk;
-  j = t % d.nj;
-  i = t / d.nj;
+  const int t = (int)d.dk.div((uint32_t)c);
+  k = c - t * d.nk;
+  i = (int)d.dj.div((uint32_t)t);
+  j = t - i * d.nj;
 }
 
 __device__ __forceinline__ void wrapped(int c, int i, int j, int k, const ADims& d, int nb[6]) {
@@ -99,6 +101,23 @@ __device__ __forceinline__ void write_prims(const double* __restrict__ q, T* __r
   store_prims<T>(P, N, c, x);
 }
 
+// The face kernel's sums: the adjoint of (rho, u, v, w, p) of each cell, in FP32
+// one 32-byte record per cell (three pad values: a cell's five additions are one
+// 16-byte vector atomic and one scalar), in FP64 five field-major arrays.
+template <typename T>
+constexpr int kLamVals = sizeof(T) == 4 ? 8 : 5;
+
+template <typename T>
+__device__ __forceinline__ void clear_sums(T* __restrict__ lamP, int N, int c) {
+  if constexpr (sizeof(T) == 4) {
+    const float z[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    sd::st_rec<float, 8>(lamP + (size_t)c * 8, z);
+  } else {
+#pragma unroll
+    for (int v = 0; v < 5; ++v) lamP[v * N + c] = T(0);
+  }
+}
+
 // With lv, also lv = lam / (vol + 1e-300) per cell, in FP64: the face adjoint
 // -lam(c)/vol(c) + lam(c+e_a)/vol(c+e_a) of every axis then costs one FP64
 // subtraction per face instead of two divisions.
@@ -106,11 +125,10 @@ template <typename T>
 __global__ void k_adj_prims(const double* __restrict__ q, T* __restrict__ P, int N, double gm1,
                             double R, const double* __restrict__ lam, const double* __restrict__ vol,
                             double* __restrict__ lv, T* __restrict__ lamP) {
+  grid_dep_wait();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= N) return;
-  if (lamP)  // cleared here for the face kernel's atomic sums
-#pragma unroll
-    for (int v = 0; v < 5; ++v) lamP[v * N + c] = T(0);
+  if (lamP) clear_sums<T>(lamP, N, c);  // for the face kernel's atomic sums
   if (lv) {
     const double iv = 1.0 / (vol[c] + 1e-300);
 #pragma unroll
@@ -119,42 +137,36 @@ __global__ void k_adj_prims(const double* __restrict__ q, T* __restrict__ P, int
   write_prims<T>(q, P, N, c, gm1, R);
 }
 
-__device__ __forceinline__ void atomic_add(float* a, float v) { atomicAdd(a, v); }
-__device__ __forceinline__ void atomic_add(double* a, double v) { atomicAdd(a, v); }
-
 // Face c | c+e_a (stride sa): loads the four MUSCL cells and the two cells'
 // metric rows, then the reverse of MUSCL + Roe; lc[s][v] = adjoint of the
 // primitive v (rho, u, v, w, p) of cell c + (s-1) e_a.
 template <typename T>
 __device__ __forceinline__ void face_vjp_cells(const T* __restrict__ P, const double* __restrict__ K, int N,
                                                int c, int sa, const T lF[5], const Phys& ph, T lc[4][5]) {
-  Prim<T> cell[4], l4[4];
+  Prim<T> cell[4];
 #pragma unroll
   for (int s = 0; s < 4; ++s) {
-    const int cc = c + (s - 1) * sa;
     T x[6];
-    load_prims<T>(P, N, cc, x);
+    load_prims<T>(P, N, c + (s - 1) * sa, x);
     cell[s] = Prim<T>{x[0], x[1], x[2], x[3], x[4]};
-    l4[s] = Prim<T>{T(0), T(0), T(0), T(0), T(0)};
   }
   const int cr = c + sa;
   invscd_face_vjp<T>(cell, (T)K[c], (T)K[N + c], (T)K[2 * N + c], (T)K[cr], (T)K[N + cr], (T)K[2 * N + cr],
-                     (T)ph.gm1, (T)ph.inv_gm1, (T)ph.eps_entropy, ph.limiter, lF, l4);
-#pragma unroll
-  for (int s = 0; s < 4; ++s) {
-    lc[s][0] = l4[s].rho;
-    lc[s][1] = l4[s].u;
-    lc[s][2] = l4[s].v;
-    lc[s][3] = l4[s].w;
-    lc[s][4] = l4[s].p;
-  }
+                     num<T>(ph).gm1, num<T>(ph).inv_gm1, num<T>(ph).eps_entropy, ph.limiter, lF, lc);
 }
 
+// lamP of cell c += v
 template <typename T>
 __device__ __forceinline__ void add_cell(T* __restrict__ lamP, int N, int c, const T v[5]) {
+  if constexpr (sizeof(T) == 4) {
+    float* a = lamP + (size_t)c * 8;
+    atomicAdd(reinterpret_cast<float4*>(a), make_float4(v[0], v[1], v[2], v[3]));
+    atomicAdd(a + 4, v[4]);
+  } else {
 #pragma unroll
-  for (int f = 0; f < 5; ++f)
-    if (v[f] != T(0)) atomic_add(lamP + f * N + c, v[f]);
+    for (int f = 0; f < 5; ++f)
+      if (v[f] != T(0)) atomicAdd(lamP + f * N + c, v[f]);
+  }
 }
 
 // The inviscid part of the RHS VJP (reverse of rhs/invscd.py:119-131 and of
@@ -198,24 +210,26 @@ __device__ __forceinline__ void adj_faces_body(const T* __restrict__ P, const do
   for (int s = 0; s < 4; ++s)
 #pragma unroll
     for (int f = 0; f < 5; ++f) lc[s][f] = T(0);
+  bool live = false;  // this thread's face exists and has a nonzero adjoint
   if (c < N) {
-    const int ia = a == 0 ? c / (d.nj * d.nk) : (a == 1 ? (c / d.nk) % d.nj : c % d.nk);
+    int ijk[3];
+    dec(c, d, ijk[0], ijk[1], ijk[2]);
+    const int ia = a == 0 ? ijk[0] : (a == 1 ? ijk[1] : ijk[2]);
     if (ia >= 1 && ia <= n_a - 3) {
       const bool inL = ia >= 2, inR = ia + 1 <= n_a - 3;
       const int cr = c + sa;
       T lF[5];
-      bool any = false;
 #pragma unroll
       for (int v = 0; v < 5; ++v) {
         const double x = (inL ? -lv[v * N + c] : 0.0) + (inR ? lv[v * N + cr] : 0.0);
         lF[v] = (T)x;
-        any |= x != 0.0;
+        live |= x != 0.0;
       }
-      if (any) face_vjp_cells<T>(P, kxyz + (size_t)(3 * a) * N, N, c, sa, lF, ph, lc);
+      if (live) face_vjp_cells<T>(P, kxyz + (size_t)(3 * a) * N, N, c, sa, lF, ph, lc);
     }
   }
   if (a != 2) {
-    if (c < N)
+    if (live)
 #pragma unroll
       for (int s = 0; s < 4; ++s) add_cell<T>(lamP, N, c + (s - 1) * sa, lc[s]);
     return;
@@ -231,15 +245,18 @@ __device__ __forceinline__ void adj_faces_body(const T* __restrict__ P, const do
              (lane >= 2 ? from_left2 : T(0));
   }
   if (c < N) add_cell<T>(lamP, N, c, own);
-  if (lane == 0) add_cell<T>(lamP, N, c - 1, lc[0]);  // nonzero only for a valid face, so c >= 1
-  if (lane == 31) add_cell<T>(lamP, N, c + 1, lc[2]);
-  if (lane >= 30) add_cell<T>(lamP, N, c + 2, lc[3]);
+  if (live) {  // what leaves the warp (an existing face: cells c-1 .. c+2 are in the block)
+    if (lane == 0) add_cell<T>(lamP, N, c - 1, lc[0]);
+    if (lane == 31) add_cell<T>(lamP, N, c + 1, lc[2]);
+    if (lane >= 30) add_cell<T>(lamP, N, c + 2, lc[3]);
+  }
 }
 
 template <typename T, int NT, int MB>
 __global__ void __launch_bounds__(NT, MB) k_adj_faces(const T* __restrict__ P, const double* __restrict__ kxyz,
                                                       const double* __restrict__ lv, T* __restrict__ lamP, ADims d,
                                                       Phys ph) {
+  grid_dep_wait();
   adj_faces_body<T>(P, kxyz, lv, lamP, d, ph, blockIdx.y, blockIdx.x);
 }
 
@@ -266,19 +283,19 @@ __device__ __forceinline__ double adj_visc_cell(const T* __restrict__ P, const d
       // side 0: c = y - e_l (y is its + neighbour, weight +0.5); side 1: c = y + e_l (-0.5)
       const int c = side == 0 ? nb[2 * l + 1] : nb[2 * l];
       const double wgt = side == 0 ? 0.5 : -0.5;
-      const double k0 = kxyz[(3 * l + 0) * N + c], k1 = kxyz[(3 * l + 1) * N + c],
-                   k2 = kxyz[(3 * l + 2) * N + c];
+      const double k0 = wgt * kxyz[(3 * l + 0) * N + c], k1 = wgt * kxyz[(3 * l + 1) * N + c],
+                   k2 = wgt * kxyz[(3 * l + 2) * N + c];
       const double L1 = lam[N + c], L2 = lam[2 * N + c], L3 = lam[3 * N + c], L4 = lam[4 * N + c];
       // comp(e, jj): tau_00 tau_01 tau_02 tau_11 tau_12 tau_22 Ge_0 Ge_1 Ge_2
-      lG[0] += wgt * (k0 * L1);
-      lG[1] += wgt * (k1 * L1 + k0 * L2);
-      lG[2] += wgt * (k2 * L1 + k0 * L3);
-      lG[3] += wgt * (k1 * L2);
-      lG[4] += wgt * (k2 * L2 + k1 * L3);
-      lG[5] += wgt * (k2 * L3);
-      lG[6] += wgt * (k0 * L4);
-      lG[7] += wgt * (k1 * L4);
-      lG[8] += wgt * (k2 * L4);
+      lG[0] += k0 * L1;
+      lG[1] += k1 * L1 + k0 * L2;
+      lG[2] += k2 * L1 + k0 * L3;
+      lG[3] += k1 * L2;
+      lG[4] += k2 * L2 + k1 * L3;
+      lG[5] += k2 * L3;
+      lG[6] += k0 * L4;
+      lG[7] += k1 * L4;
+      lG[8] += k2 * L4;
     }
   }
   // ---- forward of the viscous fluxes at y (rhs/viscous.py:36-105)
@@ -305,11 +322,11 @@ __device__ __forceinline__ double adj_visc_cell(const T* __restrict__ P, const d
   const T u = xy[1], v = xy[2], w = xy[3], Tt = xy[5];
   T mu = (T)ph.mu0, dmu_dT = T(0);
   if (ph.visc_law == 0) {
-    const T r = Tt * (T)ph.inv_T0;
-    mu = (T)ph.mu0 * (r * M::sqrt_pos(r)) * (T)ph.sfac * M::rcp(Tt + (T)ph.Ts);
-    dmu_dT = mu * (T(1.5) * M::rcp(Tt) - M::rcp(Tt + (T)ph.Ts));
+    const T r = Tt * num<T>(ph).inv_T0;
+    mu = (T)ph.mu0 * (r * M::sqrt_pos(r)) * num<T>(ph).sfac * M::rcp(Tt + num<T>(ph).Ts);
+    dmu_dT = mu * (T(1.5) * M::rcp(Tt) - M::rcp(Tt + num<T>(ph).Ts));
   }
-  const T kap = (T)ph.kap_fac;
+  const T kap = num<T>(ph).kap_fac;
   const T kappa = kap * mu;
   const T third = (T)(1.0 / 3.0);
   const T div_u = g[0][0] + g[1][1] + g[2][2];
@@ -394,11 +411,12 @@ __device__ __forceinline__ void adj_visc_body(const T* __restrict__ P, const dou
   }
 }
 
-template <typename T, int MB = 1>
+template <typename T, int MB>
 __global__ void __launch_bounds__(kAT, MB) k_adj_visc(const T* __restrict__ P, const double* __restrict__ kxyz,
                                                      const double* __restrict__ lam, T* __restrict__ lamD,
                                                      T* __restrict__ lamL, ADims d, Phys ph,
                                                      double* __restrict__ dmu, double mu_scale) {
+  grid_dep_wait();
   adj_visc_body<T>(P, kxyz, lam, lamD, lamL, d, ph, dmu, mu_scale, blockIdx.x);
 }
 
@@ -408,12 +426,14 @@ __global__ void __launch_bounds__(kAT, MB) k_adj_visc(const T* __restrict__ P, c
 // face work with the load-bound viscous work on the same SMs and reads the
 // same primitive, metric and adjoint ranges for all four tasks.  The tasks
 // write disjoint arrays (lamP by atomics; lamD, lamL), so their order does not
-// matter.
+// matter.  1.0 M cells, FP32: 181 us, of which the atomics cost about 30 (195 us
+// with five scalar atomics a cell, 0/1 weights and 256-thread CTAs).
 template <typename T, int NT, int MB>
 __global__ void __launch_bounds__(NT, MB)
     k_adj_faces_visc(const T* __restrict__ P, const double* __restrict__ kxyz, const double* __restrict__ lv,
                      T* __restrict__ lamP, const double* __restrict__ lam, T* __restrict__ lamD,
                      T* __restrict__ lamL, ADims d, Phys ph, double* __restrict__ dmu, double mu_scale) {
+  grid_dep_wait();
   const int task = blockIdx.x & 3, bx = blockIdx.x >> 2;
   if (task < 3)
     adj_faces_body<T>(P, kxyz, lv, lamP, d, ph, task, bx);
@@ -425,6 +445,7 @@ template <typename T>
 __global__ void k_adj_final(const double* __restrict__ q, T* lamP, const T* __restrict__ lamD,
                             const T* __restrict__ lamL, double* __restrict__ out, T* __restrict__ P,
                             double* __restrict__ lam_vol, ADims d, Phys ph, int flags, VjpEpilogue e) {
+  grid_dep_wait();
   const int N = d.ni * d.nj * d.nk;
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= N) return;
@@ -434,7 +455,10 @@ __global__ void k_adj_final(const double* __restrict__ q, T* lamP, const T* __re
     const int a1 = c0 + d.nj * d.nk, m1 = min(n, N - a1);
     for (int f = 0; f < 5; ++f) l2_prefetch(q + (size_t)f * N + c0, n * 8);
     if (flags & kRhsInvscd)
-      for (int f = 0; f < 5; ++f) l2_prefetch(lamP + (size_t)f * N + c0, n * (int)sizeof(T));
+      if constexpr (sizeof(T) == 4)
+        l2_prefetch(lamP + (size_t)c0 * 8, n * 32);
+      else
+        for (int f = 0; f < 5; ++f) l2_prefetch(lamP + (size_t)f * N + c0, n * (int)sizeof(T));
     if (flags & kRhsViscous) {
       for (int s = 0; s < 4; ++s) l2_prefetch(lamL + (size_t)s * N + c0, n * (int)sizeof(T));
       if (m1 > 0)
@@ -448,11 +472,20 @@ __global__ void k_adj_final(const double* __restrict__ q, T* lamP, const T* __re
   }
   double lr = 0, lu = 0, lv = 0, lw = 0, lp = 0, lT = 0;
   if (flags & kRhsInvscd) {
-    lr = lamP[x];
-    lu = lamP[N + x];
-    lv = lamP[2 * N + x];
-    lw = lamP[3 * N + x];
-    lp = lamP[4 * N + x];
+    if constexpr (sizeof(T) == 4) {
+      const float4 a = *reinterpret_cast<const float4*>(lamP + (size_t)x * 8);
+      lr = a.x;
+      lu = a.y;
+      lv = a.z;
+      lw = a.w;
+      lp = lamP[(size_t)x * 8 + 4];
+    } else {
+      lr = lamP[x];
+      lu = lamP[N + x];
+      lv = lamP[2 * N + x];
+      lw = lamP[3 * N + x];
+      lp = lamP[4 * N + x];
+    }
   }
   if (flags & kRhsViscous) {
     int i, j, k;
@@ -518,10 +551,8 @@ __global__ void k_adj_final(const double* __restrict__ q, T* lamP, const T* __re
     if (flags & kRhsInvscd) {
       const double iv = 1.0 / (e.next_vol[x] + 1e-300);
 #pragma unroll
-      for (int f = 0; f < 5; ++f) {
-        lam_vol[f * N + x] = o1[f] * iv;
-        lamP[f * N + x] = T(0);
-      }
+      for (int f = 0; f < 5; ++f) lam_vol[f * N + x] = o1[f] * iv;
+      clear_sums<T>(lamP, N, x);
     }
   }
 }
@@ -550,7 +581,7 @@ __global__ void k_ke_grad(const double* __restrict__ q, const double* __restrict
 
 template <typename T>
 size_t vjp_ws(int64_t N) {
-  return ((kPVals<T> + 5 + 12 + 4) * (size_t)N) * sizeof(T) + 5 * (size_t)N * sizeof(double) + 5 * 256;
+  return ((kPVals<T> + kLamVals<T> + 12 + 4) * (size_t)N) * sizeof(T) + 5 * (size_t)N * sizeof(double) + 5 * 256;
 }
 
 template <typename T>
@@ -563,28 +594,32 @@ int rhs_vjp_impl(fj_ctx* ctx, const double* q, const double* kxyz, const double*
   T* P = (T*)p;
   p = al(p + kPVals<T> * (size_t)N * sizeof(T));
   T* lamP = (T*)p;
-  p = al(p + 5 * (size_t)N * sizeof(T));
+  p = al(p + kLamVals<T> * (size_t)N * sizeof(T));
   T* lamD = (T*)p;
   p = al(p + 12 * (size_t)N * sizeof(T));
   T* lamL = (T*)p;
   p = al(p + 4 * (size_t)N * sizeof(T));
   double* lv = (double*)p;
-  const ADims d{ni, nj, nk};
+  ADims d{ni, nj, nk, {}, {}};
+  d.dk.init((uint32_t)nk);
+  d.dj.init((uint32_t)nj);
   const int grid = grid_for(N, kAT);
   const bool inv = (flags & kRhsInvscd) != 0;
   if (!(epi && epi->ws_ready)) {
-    k_adj_prims<T><<<grid, kAT, 0, st>>>(q, P, N, ph.gm1, ph.R, lam, vol, inv ? lv : nullptr, inv ? lamP : nullptr);
+    pdl_launch(k_adj_prims<T>, grid, kAT, 0, st, q, P, N, ph.gm1, ph.R, lam, vol, inv ? lv : nullptr,
+               inv ? lamP : nullptr);
     ctx->launches += 1;
   }
   int rest = flags;  // the parts still to launch
   if constexpr (sizeof(T) == 4) {
     if (ctx->adj_variant == 0 && (flags & kRhsInvscd) && (flags & kRhsViscous)) {
-      // FP32 default: both VJPs in one launch (80 registers, 3 CTAs of 256 per
+      // FP32 default: both VJPs in one launch (96 registers, 5 CTAs of 128 per
       // SM).  FP64 keeps two launches: its face VJP is bound by the FP64 pipe at
       // the 128-register cap, and the fused form (128 x 4) measured 4 % slower
       // on the reverse sweep
-      k_adj_faces_visc<T, kAT, 3><<<4 * (unsigned)grid, kAT, 0, st>>>(P, kxyz, lv, lamP, lam, lamD, lamL, d, ph,
-                                                                     dmu, mu_scale);
+      constexpr int nt = 128;
+      pdl_launch(k_adj_faces_visc<T, nt, 5>, 4 * (unsigned)((N + nt - 1) / nt), nt, 0, st, P, kxyz, lv, lamP, lam,
+                 lamD, lamL, d, ph, dmu, mu_scale);
       ctx->launches += 1;
       rest &= ~(kRhsInvscd | kRhsViscous);
     }
@@ -595,7 +630,7 @@ int rhs_vjp_impl(fj_ctx* ctx, const double* q, const double* kxyz, const double*
     // B200 (TGV 96^3 adjoint sweep): FP64 128 x 4 (128 registers), FP32
     // 256 x 3 (80 registers, a few spilled values)
     auto launch = [&](auto kern, int nt) {
-      kern<<<dim3((unsigned)((N + nt - 1) / nt), 3), nt, 0, st>>>(P, kxyz, lv, lamP, d, ph);
+      pdl_launch(kern, dim3((unsigned)((N + nt - 1) / nt), 3), nt, 0, st, P, kxyz, lv, lamP, d, ph);
     };
     constexpr bool f64 = sizeof(T) == 8;
     switch (ctx->adj_variant) {
@@ -614,12 +649,13 @@ int rhs_vjp_impl(fj_ctx* ctx, const double* q, const double* kxyz, const double*
   if (rest & kRhsViscous) {
     // variants 0 and 2 cap the viscous VJP at 64 registers (4 CTAs per SM)
     if (ctx->adj_variant == 0 || ctx->adj_variant == 2)
-      k_adj_visc<T, 4><<<grid, kAT, 0, st>>>(P, kxyz, lam, lamD, lamL, d, ph, dmu, mu_scale);
+      pdl_launch(k_adj_visc<T, 4>, grid, kAT, 0, st, P, kxyz, lam, lamD, lamL, d, ph, dmu, mu_scale);
     else
-      k_adj_visc<T><<<grid, kAT, 0, st>>>(P, kxyz, lam, lamD, lamL, d, ph, dmu, mu_scale);
+      pdl_launch(k_adj_visc<T, 1>, grid, kAT, 0, st, P, kxyz, lam, lamD, lamL, d, ph, dmu, mu_scale);
     ctx->launches += 1;
   }
-  k_adj_final<T><<<grid, kAT, 0, st>>>(q, lamP, lamD, lamL, out, P, lv, d, ph, flags, epi ? *epi : VjpEpilogue{});
+  pdl_launch(k_adj_final<T>, grid, kAT, 0, st, q, lamP, lamD, lamL, out, P, lv, d, ph, flags,
+             epi ? *epi : VjpEpilogue{});
   ctx->launches += 1;
   return launch_status(ctx, "rhs vjp launch");
 }

@@ -14,37 +14,39 @@ template <typename T> __device__ __forceinline__ T dsign(T x) {
   return x > T(0) ? T(1) : (x < T(0) ? T(-1) : T(0));
 }
 
-// Reverse of muscl2_fast for one variable: lamL, lamR -> lamc[0..3] (added).
+// Reverse of muscl2_fast for one variable: lamL, lamR -> lamc[0..3] (set).
 template <typename T>
 __device__ __forceinline__ void muscl2_vjp(T c0, T c1, T c2, T c3, int limiter, T lamL, T lamR,
                                            T lamc[4]) {
   const T d0 = c1 - c0, d1 = c2 - c1, d2 = c3 - c2;
-  // partials of lim(a, b) wrt a and b
-  T pa0, pb0, pa1, pb1;
-  if (limiter == 0) {  // minmod: picks a when a*b > 0 and |a| < |b|, b when a*b > 0 otherwise
-    const bool s0 = d0 * d1 > T(0), s1 = d1 * d2 > T(0);
-    const bool a0 = fj_abs(d0) < fj_abs(d1), a1 = fj_abs(d1) < fj_abs(d2);
-    pa0 = (s0 && a0) ? T(1) : T(0);
-    pb0 = (s0 && !a0) ? T(1) : T(0);
-    pa1 = (s1 && a1) ? T(1) : T(0);
-    pb1 = (s1 && !a1) ? T(1) : T(0);
-  } else {  // van Leer 2ab/(a+b) where ab > 0
-    const bool s0 = d0 * d1 > T(0), s1 = d1 * d2 > T(0);
-    const T e0 = d0 + d1, e1 = d1 + d2;
-    pa0 = s0 ? T(2) * d1 * d1 / (e0 * e0) : T(0);
-    pb0 = s0 ? T(2) * d0 * d0 / (e0 * e0) : T(0);
-    pa1 = s1 ? T(2) * d2 * d2 / (e1 * e1) : T(0);
-    pb1 = s1 ? T(2) * d1 * d1 / (e1 * e1) : T(0);
-  }
   // L = c1 + 0.5 sL(d0, d1); R = c2 - 0.5 sR(d1, d2)
   const T lsL = T(0.5) * lamL, lsR = T(-0.5) * lamR;
-  const T ld0 = lsL * pa0;
-  const T ld1 = lsL * pb0 + lsR * pa1;
-  const T ld2 = lsR * pb1;
-  lamc[0] += -ld0;
-  lamc[1] += lamL + ld0 - ld1;
-  lamc[2] += lamR + ld1 - ld2;
-  lamc[3] += ld2;
+  const bool s0 = d0 * d1 > T(0), s1 = d1 * d2 > T(0);
+  if (limiter == 0) {
+    // minmod is its smaller argument where the signs agree: the slope's adjoint
+    // goes to that one (selections, no 0/1 weights to multiply by)
+    const bool a0 = fj_abs(d0) < fj_abs(d1), a1 = fj_abs(d1) < fj_abs(d2);
+    const T ld0 = s0 && a0 ? lsL : T(0);
+    const T ld1 = (s0 && !a0 ? lsL : T(0)) + (s1 && a1 ? lsR : T(0));
+    const T ld2 = s1 && !a1 ? lsR : T(0);
+    lamc[0] = -ld0;
+    lamc[1] = lamL + ld0 - ld1;
+    lamc[2] = lamR + ld1 - ld2;
+    lamc[3] = ld2;
+  } else {  // van Leer 2ab/(a+b) where ab > 0
+    const T e0 = d0 + d1, e1 = d1 + d2;
+    const T pa0 = s0 ? T(2) * d1 * d1 / (e0 * e0) : T(0);
+    const T pb0 = s0 ? T(2) * d0 * d0 / (e0 * e0) : T(0);
+    const T pa1 = s1 ? T(2) * d2 * d2 / (e1 * e1) : T(0);
+    const T pb1 = s1 ? T(2) * d1 * d1 / (e1 * e1) : T(0);
+    const T ld0 = lsL * pa0;
+    const T ld1 = lsL * pb0 + lsR * pa1;
+    const T ld2 = lsR * pb1;
+    lamc[0] = -ld0;
+    lamc[1] = lamL + ld0 - ld1;
+    lamc[2] = lamR + ld1 - ld2;
+    lamc[3] = ld2;
+  }
 }
 
 // Reverse of roe_prim: lamF (5) -> lamL, lamR (primitive face states, set).
@@ -59,12 +61,12 @@ __device__ __forceinline__ void roe_prim_vjp(const Prim<T>& L, const Prim<T>& R,
   const T keL = T(0.5) * (L.u * L.u + L.v * L.v + L.w * L.w);
   const T keR = T(0.5) * (R.u * R.u + R.v * R.v + R.w * R.w);
   const T EL = L.p * ig + L.rho * keL, ER = R.p * ig + R.rho * keR;
-  const T irL = M::rcp(rhoL), irR = M::rcp(rhoR);
+  const T irL = M::rcp_n(rhoL), irR = M::rcp_n(rhoR);
   const T HL = (EL + L.p) * irL, HR = (ER + R.p) * irR;
-  const T sqL = M::sqrt_pos(rhoL), sqR = M::sqrt_pos(rhoR);
+  const T sqL = M::sqrt_n(rhoL), sqR = M::sqrt_n(rhoR);
   const T ssum = sqL + sqR;
   const bool css = ssum > Tiny<T>::ss();
-  const T iss = M::rcp(css ? ssum : Tiny<T>::ss());
+  const T iss = M::rcp_n(css ? ssum : Tiny<T>::ss());
   const T wl = sqL * iss, wr = sqR * iss;
   const T uh = wl * L.u + wr * R.u, vh = wl * L.v + wr * R.v, wh = wl * L.w + wr * R.w;
   const T Hh = wl * HL + wr * HR;
@@ -72,12 +74,12 @@ __device__ __forceinline__ void roe_prim_vjp(const Prim<T>& L, const Prim<T>& R,
   const T c2r = gm1 * (Hh - T(0.5) * q2);
   const bool cc2 = c2r > Tiny<T>::c2();
   const T c2 = cc2 ? c2r : Tiny<T>::c2();
-  const T ch = M::sqrt_pos(c2);
-  const T ic2 = M::rcp(c2);
+  const T ch = M::sqrt_n(c2);
+  const T ic2 = M::rcp_n(c2);
   const T unh = uh * n0 + vh * n1 + wh * n2;
   const T rhoh = sqL * sqR;
   const T eps = eps_e * (fj_abs(unh) + ch);
-  const T ieps = M::rcp(eps);
+  const T ieps = M::rcp_n(eps);
   const T lam1 = unh - ch, lam5 = unh + ch;
   const bool h1 = fj_abs(lam1) >= eps, h5 = fj_abs(lam5) >= eps;
   const T al1 = h1 ? fj_abs(lam1) : T(0.5) * (lam1 * lam1 * ieps + eps);
@@ -334,12 +336,12 @@ __device__ __forceinline__ void roe_prim_vjp(const Prim<T>& L, const Prim<T>& R,
   lR.p = lpR;
 }
 
-// Reverse of invscd_face_fast: lamF (5, on the |n|-scaled flux) -> lamc[4]
-// (primitives of the four cells, added).
+// Reverse of invscd_face_fast: lamF (5, on the |n|-scaled flux) -> lc[s][v], the
+// adjoint of the primitive v (rho, u, v, w, p) of cell s of the four (set).
 template <typename T>
 __device__ __forceinline__ void invscd_face_vjp(const Prim<T> c[4], T kl0, T kl1, T kl2, T kr0, T kr1,
                                                 T kr2, T gm1, T ig, T eps_e, int limiter,
-                                                const T lamF[5], Prim<T> lamc[4]) {
+                                                const T lamF[5], T lc[4][5]) {
   Prim<T> L, R;
   muscl2_fast(c[0].rho, c[1].rho, c[2].rho, c[3].rho, limiter, L.rho, R.rho);
   muscl2_fast(c[0].u, c[1].u, c[2].u, c[3].u, limiter, L.u, R.u);
@@ -348,25 +350,24 @@ __device__ __forceinline__ void invscd_face_vjp(const Prim<T> c[4], T kl0, T kl1
   muscl2_fast(c[0].p, c[1].p, c[2].p, c[3].p, limiter, L.p, R.p);
   const T nf0 = T(0.5) * (kl0 + kr0), nf1 = T(0.5) * (kl1 + kr1), nf2 = T(0.5) * (kl2 + kr2);
   const T nmag = FastMath<T>::sqrt_nn(nf0 * nf0 + nf1 * nf1 + nf2 * nf2) + Tiny<T>::nmag();
-  const T inv = FastMath<T>::rcp(nmag);
+  const T inv = FastMath<T>::rcp_n(nmag);
   T g[5];
 #pragma unroll
   for (int v = 0; v < 5; ++v) g[v] = lamF[v] * nmag;  // F_out = nmag F
   Prim<T> lL, lR;
   roe_prim_vjp(L, R, nf0 * inv, nf1 * inv, nf2 * inv, gm1, ig, eps_e, g, lL, lR);
-  T lc[4];
-#define FJ_MUSCL_VJP(field)                                                                    \
-  lc[0] = lc[1] = lc[2] = lc[3] = T(0);                                                        \
-  muscl2_vjp(c[0].field, c[1].field, c[2].field, c[3].field, limiter, lL.field, lR.field, lc); \
-  lamc[0].field += lc[0];                                                                      \
-  lamc[1].field += lc[1];                                                                      \
-  lamc[2].field += lc[2];                                                                      \
-  lamc[3].field += lc[3];
-  FJ_MUSCL_VJP(rho)
-  FJ_MUSCL_VJP(u)
-  FJ_MUSCL_VJP(v)
-  FJ_MUSCL_VJP(w)
-  FJ_MUSCL_VJP(p)
+  T o[4];
+#define FJ_MUSCL_VJP(field, v)                                                                \
+  muscl2_vjp(c[0].field, c[1].field, c[2].field, c[3].field, limiter, lL.field, lR.field, o); \
+  lc[0][v] = o[0];                                                                            \
+  lc[1][v] = o[1];                                                                            \
+  lc[2][v] = o[2];                                                                            \
+  lc[3][v] = o[3];
+  FJ_MUSCL_VJP(rho, 0)
+  FJ_MUSCL_VJP(u, 1)
+  FJ_MUSCL_VJP(v, 2)
+  FJ_MUSCL_VJP(w, 3)
+  FJ_MUSCL_VJP(p, 4)
 #undef FJ_MUSCL_VJP
 }
 

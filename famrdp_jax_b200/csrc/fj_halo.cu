@@ -536,7 +536,8 @@ namespace {
 
 // A target cell's value after the fill comes from its last writer's source
 // cell; the cell's own original value is discarded.
-__device__ __forceinline__ bool later_link_covers(const HaloTable& tab, int L, int ti, int tj, int tk) {
+template <int NL>
+__device__ __forceinline__ bool later_link_covers(const HaloTableN<NL>& tab, int L, int ti, int tj, int tk) {
   const HaloDesc& d = tab.d[L];
   for (int L2 = L + 1; L2 < tab.n; ++L2) {
     if (tab.d[L2].tgt_block == d.tgt_block && slab_covers(tab.d[L2], ti, tj, tk)) return true;
@@ -544,9 +545,12 @@ __device__ __forceinline__ bool later_link_covers(const HaloTable& tab, int L, i
   return false;
 }
 
-// pass 0: scratch := lam at last-writer target cells (else 0); pass 1: zero
-// every target cell; pass 2: lam[source] += scratch.
-__global__ void k_halo_transpose(const HaloTable tab, double* __restrict__ scratch, int pass) {
+// TAKE: scratch := lam at last-writer target cells (else 0), and those cells :=
+// 0 (each target cell has one last writer, and only its thread touches it);
+// else lam[source] += scratch.
+template <bool TAKE, int NL>
+__global__ void k_halo_transpose(const HaloTableN<NL> tab, double* __restrict__ scratch) {
+  grid_dep_wait();
   const int L = blockIdx.y;
   const HaloDesc& d = tab.d[L];
   const int64_t V = (int64_t)d.ext[0] * d.ext[1] * d.ext[2];
@@ -556,18 +560,17 @@ __global__ void k_halo_transpose(const HaloTable tab, double* __restrict__ scrat
   double* src = const_cast<double*>(d.src);
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < V;
        r += (int64_t)gridDim.x * blockDim.x) {
-    const int c = (int)(r % d.ext[2]);
-    const int b = (int)((r / d.ext[2]) % d.ext[1]);
-    const int a = (int)(r / ((int64_t)d.ext[2] * d.ext[1]));
-    const int ti = d.tlo[0] + a, tj = d.tlo[1] + b, tk = d.tlo[2] + c;
-    const int64_t tc = cell_index(d.tn, ti, tj, tk);
-    if (pass == 0) {
+    int a, b, c;
+    slab_coords(d, r, a, b, c);
+    if constexpr (TAKE) {
+      const int ti = d.tlo[0] + a, tj = d.tlo[1] + b, tk = d.tlo[2] + c;
+      const int64_t tc = cell_index(d.tn, ti, tj, tk);
       const bool last = !later_link_covers(tab, L, ti, tj, tk);
 #pragma unroll
       for (int v = 0; v < 5; ++v) scratch[d.off + v * V + r] = last ? tgt[v * NT + tc] : 0.0;
-    } else if (pass == 1) {
+      if (last)
 #pragma unroll
-      for (int v = 0; v < 5; ++v) tgt[v * NT + tc] = 0.0;
+        for (int v = 0; v < 5; ++v) tgt[v * NT + tc] = 0.0;
     } else {
       const int64_t sc = d.s0 + a * d.sstr[0] + b * d.sstr[1] + c * d.sstr[2];
 #pragma unroll
@@ -579,6 +582,7 @@ __global__ void k_halo_transpose(const HaloTable tab, double* __restrict__ scrat
 // Transpose of one face's farfield (lam(outer) := 0) or mirror BC
 // (lam(inner) += s lam(outer); lam(outer) := 0).
 __global__ void k_bc_transpose(const BcTable tab, int g) {
+  grid_dep_wait();
   const BcDesc& d = tab.d[blockIdx.y];
   const int ax = d.face >> 1;
   const int oa = ax == 0 ? 1 : 0, ob = ax == 2 ? 1 : 2;
@@ -635,13 +639,20 @@ int halo_transpose(fj_ctx* ctx, const fj_block* lam, int nblocks, const fj_link*
     vmax = std::max<int64_t>(vmax, (int64_t)tab.d[t].ext[0] * tab.d[t].ext[1] * tab.d[t].ext[2]);
   }
   dim3 grid((unsigned)std::min<int64_t>(grid_for(vmax), 4096), tab.n);
-  for (int pass = 0; pass < 3; ++pass) {
-    k_halo_transpose<<<grid, kThreads, 0, st>>>(tab, scratch, pass);
-    ctx->launches += 1;
-    s = launch_status(ctx, "halo transpose launch");
-    if (s != FJ_OK) return s;
+  auto launch = [&](const auto& t, auto take, auto give) {
+    pdl_launch(take, grid, kThreads, 0, st, t, scratch);
+    pdl_launch(give, grid, kThreads, 0, st, t, scratch);
+  };
+  if (tab.n <= 6) {  // a block's own faces: 0.7 KB of parameters instead of 21
+    HaloTable1 t;
+    t.n = tab.n;
+    for (int L = 0; L < tab.n; ++L) t.d[L] = tab.d[L];
+    launch(t, k_halo_transpose<true, 6>, k_halo_transpose<false, 6>);
+  } else {
+    launch(tab, k_halo_transpose<true, kMaxLinksPerLaunch>, k_halo_transpose<false, kMaxLinksPerLaunch>);
   }
-  return FJ_OK;
+  ctx->launches += 2;
+  return launch_status(ctx, "halo transpose launch");
 }
 
 int bc_transpose(fj_ctx* ctx, const fj_block* lam, int nblocks, const fj_bc* bcs, int nbcs,
@@ -679,7 +690,7 @@ int bc_transpose(fj_ctx* ctx, const fj_block* lam, int nblocks, const fj_bc* bcs
         vmax = std::max<int64_t>(vmax, (int64_t)tab.d[t].n[0] * tab.d[t].n[1] * tab.d[t].n[2] / tab.d[t].n[ax]);
       }
       dim3 grid((unsigned)std::min<int64_t>(grid_for(vmax), 4096), tab.n);
-      k_bc_transpose<<<grid, kThreads, 0, st>>>(tab, p->ghost);
+      pdl_launch(k_bc_transpose, grid, kThreads, 0, st, tab, p->ghost);
       ctx->launches += 1;
       int s = launch_status(ctx, "bc transpose launch");
       if (s != FJ_OK) return s;

@@ -15,14 +15,13 @@ template <typename T> __device__ __forceinline__ T dsign(T x) {
 }
 
 // Reverse of muscl2_fast for one variable: lamL, lamR -> lamc[0..3] (set).
-template <typename T>
-__device__ __forceinline__ void muscl2_vjp(T c0, T c1, T c2, T c3, int limiter, T lamL, T lamR,
-                                           T lamc[4]) {
+template <typename T, bool MINMOD>
+__device__ __forceinline__ void muscl2_vjp(T c0, T c1, T c2, T c3, T lamL, T lamR, T lamc[4]) {
   const T d0 = c1 - c0, d1 = c2 - c1, d2 = c3 - c2;
   // L = c1 + 0.5 sL(d0, d1); R = c2 - 0.5 sR(d1, d2)
   const T lsL = T(0.5) * lamL, lsR = T(-0.5) * lamR;
   const bool s0 = d0 * d1 > T(0), s1 = d1 * d2 > T(0);
-  if (limiter == 0) {
+  if constexpr (MINMOD) {
     // minmod is its smaller argument where the signs agree: the slope's adjoint
     // goes to that one (selections, no 0/1 weights to multiply by)
     const bool a0 = fj_abs(d0) < fj_abs(d1), a1 = fj_abs(d1) < fj_abs(d2);
@@ -343,11 +342,7 @@ __device__ __forceinline__ void invscd_face_vjp(const Prim<T> c[4], T kl0, T kl1
                                                 T kr2, T gm1, T ig, T eps_e, int limiter,
                                                 const T lamF[5], T lc[4][5]) {
   Prim<T> L, R;
-  muscl2_fast(c[0].rho, c[1].rho, c[2].rho, c[3].rho, limiter, L.rho, R.rho);
-  muscl2_fast(c[0].u, c[1].u, c[2].u, c[3].u, limiter, L.u, R.u);
-  muscl2_fast(c[0].v, c[1].v, c[2].v, c[3].v, limiter, L.v, R.v);
-  muscl2_fast(c[0].w, c[1].w, c[2].w, c[3].w, limiter, L.w, R.w);
-  muscl2_fast(c[0].p, c[1].p, c[2].p, c[3].p, limiter, L.p, R.p);
+  muscl2_fast(c, limiter, L, R);
   const T nf0 = T(0.5) * (kl0 + kr0), nf1 = T(0.5) * (kl1 + kr1), nf2 = T(0.5) * (kl2 + kr2);
   const T nmag = FastMath<T>::sqrt_nn(nf0 * nf0 + nf1 * nf1 + nf2 * nf2) + Tiny<T>::nmag();
   const T inv = FastMath<T>::rcp_n(nmag);
@@ -357,17 +352,19 @@ __device__ __forceinline__ void invscd_face_vjp(const Prim<T> c[4], T kl0, T kl1
   Prim<T> lL, lR;
   roe_prim_vjp(L, R, nf0 * inv, nf1 * inv, nf2 * inv, gm1, ig, eps_e, g, lL, lR);
   T o[4];
-#define FJ_MUSCL_VJP(field, v)                                                                \
-  muscl2_vjp(c[0].field, c[1].field, c[2].field, c[3].field, limiter, lL.field, lR.field, o); \
-  lc[0][v] = o[0];                                                                            \
-  lc[1][v] = o[1];                                                                            \
-  lc[2][v] = o[2];                                                                            \
+#define FJ_MUSCL_VJP(K, field, v)                                                                \
+  muscl2_vjp<T, K>(c[0].field, c[1].field, c[2].field, c[3].field, lL.field, lR.field, o);       \
+  lc[0][v] = o[0];                                                                               \
+  lc[1][v] = o[1];                                                                               \
+  lc[2][v] = o[2];                                                                               \
   lc[3][v] = o[3];
-  FJ_MUSCL_VJP(rho, 0)
-  FJ_MUSCL_VJP(u, 1)
-  FJ_MUSCL_VJP(v, 2)
-  FJ_MUSCL_VJP(w, 3)
-  FJ_MUSCL_VJP(p, 4)
+  if (limiter == 0) {
+    FJ_MUSCL_VJP(true, rho, 0) FJ_MUSCL_VJP(true, u, 1) FJ_MUSCL_VJP(true, v, 2)
+    FJ_MUSCL_VJP(true, w, 3) FJ_MUSCL_VJP(true, p, 4)
+  } else {
+    FJ_MUSCL_VJP(false, rho, 0) FJ_MUSCL_VJP(false, u, 1) FJ_MUSCL_VJP(false, v, 2)
+    FJ_MUSCL_VJP(false, w, 3) FJ_MUSCL_VJP(false, p, 4)
+  }
 #undef FJ_MUSCL_VJP
 }
 

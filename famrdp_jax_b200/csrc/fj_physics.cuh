@@ -258,29 +258,62 @@ template <typename T> __device__ __forceinline__ T minmod_sel(T a, T b) {
   return a * b > T(0) ? m : T(0);
 }
 
-template <typename T>
-__device__ __forceinline__ void muscl2_fast(T c0, T c1, T c2, T c3, int limiter, T& L, T& R) {
+// MINMOD: the limiter, else van Leer.
+template <typename T, bool MINMOD>
+__device__ __forceinline__ void muscl2_one(T c0, T c1, T c2, T c3, T& L, T& R) {
   const T d0 = c1 - c0, d1 = c2 - c1, d2 = c3 - c2;
   T sL, sR;
-  if (limiter == 0) {
-    if constexpr (sizeof(T) == 4) {
-      // minmod(d, d1) clamps d to the interval between 0 and d1, which both
-      // slopes share: six min/max instead of two products, four comparisons
-      // and four selections (the same values; where |d d1| underflows, the
-      // smaller magnitude instead of 0, as the reference)
-      const T lo = fj_min(d1, T(0)), hi = fj_max(d1, T(0));
-      sL = fj_min(fj_max(d0, lo), hi);
-      sR = fj_min(fj_max(d2, lo), hi);
-    } else {
-      sL = minmod_sel(d0, d1);
-      sR = minmod_sel(d1, d2);
-    }
-  } else {
+  if constexpr (!MINMOD) {
     sL = vanleer(d0, d1);
     sR = vanleer(d1, d2);
+  } else if constexpr (sizeof(T) == 4) {
+    // minmod(d, d1) clamps d to the interval between 0 and d1, which both
+    // slopes share: six min/max instead of two products, four comparisons
+    // and four selections (the same values; where |d d1| underflows, the
+    // smaller magnitude instead of 0, as the reference)
+    const T lo = fj_min(d1, T(0)), hi = fj_max(d1, T(0));
+    sL = fj_min(fj_max(d0, lo), hi);
+    sR = fj_min(fj_max(d2, lo), hi);
+  } else {
+    // picks the outer difference where it is smaller than the face's own d1, and
+    // 0 where the signs differ; the sign test reads the sign bits (a zero argument
+    // gives 0 either way), which keeps a multiplication and a comparison off the
+    // FP64 pipe.  A NaN outer difference loses the comparison, so it reaches no
+    // face whose own two cells are finite.
+    const auto pick = [&](T o) {
+      const T m = fj_abs(o) < fj_abs(d1) ? o : d1;
+      return (__double2hiint(o) ^ __double2hiint(d1)) < 0 ? T(0) : m;
+    };
+    sL = pick(d0);
+    sR = pick(d2);
   }
   L = c1 + T(0.5) * sL;
   R = c2 - T(0.5) * sR;
+}
+
+// The face states of all five variables.  FP64 tests the limiter once, so that the
+// variables' arithmetic is one straight run of instructions (FP64 step of 4.0 M
+// cells 1.776 -> 1.751 ms).  FP32 tests it per variable: in one run the compiler
+// fuses the states' last operations into the flux, which changes its rounding and
+// gains nothing.
+template <typename T>
+__device__ __forceinline__ void muscl2_fast(const Prim<T> c[4], int limiter, Prim<T>& L, Prim<T>& R) {
+#define FJ_MUSCL(K, f) muscl2_one<T, K>(c[0].f, c[1].f, c[2].f, c[3].f, L.f, R.f);
+#define FJ_MUSCL_TEST(f)       \
+  if (limiter == 0) {          \
+    FJ_MUSCL(true, f)          \
+  } else {                     \
+    FJ_MUSCL(false, f)         \
+  }
+  if constexpr (sizeof(T) == 4) {
+    FJ_MUSCL_TEST(rho) FJ_MUSCL_TEST(u) FJ_MUSCL_TEST(v) FJ_MUSCL_TEST(w) FJ_MUSCL_TEST(p)
+  } else if (limiter == 0) {
+    FJ_MUSCL(true, rho) FJ_MUSCL(true, u) FJ_MUSCL(true, v) FJ_MUSCL(true, w) FJ_MUSCL(true, p)
+  } else {
+    FJ_MUSCL(false, rho) FJ_MUSCL(false, u) FJ_MUSCL(false, v) FJ_MUSCL(false, w) FJ_MUSCL(false, p)
+  }
+#undef FJ_MUSCL_TEST
+#undef FJ_MUSCL
 }
 
 // Roe flux (flux/roe.py:21-85) of the primitive face states L, R along the unit
@@ -399,32 +432,6 @@ __device__ __forceinline__ void roe_prim(const Prim<T>& L, const Prim<T>& R, T n
          T(0.5) * (s1 * (H_h - cun) + s5 * (H_h + cun) + al2 * (a23 * (T(0.5) * q2) + t4));
 }
 
-// MUSCL-2 of one variable in FP64.  minmod of the face's own difference d1 with
-// an outer one picks the outer difference where it is smaller, and 0 where the
-// signs differ; the sign test reads the sign bits (a zero argument gives 0
-// either way), which keeps a multiplication and a comparison off the FP64 pipe.
-// A NaN outer difference loses the comparison, so it reaches no face whose
-// own two cells are finite.
-__device__ __forceinline__ double minmod_outer(double outer, double d1) {
-  const double m = fabs(outer) < fabs(d1) ? outer : d1;
-  return (__double2hiint(outer) ^ __double2hiint(d1)) < 0 ? 0.0 : m;
-}
-
-__device__ __forceinline__ void muscl2_f64(double c0, double c1, double c2, double c3, int limiter, double& L,
-                                           double& R) {
-  const double d0 = c1 - c0, d1 = c2 - c1, d2 = c3 - c2;
-  double sL, sR;
-  if (limiter == 0) {
-    sL = minmod_outer(d0, d1);
-    sR = minmod_outer(d2, d1);
-  } else {
-    sL = vanleer(d0, d1);
-    sR = vanleer(d1, d2);
-  }
-  L = c1 + 0.5 * sL;
-  R = c2 - 0.5 * sR;
-}
-
 // 1/x and 1/sqrt(x) in FP64 for a normal, finite x (whose result is normal too):
 // the hardware's seed (relative error 1e-6, measured) and one third-order Newton
 // step, y (1 + e + e^2) with e = 1 - x y, and y (1 + e/2 + 3 e^2/8) with
@@ -526,20 +533,11 @@ __device__ __forceinline__ void invscd_face_fast(const Prim<T> c[4], T kl0, T kl
                                                  T kr1, T kr2, T gm1, T inv_gm1, T eps_entropy,
                                                  int limiter, T F[5], T p_ref = T(0)) {
   Prim<T> L, R;
+  muscl2_fast(c, limiter, L, R);
   if constexpr (sizeof(T) == 8 && !POFF) {
-    muscl2_f64(c[0].rho, c[1].rho, c[2].rho, c[3].rho, limiter, L.rho, R.rho);
-    muscl2_f64(c[0].u, c[1].u, c[2].u, c[3].u, limiter, L.u, R.u);
-    muscl2_f64(c[0].v, c[1].v, c[2].v, c[3].v, limiter, L.v, R.v);
-    muscl2_f64(c[0].w, c[1].w, c[2].w, c[3].w, limiter, L.w, R.w);
-    muscl2_f64(c[0].p, c[1].p, c[2].p, c[3].p, limiter, L.p, R.p);
     roe_face_f64(L, R, 0.5 * (kl0 + kr0), 0.5 * (kl1 + kr1), 0.5 * (kl2 + kr2), gm1, inv_gm1, eps_entropy, F);
     return;
   }
-  muscl2_fast(c[0].rho, c[1].rho, c[2].rho, c[3].rho, limiter, L.rho, R.rho);
-  muscl2_fast(c[0].u, c[1].u, c[2].u, c[3].u, limiter, L.u, R.u);
-  muscl2_fast(c[0].v, c[1].v, c[2].v, c[3].v, limiter, L.v, R.v);
-  muscl2_fast(c[0].w, c[1].w, c[2].w, c[3].w, limiter, L.w, R.w);
-  muscl2_fast(c[0].p, c[1].p, c[2].p, c[3].p, limiter, L.p, R.p);
   const T nf0 = T(0.5) * (kl0 + kr0), nf1 = T(0.5) * (kl1 + kr1), nf2 = T(0.5) * (kl2 + kr2);
   const T nmag = FastMath<T>::sqrt_nn(nf0 * nf0 + nf1 * nf1 + nf2 * nf2) + Tiny<T>::nmag();
   const T inv = FastMath<T>::rcp_n(nmag);

@@ -33,9 +33,17 @@ struct FastDiv {
   __device__ __forceinline__ uint32_t div(uint32_t n) const { return (__umulhi(n, m) + n) >> s; }
 };
 
+// The boxes of t[0] x t[1] x t[2] cells a block is cut into for k_small_stage.
+struct Tile {
+  int t[3];
+  FastDiv pk, pj;            // n / boxes along k, along j
+  FastDiv tk, tj, tk1, tj1;  // n / t[2], t[1], t[2] + 1, t[1] + 1
+};
+
 struct Dev {
   SplitBlock blk;
   FastDiv dk, dj;  // n / nk, n / nj
+  Tile tile;       // k_small_stage's boxes of this block
 };
 
 // The blocks of a launch, a kernel parameter.  TableN<1> serves launches of one
@@ -397,99 +405,108 @@ struct GlobalSrc {
       o[4] = z.y;
     }
   }
-  __device__ __forceinline__ void G_rec(int32_t c, T* o) const {
-    ld_rec<T, kRecG, NC>((const T*)B.G + (size_t)c * kRecG, o);
+  // the nine viscous components of cell nb, the neighbour of the assembled cell
+  // along axis l on side 0 (+) or 1 (-)
+  __device__ __forceinline__ void G_nb(int, int, int32_t nb, T* o) const {
+    ld_rec<T, kRecG, NC>((const T*)B.G + (size_t)nb * kRecG, o);
+    o[8] = ((const T*)B.Gz)[nb];
   }
   __device__ __forceinline__ void K9(int32_t c, T* kk, T* gcl) const { metric9<T, K_AOS>(B, N, c, kk, gcl); }
 };
 
-// The assembly of one cell (rhs/invscd.py:119-131, rhs/viscous.py:86-117,
-// solver/step.py:45-53) from the intermediates Src provides.
+// The assembly of one cell in three parts, from the intermediates Src provides.
+// The inviscid part of the RHS (rhs/invscd.py:119-131).
 // fk_m / fk_p: the k faces c-1 | c and c | c+1 (the flux records hold only the
-// i and j faces); kk / gcl: the metric record of c, loaded by the caller.
-template <typename T, bool K_AOS, class Src, class SP>
-__device__ __forceinline__ void assemble_cell(const SplitBlock& B, const SP& sp, const Cell& x, const Src& src,
-                                              int flags,
-                                              int stage, int next_prims, double gm1, double R, double iR,
-                                              double ph_p_ref, const T fk_m[5], const T fk_p[5], const T kk[9],
-                                              const T gcl[3]) {
-  const int32_t N = (int32_t)x.N, c = (int32_t)x.c;
-  const int32_t si = x.nj * x.nk, sj = x.nk;
+// i and j faces); gcl: of the metric record of c, loaded by the caller.
+template <typename T, bool K_AOS, class Src>
+__device__ __forceinline__ void assemble_inv(const SplitBlock& B, const Cell& x, const Src& src, double ph_p_ref,
+                                             const T fk_m[5], const T fk_p[5], const T gcl[3], double r[5]) {
+  const int32_t c = (int32_t)x.c;
   const int n[3] = {x.ni, x.nj, x.nk};
   const int idx[3] = {x.i, x.j, x.k};
-  const int32_t st[3] = {si, sj, 1};
-  double r[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-  if (flags & kRhsInvscd) {
-    const bool on[3] = {idx[0] >= 2 && idx[0] <= n[0] - 3, idx[1] >= 2 && idx[1] <= n[1] - 3,
-                        idx[2] >= 2 && idx[2] <= n[2] - 3};
-    if (on[0] || on[1] || on[2]) {
-      const double ivd = __drcp_rn(B.vol[c] + 1e-300);
-      T Fc[kRecF];
-      src.F_rec(c, Fc);
+  const int32_t st[3] = {x.nj * x.nk, x.nk, 1};
+  const bool on[3] = {idx[0] >= 2 && idx[0] <= n[0] - 3, idx[1] >= 2 && idx[1] <= n[1] - 3,
+                      idx[2] >= 2 && idx[2] <= n[2] - 3};
+  if (on[0] || on[1] || on[2]) {
+    const double ivd = __drcp_rn(B.vol[c] + 1e-300);
+    T Fc[kRecF];
+    src.F_rec(c, Fc);
 #pragma unroll
-      for (int v = 0; v < 5; ++v) Fc[10 + v] = fk_p[v];
-      // the p_ref n part the face fluxes left out: p_ref times the sum over
-      // the active axes of the face-normal differences, evaluated in FP64 when
-      // the records were built
-      const double pg[3] = {ph_p_ref * (double)gcl[0], ph_p_ref * (double)gcl[1], ph_p_ref * (double)gcl[2]};
-      T Fm[3][5];
+    for (int v = 0; v < 5; ++v) Fc[10 + v] = fk_p[v];
+    // the p_ref n part the face fluxes left out: p_ref times the sum over
+    // the active axes of the face-normal differences, evaluated in FP64 when
+    // the records were built
+    const double pg[3] = {ph_p_ref * (double)gcl[0], ph_p_ref * (double)gcl[1], ph_p_ref * (double)gcl[2]};
+    T Fm[3][5];
 #pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        if (on[a] && a == 2) {
+    for (int a = 0; a < 3; ++a) {
+      if (on[a] && a == 2) {
 #pragma unroll
-          for (int v = 0; v < 5; ++v) Fm[2][v] = fk_m[v];
-        } else if (on[a]) {
-          src.F_axis(c - st[a], a, Fm[a]);
-        } else {
+        for (int v = 0; v < 5; ++v) Fm[2][v] = fk_m[v];
+      } else if (on[a]) {
+        src.F_axis(c - st[a], a, Fm[a]);
+      } else {
 #pragma unroll
-          for (int v = 0; v < 5; ++v) Fm[a][v] = T(0);
-        }
-      }
-#pragma unroll
-      for (int v = 0; v < 5; ++v) {
-        double dsum;
-        if (sizeof(T) == sizeof(double)) {
-          dsum = 0.0;  // axis by axis like the reference
-#pragma unroll
-          for (int a = 0; a < 3; ++a)
-            if (on[a]) dsum += (double)(Fc[5 * a + v] - Fm[a][v]);
-        } else {
-          T s = T(0);
-#pragma unroll
-          for (int a = 0; a < 3; ++a)
-            if (on[a]) s += Fc[5 * a + v] - Fm[a][v];
-          dsum = (double)s;
-          if (K_AOS && v >= 1 && v <= 3) dsum += pg[v - 1];
-        }
-        r[v] = -dsum * ivd;
-      }
-    }
-  }
-  if (flags & kRhsViscous) {
-    // sum_l 0.5 kxyz[l][jj] (G(c+e_l) - G(c-e_l)) per equation, one
-    // neighbour record at a time (rhs/viscous.py:86-117)
-    const T* Gz = (const T*)B.Gz;
-    T acc[4] = {T(0), T(0), T(0), T(0)};
-#pragma unroll
-    for (int l = 0; l < 3; ++l) {
-#pragma unroll
-      for (int side = 0; side < 2; ++side) {
-        const int32_t nb = side == 0 ? (idx[l] + 1 == n[l] ? c - (n[l] - 1) * st[l] : c + st[l])
-                                     : (idx[l] == 0 ? c + (n[l] - 1) * st[l] : c - st[l]);
-        const T s = side == 0 ? T(0.5) : T(-0.5);
-        T g[kRecG];
-        src.G_rec(nb, g);
-        const T gz = Gz[nb];
-        const T k0 = s * kk[3 * l], k1 = s * kk[3 * l + 1], k2 = s * kk[3 * l + 2];
-        acc[0] += g[0] * k0 + g[1] * k1 + g[2] * k2;
-        acc[1] += g[1] * k0 + g[3] * k1 + g[4] * k2;
-        acc[2] += g[2] * k0 + g[4] * k1 + g[5] * k2;
-        acc[3] += g[6] * k0 + g[7] * k1 + gz * k2;
+        for (int v = 0; v < 5; ++v) Fm[a][v] = T(0);
       }
     }
 #pragma unroll
-    for (int e = 0; e < 4; ++e) r[e + 1] += (double)acc[e];
+    for (int v = 0; v < 5; ++v) {
+      double dsum;
+      if (sizeof(T) == sizeof(double)) {
+        dsum = 0.0;  // axis by axis like the reference
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+          if (on[a]) dsum += (double)(Fc[5 * a + v] - Fm[a][v]);
+      } else {
+        T s = T(0);
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+          if (on[a]) s += Fc[5 * a + v] - Fm[a][v];
+        dsum = (double)s;
+        if (K_AOS && v >= 1 && v <= 3) dsum += pg[v - 1];
+      }
+      r[v] = -dsum * ivd;
+    }
   }
+}
+
+// The viscous divergence sum_l 0.5 kxyz[l][jj] (G(c+e_l) - G(c-e_l)) per equation,
+// one neighbour record at a time (rhs/viscous.py:86-117); kk: the metrics of c.
+template <typename T, class Src>
+__device__ __forceinline__ void assemble_visc(const Cell& x, const Src& src, const T kk[9], T acc[4]) {
+  const int32_t c = (int32_t)x.c;
+  const int n[3] = {x.ni, x.nj, x.nk};
+  const int idx[3] = {x.i, x.j, x.k};
+  const int32_t st[3] = {x.nj * x.nk, x.nk, 1};
+#pragma unroll
+  for (int e = 0; e < 4; ++e) acc[e] = T(0);
+#pragma unroll
+  for (int l = 0; l < 3; ++l) {
+#pragma unroll
+    for (int side = 0; side < 2; ++side) {
+      const int32_t nb = side == 0 ? (idx[l] + 1 == n[l] ? c - (n[l] - 1) * st[l] : c + st[l])
+                                   : (idx[l] == 0 ? c + (n[l] - 1) * st[l] : c - st[l]);
+      const T s = side == 0 ? T(0.5) : T(-0.5);
+      T g[9];
+      src.G_nb(l, side, nb, g);
+      const T k0 = s * kk[3 * l], k1 = s * kk[3 * l + 1], k2 = s * kk[3 * l + 2];
+      acc[0] += g[0] * k0 + g[1] * k1 + g[2] * k2;
+      acc[1] += g[1] * k0 + g[3] * k1 + g[4] * k2;
+      acc[2] += g[2] * k0 + g[4] * k1 + g[5] * k2;
+      acc[3] += g[6] * k0 + g[7] * k1 + g[8] * k2;
+    }
+  }
+}
+
+// The RHS (stage 0) or the RK combine (solver/step.py:45-53); with next_prims, also
+// the primitives of the stage result (the next stage's input) in place of a
+// separate k_split_prims launch.
+template <typename T, class SP>
+__device__ __forceinline__ void assemble_out(const SplitBlock& B, const SP& sp, const Cell& x, int stage,
+                                             int next_prims, double gm1, double R, double iR, double ph_p_ref,
+                                             const double r[5]) {
+  const int32_t N = (int32_t)x.N, c = (int32_t)x.c;
   double* out = sp.out() + c;
   if (stage == 0) {
 #pragma unroll
@@ -508,6 +525,22 @@ __device__ __forceinline__ void assemble_cell(const SplitBlock& B, const SP& sp,
     }
     if (next_prims) store_prim_record<T>(sp.prim_next(), (size_t)c, qn, gm1, R, iR, ph_p_ref);
   }
+}
+
+template <typename T, bool K_AOS, class Src, class SP>
+__device__ __forceinline__ void assemble_cell(const SplitBlock& B, const SP& sp, const Cell& x, const Src& src,
+                                              int flags, int stage, int next_prims, double gm1, double R, double iR,
+                                              double ph_p_ref, const T fk_m[5], const T fk_p[5], const T kk[9],
+                                              const T gcl[3]) {
+  double r[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+  if (flags & kRhsInvscd) assemble_inv<T, K_AOS>(B, x, src, ph_p_ref, fk_m, fk_p, gcl, r);
+  if (flags & kRhsViscous) {
+    T acc[4];
+    assemble_visc<T>(x, src, kk, acc);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) r[e + 1] += (double)acc[e];
+  }
+  assemble_out<T>(B, sp, x, stage, next_prims, gm1, R, iR, ph_p_ref, r);
 }
 
 // With next_prims, also writes the primitives of the stage result (the next
@@ -643,15 +676,14 @@ __device__ __forceinline__ void flux_cell(const SplitBlock& B, const void* prim,
   }
 }
 
-// The flux work of cell x split into three independent parts for the
-// role-split kernel of small FP32 tables (k_split_fluxes_roles): each part
-// loads only its own operands and writes only its own values, with the
-// same arithmetic as flux_cell (bit-identical results).
-// The viscous flux components G(c) (the record and Gz).
+// The flux work of one cell in separate parts, each loading only its own operands
+// and returning its values (k_small_stage), with the same arithmetic as
+// flux_cell (the same bits).
+// The viscous flux components G(c).
 template <typename T, bool K_AOS>
-__device__ __forceinline__ void flux_visc_part(const SplitBlock& B, const void* prim, const Cell& x,
-                                               const Phys& ph) {
-  static_assert(sizeof(T) == 4, "the role-split flux kernel is the FP32 records path");
+__device__ __forceinline__ void visc_value(const SplitBlock& B, const void* prim, const Cell& x, const Phys& ph,
+                                           T G[9]) {
+  static_assert(sizeof(T) == 4, "the FP32 records path");
   using M = FastMath<T>;
   const int32_t N = (int32_t)x.N, c = (int32_t)x.c;
   const int32_t si = x.nj * x.nk, sj = x.nk;
@@ -692,47 +724,32 @@ __device__ __forceinline__ void flux_visc_part(const SplitBlock& B, const void* 
   const T t11 = T(2) * mu * (g[1][1] - div_u * third);
   const T t12 = mu * (g[1][2] + g[2][1]);
   const T t22 = T(2) * mu * (g[2][2] - div_u * third);
-  const T rec[kRecG] = {t00, t01, t02, t11, t12, t22,
-                        C0.u * t00 + C0.v * t01 + C0.w * t02 + kappa * g[3][0],
-                        C0.u * t01 + C0.v * t11 + C0.w * t12 + kappa * g[3][1]};
-  st_rec<T, kRecG>((T*)B.G + (size_t)c * kRecG, rec);
-  ((T*)B.Gz)[c] = C0.u * t02 + C0.v * t12 + C0.w * t22 + kappa * g[3][2];
+  G[0] = t00;
+  G[1] = t01;
+  G[2] = t02;
+  G[3] = t11;
+  G[4] = t12;
+  G[5] = t22;
+  G[6] = C0.u * t00 + C0.v * t01 + C0.w * t02 + kappa * g[3][0];
+  G[7] = C0.u * t01 + C0.v * t11 + C0.w * t12 + kappa * g[3][1];
+  G[8] = C0.u * t02 + C0.v * t12 + C0.w * t22 + kappa * g[3][2];
 }
 
-// The Roe face c | c+e_AXIS for c_a in [1, n_a-3], zeros elsewhere: AXIS 0
-// (i) writes floats 0..4 of the cell's face record, AXIS 1 (j) floats 5..7
-// and the Fz pair, AXIS 2 (k) the cell's 5 values of Fk.
-template <typename T, bool K_AOS, int AXIS>
-__device__ __forceinline__ void flux_face_part(const SplitBlock& B, const void* prim, const Cell& x,
-                                               const Phys& ph) {
-  static_assert(sizeof(T) == 4, "the role-split flux kernel is the FP32 records path");
-  const int32_t N = (int32_t)x.N, c = (int32_t)x.c;
-  const int32_t sa = AXIS == 0 ? x.nj * x.nk : (AXIS == 1 ? x.nk : 1);
-  const int ia = AXIS == 0 ? x.i : (AXIS == 1 ? x.j : x.k), na = AXIS == 0 ? x.ni : (AXIS == 1 ? x.nj : x.nk);
+// The Roe face c | c+e_a (stride sa) for c_a = ia in [1, na-3], zeros elsewhere.
+template <typename T, bool K_AOS>
+__device__ __forceinline__ void face_value(const SplitBlock& B, const void* prim, int32_t N, int axis, int32_t c,
+                                           int32_t sa, int ia, int na, const Phys& ph, T F[5]) {
+  static_assert(sizeof(T) == 4, "the FP32 records path");
   const T* __restrict__ P = (const T*)prim;
-  T F[5] = {T(0), T(0), T(0), T(0), T(0)};
+#pragma unroll
+  for (int v = 0; v < 5; ++v) F[v] = T(0);
   if (ia >= 1 && ia <= na - 3) {
     const Cell6<T> A0 = load_cell<T, true>(P, c - sa), A1 = load_cell<T, true>(P, c),
                    A2 = load_cell<T, true>(P, c + sa), A3 = load_cell<T, true>(P, c + 2 * sa);
     T kc[3], kn[3];
-    metric_row<T, K_AOS>(B, N, AXIS, c, kc);
-    metric_row<T, K_AOS>(B, N, AXIS, c + sa, kn);
+    metric_row<T, K_AOS>(B, N, axis, c, kc);
+    metric_row<T, K_AOS>(B, N, axis, c + sa, kn);
     face_from_cells<T, K_AOS>(A0, A1, A2, A3, kc, kn, ph, F, K_AOS ? num<T>(ph).p_ref : T(0));
-  }
-  if (AXIS == 2) {
-    T* fk = (T*)B.Fk + (size_t)c * 5;
-#pragma unroll
-    for (int v = 0; v < 5; ++v) fk[v] = F[v];
-    return;
-  }
-  T* rec = (T*)B.F + (size_t)c * kRecFA;
-  if (AXIS == 0) {
-    reinterpret_cast<float4*>(rec)[0] = make_float4(F[0], F[1], F[2], F[3]);
-    rec[4] = F[4];
-  } else {
-    rec[5] = F[0];
-    reinterpret_cast<float2*>(rec + 6)[0] = make_float2(F[1], F[2]);
-    reinterpret_cast<float2*>(B.Fz)[c] = make_float2(F[3], F[4]);
   }
 }
 
@@ -773,44 +790,6 @@ __device__ __forceinline__ void asm_chunk(const Dev& d, const SP& sp, int64_t c0
 #pragma unroll
   for (int v = 0; v < 5; ++v) fr[v] = __shfl_down_sync(0xffffffffu, fl[v], 1);
   if (lane == 31 || !alive) return;
-  assemble_cell<T, K_AOS>(B, sp, x, src, flags, stage, next_prims, gm1, R, iR, K_AOS ? ph.p_ref : 0.0, fl, fr, kk,
-                          gcl);
-}
-
-// asm_chunk with the k faces read from Fk (written by the k-face role of
-// k_split_fluxes_roles) instead of evaluated: the face c-1 | c (for k-1 in
-// [1, nk-3]) is Fk of c-1, the face c | c+1 is Fk of c (zero where it does not
-// exist).  The same values as asm_chunk's shuffled ones, so the same result.
-template <typename T, bool K_AOS, class SP>
-__device__ __forceinline__ void asm_chunk_kmem(const Dev& d, const SP& sp, int64_t c0, int flags, int stage,
-                                               int next_prims, double gm1, double R, double iR, const Phys& ph) {
-  const SplitBlock& B = d.blk;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t N = (int64_t)B.ni * B.nj * B.nk;
-  const int64_t c = c0 + warp * 31 + lane;
-  if (lane == 31 || c >= N) return;
-  Cell x;
-  const uint32_t t1 = d.dk.div((uint32_t)c);
-  x.k = (int)((uint32_t)c - t1 * (uint32_t)B.nk);
-  x.i = (int)d.dj.div(t1);
-  x.j = (int)(t1 - (uint32_t)x.i * (uint32_t)B.nj);
-  x.c = c;
-  x.N = N;
-  x.ni = B.ni;
-  x.nj = B.nj;
-  x.nk = B.nk;
-  const GlobalSrc<T, K_AOS, true> src{B, (int32_t)N};
-  T kk[9], gcl[3] = {T(0), T(0), T(0)};
-  src.K9((int32_t)c, kk, K_AOS ? gcl : nullptr);
-  T fl[5] = {T(0), T(0), T(0), T(0), T(0)}, fr[5] = {T(0), T(0), T(0), T(0), T(0)};
-  if (flags & kRhsInvscd) {
-    const T* fk = (const T*)B.Fk;
-    if (x.k >= 2 && x.k <= x.nk - 2)
-#pragma unroll
-      for (int v = 0; v < 5; ++v) fl[v] = __ldg(fk + (c - 1) * 5 + v);
-#pragma unroll
-    for (int v = 0; v < 5; ++v) fr[v] = __ldg(fk + c * 5 + v);
-  }
   assemble_cell<T, K_AOS>(B, sp, x, src, flags, stage, next_prims, gm1, R, iR, K_AOS ? ph.p_ref : 0.0, fl, fr, kk,
                           gcl);
 }

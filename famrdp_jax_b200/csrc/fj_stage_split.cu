@@ -29,6 +29,8 @@
 // field-major kxyz; without one the kernels read kxyz field by field.
 // Each launch covers every block of a table; a CTA handles 128 (assembly: 124)
 // consecutive cells of one block, and neighbours are read through L1/L2.
+#include <type_traits>
+
 #include "fj_common.cuh"
 #include "fj_physics.cuh"
 #include "fj_rhs.cuh"
@@ -42,9 +44,6 @@ namespace {
 
 using namespace sd;
 
-// NW: warps per CTA.  4 normally; 2 for tables of less than two 256-cell ranges
-// per SM (the 32^3 block), whose flux and assembly work runs in
-// k_split_fluxes_roles and k_split_assemble_kmem over 64-cell ranges.
 template <typename T, int NW, class TB>
 __global__ void __launch_bounds__(32 * NW) k_split_prims(const TB tab, const double gm1, const double R,
                                                          const double iR, const double p_ref) {
@@ -65,49 +64,6 @@ __global__ void __launch_bounds__(NT, OCC) k_split_fluxes(const TB tab, const Ph
   Cell x;
   if (!decode_cell(tab.b[b], (int64_t)(blockIdx.x - tab.b[b].blk.cta_begin) * NT + threadIdx.x, x)) return;
   flux_cell<T, K_AOS, true>(tab.b[b].blk, tab.b[b].blk.prim, x, ph, flags);
-}
-
-// The flux work of small FP32 tables split by warp roles: a CTA of 256 threads
-// takes the 64 cells of one 2-warp flux CTA; warps 0-1 evaluate their cells'
-// i faces, warps 2-3 the j faces, warps 4-5 the viscous components and warps
-// 6-7 the k faces (into Fk, which k_split_assemble_kmem reads instead of
-// evaluating them).  Each thread's dependency chain is about a third of
-// k_split_fluxes' (a small table leaves most of the GPU's warp slots free,
-// and its kernels' times are set by those chains).
-template <typename T, bool K_AOS, class TB>
-__global__ void __launch_bounds__(256, 4) k_split_fluxes_roles(const TB tab, const Phys ph, const int flags) {
-  const int b = find_block(tab, blockIdx.x);
-  if (threadIdx.x == 0) prefetch_fluxes<T, K_AOS, false>(tab.b[b], blockIdx.x, 64);
-  grid_dep_wait();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const SplitBlock& B = tab.b[b].blk;
-  Cell x;
-  if (!decode_cell(tab.b[b], (int64_t)(blockIdx.x - B.cta_begin) * 64 + (warp & 1) * 32 + lane, x)) return;
-  if (warp < 2) {
-    if (flags & kRhsInvscd) flux_face_part<T, K_AOS, 0>(B, B.prim, x, ph);
-  } else if (warp < 4) {
-    if (flags & kRhsInvscd) flux_face_part<T, K_AOS, 1>(B, B.prim, x, ph);
-  } else if (warp < 6) {
-    if (flags & kRhsViscous) flux_visc_part<T, K_AOS>(B, B.prim, x, ph);
-  } else if (flags & kRhsInvscd) {
-    flux_face_part<T, K_AOS, 2>(B, B.prim, x, ph);
-  }
-}
-
-// The assembly of small FP32 tables: asm_chunk with the k faces read from Fk
-// (2-warp CTAs of 62 cells; a small table puts about five of them on an SM,
-// so the register cap is loose).
-template <typename T, bool K_AOS, class TB>
-__global__ void __launch_bounds__(64, 8) k_split_assemble_kmem(const TB tab, const int flags, const int stage,
-                                                                 const int next_prims, const double gm1,
-                                                                 const double R, const double iR, const Phys ph) {
-  const int b = find_block_asm(tab, blockIdx.x);
-  const Dev& d = tab.b[b];
-  const SplitBlock& B = d.blk;
-  if (threadIdx.x == 0) prefetch_assembly<T, K_AOS, false>(d, blockIdx.x, flags, stage, 62, B.cta_begin_asm);
-  grid_dep_wait();
-  asm_chunk_kmem<T, K_AOS>(d, TablePtrs{B}, (int64_t)(blockIdx.x - B.cta_begin_asm) * 62, flags, stage, next_prims,
-                           gm1, R, iR, ph);
 }
 
 template <typename T, bool K_AOS, int OCC, int NW, class TB>
@@ -280,29 +236,25 @@ __global__ void __launch_bounds__(NT, OCC) k_fm_fluxes(const TB tab, const Phys 
   }
 }
 
-// The FP64 flux work of small tables split by warp roles (192-thread CTAs over
-// the 64 cells of one 2-warp CTA: warps 0-1 the i faces, 2-3 the j faces, 4-5
-// the viscous components), the same arithmetic and stores as k_fm_fluxes.
-template <typename T, int AXIS>
-__device__ __forceinline__ void fm_face_role(const SplitBlock& B, const Cell& x, const Phys& ph) {
-  const int32_t N = (int32_t)x.N, c = (int32_t)x.c;
-  const int ia = AXIS == 0 ? x.i : x.j, na = AXIS == 0 ? x.ni : x.nj;
-  if (ia < 1 || ia > na - 3) return;
-  const int32_t sa = AXIS == 0 ? x.nj * x.nk : x.nk;
+// The FP64 flux work of one cell in separate parts (k_small_stage), the same
+// arithmetic as k_fm_fluxes and the k faces of k_fm_assemble.
+template <typename T>
+__device__ __forceinline__ void face_value(const SplitBlock& B, int32_t N, int axis, int32_t c, int32_t sa, int ia,
+                                           int na, const Phys& ph, T F[5]) {
   const T* __restrict__ P = (const T*)B.prim;
-  const Cell6<T> a0 = load_cell<T>(P, c - sa), a1 = load_cell<T>(P, c),
-                 a2 = load_cell<T>(P, c + sa), a3 = load_cell<T>(P, c + 2 * sa);
-  T kc[3], kn[3], Fo[5];
-  metric_row<T>(B, N, AXIS, c, kc);
-  metric_row<T>(B, N, AXIS, c + sa, kn);
-  face_from_cells<T>(a0, a1, a2, a3, kc, kn, ph, Fo);
-  T* __restrict__ F = (T*)B.F;
 #pragma unroll
-  for (int v = 0; v < 5; ++v) F[(5 * AXIS + v) * N + c] = Fo[v];
+  for (int v = 0; v < 5; ++v) F[v] = T(0);
+  if (ia < 1 || ia > na - 3) return;
+  const Cell6<T> a0 = load_cell<T>(P, c - sa), a1 = load_cell<T>(P, c), a2 = load_cell<T>(P, c + sa),
+                 a3 = load_cell<T>(P, c + 2 * sa);
+  T kc[3], kn[3];
+  metric_row<T>(B, N, axis, c, kc);
+  metric_row<T>(B, N, axis, c + sa, kn);
+  face_from_cells<T>(a0, a1, a2, a3, kc, kn, ph, F);
 }
 
 template <typename T>
-__device__ __forceinline__ void fm_visc_role(const SplitBlock& B, const Cell& x, const Phys& ph) {
+__device__ __forceinline__ void visc_value(const SplitBlock& B, const Cell& x, const Phys& ph, T G[9]) {
   using M = FastMath<T>;
   const int32_t N = (int32_t)x.N, c = (int32_t)x.c;
   const int32_t si = x.nj * x.nk, sj = x.nk;
@@ -345,34 +297,15 @@ __device__ __forceinline__ void fm_visc_role(const SplitBlock& B, const Cell& x,
   const T t11 = mu * (g[1][1] - div_u * third);
   const T t12 = muh * (g[1][2] + g[2][1]);
   const T t22 = mu * (g[2][2] - div_u * third);
-  T* __restrict__ G = (T*)B.G;
-  G[c] = t00;
-  G[N + c] = t01;
-  G[2 * N + c] = t02;
-  G[3 * N + c] = t11;
-  G[4 * N + c] = t12;
-  G[5 * N + c] = t22;
-  G[6 * N + c] = C0.u * t00 + C0.v * t01 + C0.w * t02 + kappa * g[3][0];
-  G[7 * N + c] = C0.u * t01 + C0.v * t11 + C0.w * t12 + kappa * g[3][1];
-  G[8 * N + c] = C0.u * t02 + C0.v * t12 + C0.w * t22 + kappa * g[3][2];
-}
-
-template <typename T, class TB>
-__global__ void __launch_bounds__(192, 2) k_fm_fluxes_roles(const TB tab, const Phys ph, const int flags) {
-  const int b = find_block(tab, blockIdx.x);
-  if (threadIdx.x == 0) prefetch_fluxes<T, false, true>(tab.b[b], blockIdx.x, 64);
-  grid_dep_wait();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const SplitBlock& B = tab.b[b].blk;
-  Cell x;
-  if (!decode_cell(tab.b[b], (int64_t)(blockIdx.x - B.cta_begin) * 64 + (warp & 1) * 32 + lane, x)) return;
-  if (warp < 2) {
-    if (flags & kRhsInvscd) fm_face_role<T, 0>(B, x, ph);
-  } else if (warp < 4) {
-    if (flags & kRhsInvscd) fm_face_role<T, 1>(B, x, ph);
-  } else if (flags & kRhsViscous) {
-    fm_visc_role<T>(B, x, ph);
-  }
+  G[0] = t00;
+  G[1] = t01;
+  G[2] = t02;
+  G[3] = t11;
+  G[4] = t12;
+  G[5] = t22;
+  G[6] = C0.u * t00 + C0.v * t01 + C0.w * t02 + kappa * g[3][0];
+  G[7] = C0.u * t01 + C0.v * t11 + C0.w * t12 + kappa * g[3][1];
+  G[8] = C0.u * t02 + C0.v * t12 + C0.w * t22 + kappa * g[3][2];
 }
 
 // The k face c-1 | c (rhs/invscd.py:62-100) of the FP64 path from the
@@ -388,16 +321,95 @@ __device__ __forceinline__ void fm_k_face_left(const SplitBlock& B, int32_t N, i
   face_from_cells<T>(a0, a1, a2, a3, kl, kr, ph, F);
 }
 
-// Each warp assembles 31 consecutive cells; lane l evaluates the k face on the
-// left of its cell and takes the one on its right from lane l+1 by shuffle
-// (lane 31's cell is the next warp's first, for which it only supplies the
-// face), as in the FP32 assembly.
-// NW: warps per CTA (4; 2 for the small tables of launch_tab, with a looser
-// register cap since such a table puts few CTAs on an SM).
+// Where the assembly of cell c finds its differences of face fluxes and viscous
+// components: the scratch arrays (k faces given), or shared memory (k_small_stage).
+template <typename T>
+struct GlobalSrc {
+  const T* F;  // at c
+  const T* G;
+  int32_t N, si, sj;
+  const T* fl;
+  const T* fr;
+  // F(c) - F(c-e_a); a face that does not count is read at the cell itself
+  __device__ __forceinline__ void faces(bool on_i, bool on_j, T di[5], T dj[5], T dk[5]) const {
+    const T* __restrict__ Fi = F - (on_i ? si : 0);
+    const T* __restrict__ Fj = F - (on_j ? sj : 0);
+#pragma unroll
+    for (int v = 0; v < 5; ++v) {
+      di[v] = __ldg(F + v * N) - __ldg(Fi + v * N);
+      dj[v] = __ldg(F + (5 + v) * N) - __ldg(Fj + (5 + v) * N);
+      dk[v] = fr[v] - fl[v];
+    }
+  }
+  // G(cp) - G(cm), the neighbours along axis l
+  __device__ __forceinline__ void gdiff(int, int32_t cp, int32_t cm, T g[9]) const {
+#pragma unroll
+    for (int m = 0; m < 9; ++m) g[m] = __ldg(G + cp + m * N) - __ldg(G + cm + m * N);
+  }
+};
+
+// The assembly of one cell (rhs/invscd.py:119-131, rhs/viscous.py:86-117,
+// solver/step.py:45-53).
 // Bound by the latency of its loads (about 100 values a cell, most from L2): what
 // counts is how many times a thread waits, so the faces are one batch of loads
 // and the viscous components one per axis, with nothing branched around (4.0 M
 // cells: 369 -> 330 us against a branch per face and equation).
+template <typename T, class Src>
+__device__ __forceinline__ void assemble_inv(const SplitBlock& B, const Cell& x, const Src& src, double r[5]) {
+  // every face value in one batch of loads: a face that does not count is read
+  // at the cell itself and left out of the sum, not branched around
+  const bool on_i = x.i >= 2 && x.i <= x.ni - 3, on_j = x.j >= 2 && x.j <= x.nj - 3, on_k = x.k >= 2 && x.k <= x.nk - 3;
+  const double ivd = rcp_normal(__ldg(B.vol + x.c) + 1e-300);
+  T di[5], dj[5], dk[5];
+  src.faces(on_i, on_j, di, dj, dk);
+#pragma unroll
+  for (int v = 0; v < 5; ++v)  // axis by axis like the reference
+    r[v] = -((on_i ? di[v] : 0.0) + (on_j ? dj[v] : 0.0) + (on_k ? dk[v] : 0.0)) * ivd;
+}
+
+// sum over l of 0.5 kxyz[l][jj] (G(c+e_l) - G(c-e_l)): the 18 components of an axis
+// in one batch of loads
+template <typename T, class Src>
+__device__ __forceinline__ void assemble_visc(const SplitBlock& B, const Cell& x, const Src& src, T acc[4]) {
+  const int32_t N = (int32_t)x.N, c = (int32_t)x.c;
+  const int n[3] = {x.ni, x.nj, x.nk};
+  const int idx[3] = {x.i, x.j, x.k};
+  const int32_t st[3] = {x.nj * x.nk, x.nk, 1};
+  const T* __restrict__ K = B.kxyz + c;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) acc[e] = T(0);
+#pragma unroll
+  for (int l = 0; l < 3; ++l) {
+    T g[9];
+    src.gdiff(l, idx[l] + 1 == n[l] ? c - (n[l] - 1) * st[l] : c + st[l],
+              idx[l] == 0 ? c + (n[l] - 1) * st[l] : c - st[l], g);
+    const T k0 = T(0.5) * __ldg(K + (3 * l) * N), k1 = T(0.5) * __ldg(K + (3 * l + 1) * N),
+            k2 = T(0.5) * __ldg(K + (3 * l + 2) * N);
+    acc[0] += g[0] * k0 + g[1] * k1 + g[2] * k2;
+    acc[1] += g[1] * k0 + g[3] * k1 + g[4] * k2;
+    acc[2] += g[2] * k0 + g[4] * k1 + g[5] * k2;
+    acc[3] += g[6] * k0 + g[7] * k1 + g[8] * k2;
+  }
+}
+
+template <typename T, class Src>
+__device__ __forceinline__ void assemble_cell(const SplitBlock& B, const Cell& x, const Src& src, int flags, int stage,
+                                              int next_prims, double gm1, double R, double iR) {
+  double r[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+  if (flags & kRhsInvscd) assemble_inv<T>(B, x, src, r);
+  if (flags & kRhsViscous) {
+    T acc[4];
+    assemble_visc<T>(B, x, src, acc);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) r[e + 1] += acc[e];
+  }
+  sd::assemble_out<T>(B, TablePtrs{B}, x, stage, next_prims, gm1, R, iR, 0.0, r);
+}
+
+// Each warp assembles 31 consecutive cells; lane l evaluates the k face on the
+// left of its cell and takes the one on its right from lane l+1 by shuffle
+// (lane 31's cell is the next warp's first, for which it only supplies the
+// face), as in the FP32 assembly.
 template <typename T, int OCC, int NW, class TB>
 __global__ void __launch_bounds__(32 * NW, OCC) k_fm_assemble(const TB tab, const int flags,
                                                                  const int stage, const int next_prims,
@@ -429,71 +441,13 @@ __global__ void __launch_bounds__(32 * NW, OCC) k_fm_assemble(const TB tab, cons
 #pragma unroll
   for (int v = 0; v < 5; ++v) fr[v] = __shfl_down_sync(0xffffffffu, fl[v], 1);
   if (lane == 31 || !alive) return;
-  // 32-bit offsets: 15 N < 2^31 is checked on the host
-  const int32_t N = (int32_t)x.N, c = (int32_t)x.c;
-  const int32_t si = x.nj * x.nk, sj = x.nk;
-  const int n[3] = {x.ni, x.nj, x.nk};
-  const int idx[3] = {x.i, x.j, x.k};
-  const int32_t st[3] = {si, sj, 1};
-  double r[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-  if (flags & kRhsInvscd) {
-    // every face value in one batch of loads: a face that does not count is read
-    // at the cell itself and left out of the sum, not branched around
-    const bool on_i = idx[0] >= 2 && idx[0] <= n[0] - 3, on_j = idx[1] >= 2 && idx[1] <= n[1] - 3,
-               on_k = idx[2] >= 2 && idx[2] <= n[2] - 3;
-    const double ivd = rcp_normal(__ldg(B.vol + c) + 1e-300);
-    const T* __restrict__ F = (const T*)B.F + c;
-    const T* __restrict__ Fi = F - (on_i ? si : 0);
-    const T* __restrict__ Fj = F - (on_j ? sj : 0);
-    T di[5], dj[5];
-#pragma unroll
-    for (int v = 0; v < 5; ++v) {
-      di[v] = __ldg(F + v * N) - __ldg(Fi + v * N);
-      dj[v] = __ldg(F + (5 + v) * N) - __ldg(Fj + (5 + v) * N);
-    }
-#pragma unroll
-    for (int v = 0; v < 5; ++v)  // axis by axis like the reference
-      r[v] = -((on_i ? di[v] : 0.0) + (on_j ? dj[v] : 0.0) + (on_k ? fr[v] - fl[v] : 0.0)) * ivd;
-  }
-  if (flags & kRhsViscous) {
-    // sum over l of 0.5 kxyz[l][jj] (G(c+e_l) - G(c-e_l)): the 18 components of
-    // an axis in one batch of loads
-    const T* __restrict__ G = (const T*)B.G;
-    const T* __restrict__ K = B.kxyz + c;
-#pragma unroll
-    for (int l = 0; l < 3; ++l) {
-      const T* __restrict__ gp = G + (idx[l] + 1 == n[l] ? c - (n[l] - 1) * st[l] : c + st[l]);
-      const T* __restrict__ gm = G + (idx[l] == 0 ? c + (n[l] - 1) * st[l] : c - st[l]);
-      T g[9];
-#pragma unroll
-      for (int m = 0; m < 9; ++m) g[m] = __ldg(gp + m * N) - __ldg(gm + m * N);
-      const T k0 = T(0.5) * __ldg(K + (3 * l) * N), k1 = T(0.5) * __ldg(K + (3 * l + 1) * N),
-              k2 = T(0.5) * __ldg(K + (3 * l + 2) * N);
-      r[1] += g[0] * k0 + g[1] * k1 + g[2] * k2;
-      r[2] += g[1] * k0 + g[3] * k1 + g[4] * k2;
-      r[3] += g[2] * k0 + g[4] * k1 + g[5] * k2;
-      r[4] += g[6] * k0 + g[7] * k1 + g[8] * k2;
-    }
-  }
-  if (stage == 0) {
-#pragma unroll
-    for (int v = 0; v < 5; ++v) B.out[v * N + c] = r[v];
-  } else {
-    const double ca = stage == 2 ? 0.75 : 1.0 / 3.0;
-    const double cb = stage == 2 ? 0.25 : 2.0 / 3.0;
-    double qn[5];
-#pragma unroll
-    for (int v = 0; v < 5; ++v) {
-      const int32_t o = v * N + c;
-      const double t = B.q[o] + B.dt * r[v];
-      qn[v] = stage == 1 ? t : ca * B.q0[o] + cb * t;
-      B.out[o] = qn[v];
-    }
-    if (next_prims) store_prim_record<T>(B.prim_next, (size_t)c, qn, gm1, R, iR, 0.0);
-  }
+  const GlobalSrc<T> src{(const T*)B.F + x.c, (const T*)B.G, (int32_t)x.N, x.nj * x.nk, x.nk, fl, fr};
+  assemble_cell<T>(B, x, src, flags, stage, next_prims, gm1, R, iR);
 }
 
 }  // namespace fm
+
+#include "fj_split_small.cuh"
 
 // Record of cell c: the nine kxyz[l][m], then (FP32 records) the three
 // gcl[m] = sum over the axes a with c_a in [2, n_a-3] of
@@ -608,29 +562,11 @@ void launch_pair(const TB& tab, int ctas, int asm_ctas, const Phys& ph, int flag
 
 template <typename T, bool K_AOS, class TB>
 int launch_tab(const TB& tab, int ctas, int asm_ctas, const Phys& ph, int flags, int stage, bool prims_ready,
-               bool next_prims, int variant, cudaStream_t st, cudaEvent_t after_fluxes, int nw = 8) {
+               bool next_prims, int variant, cudaStream_t st, cudaEvent_t after_fluxes) {
   const int np = next_prims ? 1 : 0;
-  if constexpr (sizeof(T) == 4) {
-    if (nw == 2) {  // a small table: the role-split flux kernel and 2-warp assembly CTAs
-      if (!prims_ready)
-        pdl_launch(k_split_prims<T, 2, TB>, ctas, 64, 0, st, tab, ph.gm1, ph.R, 1.0 / ph.R, K_AOS ? ph.p_ref : 0.0);
-      pdl_launch(k_split_fluxes_roles<T, K_AOS, TB>, ctas, 256, 0, st, tab, ph, flags);
-      if (after_fluxes) cudaEventRecord(after_fluxes, st);
-      pdl_launch(k_split_assemble_kmem<T, K_AOS, TB>, asm_ctas, 64, 0, st, tab, flags, stage, np, ph.gm1, ph.R,
-                 1.0 / ph.R, ph);
-      return prims_ready ? 2 : 3;
-    }
-  }
   if constexpr (sizeof(T) == 8) {
-    if (nw == 2) {  // a small table: the role-split flux kernel and 2-warp CTAs
-      if (!prims_ready) pdl_launch(fm::k_fm_prims<double, 2, TB>, ctas, 64, 0, st, tab, ph.gm1, ph.R, 1.0 / ph.R);
-      pdl_launch(fm::k_fm_fluxes_roles<double, TB>, ctas, 192, 0, st, tab, ph, flags);
-      if (after_fluxes) cudaEventRecord(after_fluxes, st);
-      pdl_launch(fm::k_fm_assemble<double, 8, 2, TB>, asm_ctas, 64, 0, st, tab, flags, stage, np, ph.gm1, ph.R,
-                 1.0 / ph.R, ph);
-      return prims_ready ? 2 : 3;
-    }
-    if (!prims_ready) pdl_launch(fm::k_fm_prims<double, kWarps64, TB>, ctas, 32 * kWarps64, 0, st, tab, ph.gm1, ph.R, 1.0 / ph.R);
+    if (!prims_ready)
+      pdl_launch(fm::k_fm_prims<double, kWarps64, TB>, ctas, 32 * kWarps64, 0, st, tab, ph.gm1, ph.R, 1.0 / ph.R);
     switch (variant) {
       case 1: launch_pair64<1>(tab, ctas, asm_ctas, ph, flags, stage, np, st, after_fluxes); break;
       case 2: launch_pair64<2>(tab, ctas, asm_ctas, ph, flags, stage, np, st, after_fluxes); break;
@@ -641,7 +577,8 @@ int launch_tab(const TB& tab, int ctas, int asm_ctas, const Phys& ph, int flags,
     }
   } else {
     if (!prims_ready)
-      pdl_launch(k_split_prims<T, kWarps32, TB>, ctas, 32 * kWarps32, 0, st, tab, ph.gm1, ph.R, 1.0 / ph.R, K_AOS ? ph.p_ref : 0.0);
+      pdl_launch(k_split_prims<T, kWarps32, TB>, ctas, 32 * kWarps32, 0, st, tab, ph.gm1, ph.R, 1.0 / ph.R,
+                 K_AOS ? ph.p_ref : 0.0);
     switch (K_AOS ? variant : 0) {
       case 1: launch_pair<T, K_AOS, 1>(tab, ctas, asm_ctas, ph, flags, stage, np, st, after_fluxes); break;
       case 2: launch_pair<T, K_AOS, 2>(tab, ctas, asm_ctas, ph, flags, stage, np, st, after_fluxes); break;
@@ -654,6 +591,27 @@ int launch_tab(const TB& tab, int ctas, int asm_ctas, const Phys& ph, int flags,
   return prims_ready ? 2 : 3;
 }
 
+// A small table: the primitives (unless the producer of q left them), then the
+// whole stage in one launch.  ctas: boxes (numbered by cta_begin_asm); prim_ctas:
+// 128-cell ranges (by cta_begin).
+template <typename T, bool K_AOS, class TB>
+int launch_small(const TB& tab, int ctas, int prim_ctas, size_t smem, const Phys& ph, int flags, int stage,
+                 bool prims_ready, bool next_prims, cudaStream_t st, cudaEvent_t after_fluxes) {
+  if (!prims_ready) {
+    if constexpr (sizeof(T) == 8)
+      pdl_launch(fm::k_fm_prims<double, kWarps64, TB>, prim_ctas, 32 * kWarps64, 0, st, tab, ph.gm1, ph.R, 1.0 / ph.R);
+    else
+      pdl_launch(k_split_prims<T, kWarps32, TB>, prim_ctas, 32 * kWarps32, 0, st, tab, ph.gm1, ph.R, 1.0 / ph.R,
+                 K_AOS ? ph.p_ref : 0.0);
+  }
+  auto kern = small::k_small_stage<T, K_AOS, TB>;
+  if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  pdl_launch(kern, ctas, 32 * small::kWarpsOf<T>, smem, st, tab, flags, stage, next_prims ? 1 : 0, ph.gm1, ph.R,
+             1.0 / ph.R, ph);
+  if (after_fluxes) cudaEventRecord(after_fluxes, st);
+  return prims_ready ? 1 : 2;
+}
+
 template <typename T>
 int launch_split(fj_ctx* ctx, const SplitBlock* blocks, int nblocks, const Phys& ph, int flags,
                  int stage, bool prims_ready, bool next_prims, int variant, cudaStream_t st,
@@ -664,17 +622,21 @@ int launch_split(fj_ctx* ctx, const SplitBlock* blocks, int nblocks, const Phys&
   for (int base = 0; base < nblocks; base += kMaxSplitBlocks) {
     Table tab;
     tab.n = std::min(kMaxSplitBlocks, nblocks - base);
-    // tables with fewer 256-thread flux CTAs than two per SM run 2-warp CTAs
-    int nw = sizeof(T) == 8 ? kWarps64 : kWarps32;
-    {
-      int64_t wide = 0;
-      for (int t = 0; t < tab.n; ++t) {
-        const SplitBlock& sb = blocks[base + t];
-        wide += ((int64_t)sb.ni * sb.nj * sb.nk + kSplitThreads - 1) / kSplitThreads;
-      }
-      if (wide < 2 * (int64_t)sms) nw = 2;
+    int64_t cells = 0;
+    for (int t = 0; t < tab.n; ++t) cells += (int64_t)blocks[base + t].ni * blocks[base + t].nj * blocks[base + t].nk;
+    // a small table runs in one launch if its boxes fit the SMs once
+    bool small_tab = cells <= small::kMaxCellsPerSm * (int64_t)sms;
+    int boxes = 0;
+    size_t smem = 0;
+    for (int t = 0; t < tab.n && small_tab; ++t) {
+      const SplitBlock& sb = blocks[base + t];
+      const int64_t N = (int64_t)sb.ni * sb.nj * sb.nk;
+      tab.b[t].blk.cta_begin_asm = boxes;
+      boxes += small::cut(sb.ni, sb.nj, sb.nk, std::max(1, (int)(sms * N / cells)), tab.b[t].tile);
+      smem = std::max(smem, small::values(tab.b[t].tile) * sizeof(T));
+      small_tab = boxes <= sms;
     }
-    const int fcells = 32 * nw, acells = 31 * nw;
+    constexpr int nw = sizeof(T) == 8 ? kWarps64 : kWarps32, fcells = 32 * nw, acells = 31 * nw;
     int ctas = 0, asm_ctas = 0;
     const bool k_aos = blocks[base].kaos != nullptr;
     for (int t = 0; t < tab.n; ++t) {
@@ -684,9 +646,10 @@ int launch_split(fj_ctx* ctx, const SplitBlock* blocks, int nblocks, const Phys&
         return set_err(ctx, FJ_ERR_INVALID_ARGUMENT, "block too large for the split pipeline");
       if ((sb.kaos != nullptr) != k_aos)
         return set_err(ctx, FJ_ERR_INVALID_ARGUMENT, "metric records on some blocks only");
+      const int box0 = tab.b[t].blk.cta_begin_asm;
       tab.b[t].blk = sb;
       tab.b[t].blk.cta_begin = ctas;
-      tab.b[t].blk.cta_begin_asm = asm_ctas;
+      tab.b[t].blk.cta_begin_asm = small_tab ? box0 : asm_ctas;
       tab.b[t].dk.init((uint32_t)sb.nk);
       tab.b[t].dj.init((uint32_t)sb.nj);
       const int64_t N = (int64_t)sb.ni * sb.nj * sb.nk;
@@ -697,11 +660,19 @@ int launch_split(fj_ctx* ctx, const SplitBlock* blocks, int nblocks, const Phys&
       return set_err(ctx, FJ_ERR_INVALID_ARGUMENT, "the FP64 split path reads kxyz directly");
     // the event marks the first chunk's flux launch
     cudaEvent_t ev = base == 0 ? after_fluxes : nullptr;
-    auto launch = [&](const auto& t) {
-      return k_aos ? launch_tab<T, true>(t, ctas, asm_ctas, ph, flags, stage, prims_ready, next_prims, variant, st, ev, nw)
-                   : launch_tab<T, false>(t, ctas, asm_ctas, ph, flags, stage, prims_ready, next_prims, variant, st, ev, nw);
+    auto launch = [&](const auto& t, auto aos) {
+      constexpr bool AOS = decltype(aos)::value;
+      if (small_tab)
+        return launch_small<T, AOS>(t, boxes, ctas, smem, ph, flags, stage, prims_ready, next_prims, st, ev);
+      return launch_tab<T, AOS>(t, ctas, asm_ctas, ph, flags, stage, prims_ready, next_prims, variant, st, ev);
     };
-    ctx->launches += tab.n == 1 ? launch(TableN<1>{1, {tab.b[0]}}) : launch(tab);
+    auto pick = [&](const auto& t) {
+      if constexpr (sizeof(T) == 4) {
+        if (k_aos) return launch(t, std::true_type());
+      }
+      return launch(t, std::false_type());
+    };
+    ctx->launches += tab.n == 1 ? pick(TableN<1>{1, {tab.b[0]}}) : pick(tab);
     int s = launch_status(ctx, "split stage launch");
     if (s != FJ_OK) return s;
   }
@@ -753,10 +724,9 @@ static void split_counts(int precision, int& nP, int& nF, int& nG) {
   // the stage input's primitives and the next stage's: the assembly reads the
   // first (its k faces) while writing the second
   nP = rec ? 2 * kRecP : 2 * kRecP64;
-  // FP32: the i/j face records and, for the kernels of small tables, the k
-  // faces (Fk, 5 per cell); FP64: the i and j faces, field-major (the k faces
-  // stay in the assembly)
-  nF = rec ? kRecFA + kRecFB + 5 : 10;
+  // the i and j faces: records (FP32), field-major (FP64); the k faces stay in
+  // the assembly
+  nF = rec ? kRecFA + kRecFB : 10;
   nG = 9;  // records: kRecG per cell in G, then one per cell in Gz
 }
 
@@ -788,11 +758,9 @@ void split_assign_scratch(int precision, SplitBlock* blocks, int nblocks, void* 
     if (precision == FJ_PREC_F32FLUX) {
       blocks[b].F = F + kRecFA * off * t;
       blocks[b].Fz = F + (kRecFA * total + kRecFB * off) * t;
-      blocks[b].Fk = F + ((kRecFA + kRecFB) * total + 5 * off) * t;
     } else {
       blocks[b].F = F + nF * off * t;
       blocks[b].Fz = nullptr;
-      blocks[b].Fk = nullptr;
     }
     if (precision == FJ_PREC_F32FLUX) {
       blocks[b].G = G + kRecG * off * t;

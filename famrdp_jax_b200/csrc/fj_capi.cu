@@ -254,8 +254,9 @@ int step_body(fj_ctx* ctx, const fj_block* blocks, double* const* q0p, double* c
   int s;
   const bool persist = ctx->pipeline == FJ_PIPELINE_SPLIT && o.persist && p->precision == FJ_PREC_F32FLUX && kmet;
   const bool fused_fill = ctx->pipeline == FJ_PIPELINE_SPLIT && o.fill && p->precision == FJ_PREC_F32FLUX && kmet;
-  // the copy, the halo fill and the stage-1 primitives as one kernel where the
-  // step is not in place (its sources are then the untouched input states);
+  // the copy, the halo fill, the boundary conditions and the stage-1 primitives
+  // as one kernel where the step is not in place (its sources are then the
+  // untouched input states);
   // the persistent and fused-fill paths fill the halo themselves
   const bool split_run = ctx->pipeline == FJ_PIPELINE_SPLIT && !persist &&
                          !(o.tile && p->precision == FJ_PREC_F32FLUX && kmet);
@@ -273,10 +274,11 @@ int step_body(fj_ctx* ctx, const fj_block* blocks, double* const* q0p, double* c
   for (size_t b = 0; b < sb.size(); ++b) prim[b] = sb[b].prim;
   const PrimsOut prims{p->precision, prim.data(), p->gamma - 1.0, p->R, kmet ? o.p_ref : 0.0};
   bool filled = false;
-  bool apart = nlinks > 0 && !persist && !fused_fill;
+  bool apart = nlinks + nbcs > 0 && !persist && !fused_fill;
   for (int b = 0; b < nblocks && apart; ++b) apart = q0p[b] != blocks[b].q;
   if (apart) {
-    s = copy_fill(ctx, blocks, q0p, nblocks, links, nlinks, p->ghost, st, &filled, split_run ? &prims : nullptr);
+    s = copy_fill(ctx, blocks, q0p, nblocks, links, nlinks, p->ghost, bcs, nbcs, p, st, &filled,
+                  split_run ? &prims : nullptr);
     if (s != FJ_OK) return s;
   }
   for (int b = 0; b < nblocks; ++b) out[b].q = q0p[b];
@@ -308,9 +310,8 @@ int step_body(fj_ctx* ctx, const fj_block* blocks, double* const* q0p, double* c
   } else {
     if (!filled) {
       s = halo_exchange(ctx, out.data(), nblocks, links, nlinks, p->ghost, (double*)tail, tail_b, st);
-      if (s != FJ_OK) return s;
+      if (s == FJ_OK) s = apply_bc(ctx, out.data(), nblocks, bcs, nbcs, p, st);
     }
-    s = apply_bc(ctx, out.data(), nblocks, bcs, nbcs, p, st, filled && split_run ? &prims : nullptr);
   }
   if (s != FJ_OK) return s;
   const int flags = kRhsInvscd | kRhsViscous;

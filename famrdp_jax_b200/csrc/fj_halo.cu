@@ -25,6 +25,8 @@
 // Boundary conditions run after the halo, one launch per face in Face enum
 // order (physics/bc/dispatch.py:15), each launch covering that face of every
 // block (blocks are independent).
+#include <algorithm>
+#include <cstring>
 #include <vector>
 
 #include "fj_common.cuh"
@@ -50,9 +52,8 @@ using HaloTable = HaloTableN<kMaxLinksPerLaunch>;
 
 struct BcTable {
   int n;
-  double gamma, R, p_ref;
+  double gamma, R;
   BcDesc d[kMaxBcPerLaunch];
-  void* prim[kMaxBcPerLaunch];  // the face's block's primitive records (k_bc<4>, <8>)
 };
 
 // Primitive records of conserved values q: PR = bytes of a record's values (4:
@@ -98,7 +99,6 @@ __global__ void k_halo_scatter(const HaloTable tab, const double* __restrict__ s
   }
 }
 
-template <int PR>
 __global__ void k_bc(const BcTable tab, int g) {
   grid_dep_wait();
   const BcDesc& d = tab.d[blockIdx.y];
@@ -111,15 +111,6 @@ __global__ void k_bc(const BcTable tab, int g) {
     const int x = (int)((r / d.n[ob]) % d.n[oa]);
     const int o = (int)(r / ((int64_t)d.n[ob] * d.n[oa]));
     bc_cell(d, d.q, ax, oa, ob, o, x, y, g, tab.gamma, tab.R);
-    if constexpr (PR != 0) {
-      int at[3], inner;
-      bc_layers(d.face, d.n[ax], g, o, at[ax], inner);
-      at[oa] = x;
-      at[ob] = y;
-      const int64_t c = cell_index(d.n, at[0], at[1], at[2]), N = (int64_t)d.n[0] * d.n[1] * d.n[2];
-      const double q[5] = {d.q[c], d.q[N + c], d.q[2 * N + c], d.q[3 * N + c], d.q[4 * N + c]};
-      put_prims<PR>(tab.prim[blockIdx.y], (size_t)c, q, tab.gamma - 1.0, tab.R, tab.p_ref);
-    }
   }
 }
 
@@ -321,6 +312,10 @@ namespace {
 // would not give every SM 16 CTAs so (their time is the per-thread latency),
 // else kFillCells.
 constexpr int kMaxFillBlocks = 64, kFillCells = 4;
+// The boundary condition on each face of a block: its kind and the entry of the
+// table's parameter sets it uses (farfield state or wall temperature).
+enum : unsigned char { kBcNone = 0, kBcFar, kBcWall, kBcIso, kBcSym };
+constexpr int kMaxBcSets = 16;
 struct FillBlock {
   const double* src;
   double* dst;
@@ -329,16 +324,18 @@ struct FillBlock {
   sd::FastDiv dk, dj;
   int cta_begin;
   short first, count;
+  unsigned char bc[6], set[6], any_bc;
 };
 template <int NB, int NL>
 struct CopyFillTableN {
   int nb, ghost, cells;
   double gm1, R, p_ref;
+  double set[kMaxBcSets][5];
   FillBlock b[NB];
   short order[NL];
 };
 using CopyFillTable = CopyFillTableN<kMaxFillBlocks, kMaxLinksPerLaunch>;
-// one block with a link on each face at most: 0.9 KB of parameters instead of 26
+// one block with a link on each face at most: 1.5 KB of parameters instead of 28
 using HaloTable1 = HaloTableN<6>;
 using CopyFillTable1 = CopyFillTableN<1, 6>;
 static_assert(sizeof(HaloTable) + sizeof(CopyFillTable) <= 32764, "kernel parameter space");
@@ -347,11 +344,20 @@ static_assert(sizeof(HaloTable) + sizeof(CopyFillTable) <= 32764, "kernel parame
 // covers: those take the source cell of the LAST such link (list order), read
 // from the source block's src, i.e. from the pre-exchange states (src is
 // never written here).  The same values as a copy followed by the gather and
-// the ordered scatter.  With PR, the cells' primitive records too, from the
+// the ordered scatter.  Then the block's boundary conditions, in Face order
+// (physics/bc/dispatch.py:15): a ghost cell takes the value that the last face
+// covering it gives, which mirrors a cell whose own value is resolved with the
+// faces before that one, and so on down to a farfield state, a link's source cell
+// or the cell itself -- the same values as one pass over the block per face, each
+// reading what the passes before it wrote.  With PR, the cells' primitive records
+// too, from the
 // values in registers (a separate kernel read the 40 bytes a cell again).
 // Bound by memory: a thread's U cells are all loaded before the first store.
 // 4.0 M cells: 70 us with FP32 records, 86 us with FP64 ones (4.9 TB/s); the copy
 // alone took 77 us cell by cell and the primitive kernel after it 40 and 59 us.
+// With the boundary faces in it a 97 x 61 x 45 block between walls and symmetry
+// planes takes 219 us an FP64 step instead of 240 (four launches less), a 12-block
+// tree with farfield faces 758 instead of 810.
 template <int PR, int U, int NB, int NL>
 __global__ void __launch_bounds__(kThreads) k_copy_fill(const HaloTableN<NL> tab, const CopyFillTableN<NB, NL> ct) {
   grid_dep_wait();
@@ -382,13 +388,52 @@ __global__ void __launch_bounds__(kThreads) k_copy_fill(const HaloTableN<NL> tab
     const double* from = s + c;
     int64_t NS = N;
     if (i < g || i >= ni - g || j < g || j >= nj - g || k < g || k >= nk - g) {
+      int x[3] = {i, j, k}, far = -1;
+      uint32_t faces = 0, depth = 0;  // mirrored faces, three bits each, innermost lowest
+      if (B.any_bc) {
+        for (int f = 5; f >= 0; --f) {
+          const int a = f >> 1, n = B.n[a];
+          if (B.bc[f] == kBcNone || !((f & 1) == 0 ? x[a] < g : x[a] >= n - g)) continue;
+          if (B.bc[f] == kBcFar) {
+            far = B.set[f];
+            break;
+          }
+          x[a] = (f & 1) == 0 ? 2 * g - 1 - x[a] : 2 * (n - g) - 1 - x[a];
+          faces = (faces << 3) | (uint32_t)f;
+          ++depth;
+        }
+      }
       int L = -1;
-      for (int e = e1 - 1; e >= e0 && L < 0; --e)
-        if (slab_covers(tab.d[ct.order[e]], i, j, k)) L = ct.order[e];
+      if (far < 0)
+        for (int e = e1 - 1; e >= e0 && L < 0; --e)
+          if (slab_covers(tab.d[ct.order[e]], x[0], x[1], x[2])) L = ct.order[e];
       if (L >= 0) {
         const HaloDesc& h = tab.d[L];
         NS = (int64_t)h.sn[0] * h.sn[1] * h.sn[2];
-        from = h.src + (h.s0 + (i - h.tlo[0]) * h.sstr[0] + (j - h.tlo[1]) * h.sstr[1] + (k - h.tlo[2]) * h.sstr[2]);
+        from = h.src + (h.s0 + (x[0] - h.tlo[0]) * h.sstr[0] + (x[1] - h.tlo[1]) * h.sstr[1] + (x[2] - h.tlo[2]) * h.sstr[2]);
+      } else {
+        from = s + ((int64_t)x[0] * nj + x[1]) * nk + x[2];
+      }
+      if (far >= 0 || depth > 0) {
+        double y[5];
+#pragma unroll
+        for (int v = 0; v < 5; ++v) y[v] = far >= 0 ? ct.set[far][v] : __ldg(from + v * NS);
+        for (; depth > 0; --depth, faces >>= 3) {
+          const int f = (int)(faces & 7u);
+          if (B.bc[f] == kBcIso) {
+            double o[5];
+            isothermal_ghost(y, ct.gm1, ct.R, ct.set[B.set[f]][0], o);
+#pragma unroll
+            for (int v = 0; v < 5; ++v) y[v] = o[v];
+          } else {
+#pragma unroll
+            for (int v = 1; v < 4; ++v)
+              if (B.bc[f] == kBcWall || (f >> 1) == v - 1) y[v] = -y[v];
+          }
+        }
+#pragma unroll
+        for (int v = 0; v < 5; ++v) q[u][v] = y[v];
+        continue;
       }
     }
 #pragma unroll
@@ -406,12 +451,39 @@ __global__ void __launch_bounds__(kThreads) k_copy_fill(const HaloTableN<NL> tab
 
 }  // namespace
 
+static int check_bcs(fj_ctx* ctx, int nblocks, const fj_bc* bcs, int nbcs);
+
 int copy_fill(fj_ctx* ctx, const fj_block* blocks, double* const* dst, int nblocks, const fj_link* links, int nlinks,
-              int ghost, cudaStream_t st, bool* done, const PrimsOut* prims) {
+              int ghost, const fj_bc* bcs, int nbcs, const fj_params* p, cudaStream_t st, bool* done,
+              const PrimsOut* prims) {
   *done = false;
+  const int bad = check_bcs(ctx, nblocks, bcs, nbcs);
+  if (bad != FJ_OK) return bad;
   if (nblocks > kMaxFillBlocks || nlinks > kMaxLinksPerLaunch) return FJ_OK;  // the separate copy and fill
   for (int b = 0; b < nblocks; ++b)
     if ((int64_t)blocks[b].ni * blocks[b].nj * blocks[b].nk >= ((int64_t)1 << 31)) return FJ_OK;
+  CopyFillTable ct;
+  for (int b = 0; b < nblocks; ++b) {
+    for (int f = 0; f < 6; ++f) ct.b[b].bc[f] = kBcNone;
+    ct.b[b].any_bc = 0;
+  }
+  int sets = 0;
+  for (int e = 0; e < nbcs; ++e) {  // validated by the caller (check_bcs)
+    const fj_bc& c = bcs[e];
+    FillBlock& F = ct.b[c.block];
+    if (F.bc[c.face] != kBcNone) return FJ_OK;  // a face listed twice: the separate passes
+    const bool far = c.type == FJ_BC_FARFIELD, iso = c.type == FJ_BC_WALL && c.isothermal;
+    F.bc[c.face] = far ? kBcFar : (iso ? kBcIso : (c.type == FJ_BC_WALL ? kBcWall : kBcSym));
+    F.any_bc = 1;
+    if (!far && !iso) continue;
+    double v[5] = {c.T_wall, 0.0, 0.0, 0.0, 0.0};
+    if (far) std::copy(c.q_inf, c.q_inf + 5, v);
+    int at = 0;
+    while (at < sets && std::memcmp(ct.set[at], v, sizeof(v)) != 0) ++at;
+    if (at == kMaxBcSets) return FJ_OK;  // too many different states for one launch's table
+    if (at == sets) std::copy(v, v + 5, ct.set[sets++]);
+    F.set[c.face] = (unsigned char)at;
+  }
   std::vector<HaloDesc> descs;
   size_t nd = 0;
   int s = build_links(ctx, blocks, nblocks, links, nlinks, ghost, descs, nd);
@@ -419,7 +491,6 @@ int copy_fill(fj_ctx* ctx, const fj_block* blocks, double* const* dst, int nbloc
   HaloTable tab;
   tab.n = (int)descs.size();
   for (int L = 0; L < tab.n; ++L) tab.d[L] = descs[(size_t)L];
-  CopyFillTable ct;
   ct.nb = nblocks;
   ct.ghost = ghost;
   int pos = 0;
@@ -427,8 +498,8 @@ int copy_fill(fj_ctx* ctx, const fj_block* blocks, double* const* dst, int nbloc
   for (int b = 0; b < nblocks; ++b) narrow += ((int64_t)blocks[b].ni * blocks[b].nj * blocks[b].nk + kThreads - 1) / kThreads;
   const bool wide = narrow >= 16 * 148;
   ct.cells = wide ? kFillCells * kThreads : kThreads;
-  ct.gm1 = prims ? prims->gm1 : 0.0;
-  ct.R = prims ? prims->R : 1.0;
+  ct.gm1 = p->gamma - 1.0;
+  ct.R = p->R;
   ct.p_ref = prims ? prims->p_ref : 0.0;
   for (int b = 0; b < nblocks; ++b) {
     FillBlock& F = ct.b[b];
@@ -459,7 +530,15 @@ int copy_fill(fj_ctx* ctx, const fj_block* blocks, double* const* dst, int nbloc
   if (nblocks == 1 && tab.n <= 6) {
     HaloTable1 h1;
     h1.n = tab.n;
-    CopyFillTable1 f1{1, ct.ghost, ct.cells, ct.gm1, ct.R, ct.p_ref, {ct.b[0]}, {}};
+    CopyFillTable1 f1;
+    f1.nb = 1;
+    f1.ghost = ct.ghost;
+    f1.cells = ct.cells;
+    f1.gm1 = ct.gm1;
+    f1.R = ct.R;
+    f1.p_ref = ct.p_ref;
+    std::copy(&ct.set[0][0], &ct.set[0][0] + 5 * kMaxBcSets, &f1.set[0][0]);
+    f1.b[0] = ct.b[0];
     for (int L = 0; L < tab.n; ++L) {
       h1.d[L] = tab.d[L];
       f1.order[L] = ct.order[L];
@@ -474,8 +553,7 @@ int copy_fill(fj_ctx* ctx, const fj_block* blocks, double* const* dst, int nbloc
   return s;
 }
 
-int apply_bc(fj_ctx* ctx, const fj_block* blocks, int nblocks, const fj_bc* bcs, int nbcs,
-             const fj_params* p, cudaStream_t st, const PrimsOut* prims) {
+static int check_bcs(fj_ctx* ctx, int nblocks, const fj_bc* bcs, int nbcs) {
   for (int b = 0; b < nbcs; ++b) {
     const fj_bc& e = bcs[b];
     if (e.block < 0 || e.block >= nblocks)
@@ -485,14 +563,19 @@ int apply_bc(fj_ctx* ctx, const fj_block* blocks, int nblocks, const fj_bc* bcs,
     if (e.type != FJ_BC_WALL && e.type != FJ_BC_SYMMETRY && e.type != FJ_BC_FARFIELD)
       return set_err(ctx, FJ_ERR_INVALID_ARGUMENT, "unsupported bc type");
   }
+  return FJ_OK;
+}
+
+int apply_bc(fj_ctx* ctx, const fj_block* blocks, int nblocks, const fj_bc* bcs, int nbcs,
+             const fj_params* p, cudaStream_t st) {
+  const int bad = check_bcs(ctx, nblocks, bcs, nbcs);
+  if (bad != FJ_OK) return bad;
   for (int face = 0; face < 6; ++face) {
     std::vector<BcDesc> ds;
-    std::vector<void*> rec;
     for (int b = 0; b < nbcs; ++b) {
       const fj_bc& e = bcs[b];
       if (e.face != face) continue;
       const fj_block& blk = blocks[e.block];
-      rec.push_back(prims ? prims->prim[e.block] : nullptr);
       BcDesc d;
       d.q = blk.q;
       d.n[0] = blk.ni; d.n[1] = blk.nj; d.n[2] = blk.nk;
@@ -508,18 +591,15 @@ int apply_bc(fj_ctx* ctx, const fj_block* blocks, int nblocks, const fj_bc* bcs,
       tab.n = (int)std::min<size_t>(kMaxBcPerLaunch, ds.size() - base);
       tab.gamma = p->gamma;
       tab.R = p->R;
-      tab.p_ref = prims ? prims->p_ref : 0.0;
       int64_t vmax = 0;
       for (int t = 0; t < tab.n; ++t) {
         tab.d[t] = ds[base + t];
-        tab.prim[t] = rec[base + t];
         const int ax = face >> 1;
         int64_t area = (int64_t)tab.d[t].n[0] * tab.d[t].n[1] * tab.d[t].n[2] / tab.d[t].n[ax];
         vmax = std::max<int64_t>(vmax, area * p->ghost);
       }
       dim3 grid((unsigned)std::min<int64_t>(grid_for(vmax), 4096), tab.n);
-      auto kern = !prims ? k_bc<0> : (prims->precision == FJ_PREC_F32FLUX ? k_bc<4> : k_bc<8>);
-      pdl_launch(kern, grid, kThreads, 0, st, tab, p->ghost);
+      pdl_launch(k_bc, grid, kThreads, 0, st, tab, p->ghost);
       ctx->launches += 1;
       int s = launch_status(ctx, "bc launch");
       if (s != FJ_OK) return s;

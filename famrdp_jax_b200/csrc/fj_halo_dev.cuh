@@ -67,6 +67,21 @@ __device__ __forceinline__ void bc_layers(int face, int n, int g, int o, int& ou
   }
 }
 
+// The isothermal wall's ghost state from its image cell's (physics/bc/wall.py:32-55).
+__device__ __forceinline__ void isothermal_ghost(const double r[5], double gm1, double R, double T_wall, double o[5]) {
+  const double ke_i = 0.5 * (r[1] * r[1] + r[2] * r[2] + r[3] * r[3]) / r[0];
+  const double p_g = gm1 * (r[4] - ke_i);
+  const double rho_g = p_g / (R * T_wall);
+  const double scale = rho_g / r[0];
+  const double u_g = -r[1] * scale, v_g = -r[2] * scale, w_g = -r[3] * scale;
+  const double ke_g = 0.5 * (u_g * u_g + v_g * v_g + w_g * w_g) / rho_g;
+  o[0] = rho_g;
+  o[1] = u_g;
+  o[2] = v_g;
+  o[3] = w_g;
+  o[4] = p_g / gm1 + ke_g;
+}
+
 // The boundary condition d on ghost layer o, cell (x, y) of the face's two
 // other axes oa, ob (ax: the face's axis), in place on q (5, n0, n1, n2).
 __device__ __forceinline__ void bc_cell(const BcDesc& d, double* q, int ax, int oa, int ob, int o, int x, int y,
@@ -84,19 +99,11 @@ __device__ __forceinline__ void bc_cell(const BcDesc& d, double* q, int ax, int 
 #pragma unroll
     for (int v = 0; v < 5; ++v) q[v * NT + co] = d.qinf[v];
   } else if (d.type == FJ_BC_WALL && d.iso) {  // physics/bc/wall.py:32-55
-    const double r0 = q[ci], r1 = q[NT + ci], r2 = q[2 * NT + ci], r3 = q[3 * NT + ci], r4 = q[4 * NT + ci];
-    const double gm1 = gamma - 1.0;
-    const double ke_i = 0.5 * (r1 * r1 + r2 * r2 + r3 * r3) / r0;
-    const double p_g = gm1 * (r4 - ke_i);
-    const double rho_g = p_g / (R * d.T_wall);
-    const double scale = rho_g / r0;
-    const double u_g = -r1 * scale, v_g = -r2 * scale, w_g = -r3 * scale;
-    const double ke_g = 0.5 * (u_g * u_g + v_g * v_g + w_g * w_g) / rho_g;
-    q[co] = rho_g;
-    q[NT + co] = u_g;
-    q[2 * NT + co] = v_g;
-    q[3 * NT + co] = w_g;
-    q[4 * NT + co] = p_g / gm1 + ke_g;
+    const double r[5] = {q[ci], q[NT + ci], q[2 * NT + ci], q[3 * NT + ci], q[4 * NT + ci]};
+    double o5[5];
+    isothermal_ghost(r, gamma - 1.0, R, d.T_wall, o5);
+#pragma unroll
+    for (int v = 0; v < 5; ++v) q[v * NT + co] = o5[v];
   } else {  // mirror: adiabatic wall (wall.py:27-29) or symmetry (symmetry.py:8-11)
     double s[5] = {1.0, 1.0, 1.0, 1.0, 1.0};
     if (d.type == FJ_BC_WALL) {

@@ -42,7 +42,7 @@ struct CopyTable {
 int copy_states(const double* const* src, double* const* dst, const int64_t* len, int n, cudaStream_t st,
                 int64_t* launches);
 
-// Where the fill of a step's start state (copy_fill, apply_bc) also leaves the
+// Where the fill of a step's start state (copy_fill) also leaves the
 // primitive records stage 1 of the split pipeline reads (fj_split_dev.cuh):
 // prim[b] for block b, in the records of `precision`.
 struct PrimsOut {
@@ -56,16 +56,17 @@ struct PrimsOut {
 int halo_exchange(fj_ctx* ctx, const fj_block* blocks, int nblocks, const fj_link* links,
                   int nlinks, int ghost, double* scratch, size_t scratch_bytes,
                   cudaStream_t st);
-// With prims, the primitives of every cell written are written too.
 int apply_bc(fj_ctx* ctx, const fj_block* blocks, int nblocks, const fj_bc* bcs, int nbcs,
-             const fj_params* p, cudaStream_t st, const PrimsOut* prims = nullptr);
-// The step's start state blocks[b].q -> dst[b] with the halo fill of `links`
-// folded in (one kernel over all blocks; dst must not overlap blocks[].q).
-// *done = false, without launching, when the link or block count exceeds one
-// launch's table: the caller then copies and fills separately.  With prims, the
-// primitives of every cell are written too.
+             const fj_params* p, cudaStream_t st);
+// The step's start state blocks[b].q -> dst[b] with the halo fill of `links` and
+// the boundary conditions folded in (one kernel over all blocks; dst must not
+// overlap blocks[].q).  *done = false, without launching, when the links, blocks
+// or distinct boundary states exceed one launch's table or a face is listed
+// twice: the caller then copies, fills and applies the conditions separately.
+// With prims, the primitives of every cell are written too.
 int copy_fill(fj_ctx* ctx, const fj_block* blocks, double* const* dst, int nblocks, const fj_link* links, int nlinks,
-              int ghost, cudaStream_t st, bool* done, const PrimsOut* prims = nullptr);
+              int ghost, const fj_bc* bcs, int nbcs, const fj_params* p, cudaStream_t st, bool* done,
+              const PrimsOut* prims = nullptr);
 // Bytes of scratch the halo gather needs for these links (0 on shape errors).
 size_t halo_ws_bytes(const fj_block* blocks, const fj_link* links, int nlinks, int ghost);
 // One device's part of a halo fill whose blocks live on several devices: the

@@ -58,3 +58,26 @@ def test_fill_with_primitives_matches_separate_kernels(cuda_device, nij, nk0, nk
         assert torch.equal(q, k)  # the input is untouched
         assert torch.equal(o, s)
         assert torch.isfinite(o).all()
+
+
+@pytest.mark.parametrize("precision", ["f64", "f32"])
+@pytest.mark.parametrize("shape", [(5, 5, 5), (6, 5, 9), (9, 12, 33)])
+def test_boundary_faces_alone(cuda_device, shape, precision):
+    """No interface at all: every ghost cell comes from boundary faces, edges and
+    corners through up to three of them, thin blocks through both faces of an
+    axis."""
+    F, B = Face, BCType
+    topo = (BlockTopology(0, {}, {F.IMIN: B.WALL, F.IMAX: B.SYMMETRY, F.JMIN: B.SYMMETRY, F.JMAX: B.WALL,
+                                  F.KMIN: B.WALL, F.KMAX: B.FARFIELD}),)
+    prm = {F.JMAX: {"wall_type": "isothermal", "T_wall": 0.8}, F.KMAX: {"q_inf": [1.0, 0.3, 0.0, 0.1, 2.0]}}
+    cfg = Config(gas=GAS, scheme=SchemeChoice("muscl2", "roe", 3, "minmod"), bc_params=prm, topology=topo, ghost=2,
+                 nan_check=False, precision=precision)
+    q, kxyz, vol = (dev(x) for x in random_block(shape, 9))
+    state = State(blocks=(Block(q=q, xyz=torch.zeros((3,) + shape, dtype=torch.float64, device="cuda")),),
+                  metrics=(Metrics(jac=vol, kxyz=kxyz, vol=vol),))
+    plan = StepPlan(state, cfg)
+    out = torch.full_like(q, float("nan"))
+    plan.run([q], [out], 1e-5)
+    same = q.clone()
+    plan.run([same], [same], 1e-5)
+    assert torch.equal(out, same)

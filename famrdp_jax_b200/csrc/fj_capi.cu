@@ -66,6 +66,7 @@ SplitBlock split_block(const double* q, const double* q0, double* out, const dou
   b.out = out;
   b.kxyz = kxyz;
   b.kaos = kaos;
+  b.kstep = kaos ? kRecK<float> : 1;
   b.vol = vol;
   b.ni = ni;
   b.nj = nj;
@@ -208,6 +209,7 @@ struct StepOpts {
   // persistent launch (the persistent step's work-list head)
   const PersistPlan* fill = nullptr;
   int wait_limit = -1;
+  const char* uniform = nullptr;  // per block: every cell has the same metrics (fj_plan::uniform), or nullptr
 };
 
 // The three stages of all blocks with the tile kernel: the primitives of the
@@ -267,6 +269,7 @@ int step_body(fj_ctx* ctx, const fj_block* blocks, double* const* q0p, double* c
       const fj_block& B = out[b];
       sb[b] = split_block(q0p[b], q0p[b], q1s[b], B.kxyz, kmet ? kmet[b] : nullptr, B.vol, B.ni, B.nj, B.nk,
                           mu0_b ? mu0_b[b] : p->mu0, dt_b ? dt_b[b] : dt);
+      if (o.uniform && o.uniform[b]) sb[b].kstep = 0;
     }
     split_assign_scratch(p->precision, sb.data(), nblocks, tail);
   }
@@ -665,8 +668,7 @@ int fj_plan_create(fj_ctx* ctx, const fj_block* blocks, int nblocks, const fj_li
     fj_plan_destroy(pl);
     return cuda_status(ctx, e, "plan stream creation");
   }
-  if (p->precision == FJ_PREC_F32FLUX &&
-      (pl->pipeline == FJ_PIPELINE_SPLIT || pl->pipeline == FJ_PIPELINE_FUSED)) {
+  if (p->precision == FJ_PREC_F32FLUX && (split || pl->pipeline == FJ_PIPELINE_FUSED)) {
     pl->kmet.assign(nblocks, nullptr);
     for (int b = 0; b < nblocks; ++b) {
       const int64_t N = (int64_t)blocks[b].ni * blocks[b].nj * blocks[b].nk;
@@ -724,6 +726,29 @@ int fj_plan_create(fj_ctx* ctx, const fj_block* blocks, int nblocks, const fj_li
       }
     }
   }
+  // blocks whose cells all have the same metrics (uniform Cartesian grids; the
+  // metrics stay unchanged while the plan lives): the split kernels then read one
+  // cell's for all
+  if (split) {
+    std::vector<int> differ(nblocks, 1);
+    int* flags = (int*)pl->scratch;  // no step has used it yet
+    e = total >= nblocks * sizeof(int) ? cudaMemsetAsync(flags, 0, nblocks * sizeof(int), pl->capture_stream)
+                                       : cudaErrorMemoryAllocation;
+    for (int b = 0; b < nblocks && e == cudaSuccess; ++b)
+      if (split_metrics_differ(pl->kmet.empty() ? nullptr : pl->kmet[b], blocks[b].kxyz,
+                               (int64_t)blocks[b].ni * blocks[b].nj * blocks[b].nk, flags + b,
+                               pl->capture_stream) != FJ_OK)
+        e = cudaErrorUnknown;
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(differ.data(), flags, nblocks * sizeof(int), cudaMemcpyDeviceToHost, pl->capture_stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(pl->capture_stream);
+    if (e != cudaSuccess) {
+      fj_plan_destroy(pl);
+      return cuda_status(ctx, e, "plan metric check");
+    }
+    pl->uniform.resize(nblocks);
+    for (int b = 0; b < nblocks; ++b) pl->uniform[b] = differ[b] == 0;
+  }
   *out = pl;
   return FJ_OK;
 }
@@ -753,6 +778,7 @@ static int plan_step_impl(fj_plan* pl, double* const* q_in, double* const* q_out
   opts.mu0_b = pl->mu0_b.empty() ? nullptr : pl->mu0_b.data();
   opts.dt_b = pl->dt_b.empty() ? nullptr : pl->dt_b.data();
   opts.p_ref = pl->p_ref;
+  opts.uniform = pl->uniform.empty() ? nullptr : pl->uniform.data();
   opts.variant = pl->variant;
   if (pl->kernel == FJ_KERNEL_TILE && pl->tile) {
     opts.tile = (const TileMaps*)pl->tile;
@@ -1136,6 +1162,7 @@ int fj_plan_stage(fj_plan* pl, double* const* q, double* const* q0, double* cons
       sb[b] = split_block(q[b], stage > 1 ? q0[b] : q[b], out[b], B.kxyz,
                           pl->kmet.empty() ? nullptr : pl->kmet[b], B.vol, B.ni, B.nj, B.nk,
                           pl->mu0_b.empty() ? pl->p.mu0 : pl->mu0_b[b], pl->dt_b.empty() ? dt : pl->dt_b[b]);
+      if (!pl->uniform.empty() && pl->uniform[b]) sb[b].kstep = 0;
     }
     split_assign_scratch(pl->p.precision, sb.data(), nb, tail);
     Phys ph = make_phys(&pl->p);

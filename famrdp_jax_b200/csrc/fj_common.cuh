@@ -45,6 +45,7 @@ struct fj_plan {
   std::vector<fj_bc> bcs;
   fj_params p{};
   std::vector<void*> kmet;  // per-block metric copy for the plan's pipeline (or empty)
+  std::vector<char> uniform;  // per block: every cell has the same metrics (split plans, else empty)
   void* scratch = nullptr;   // q1 | q2 | tail (intermediates, halo slabs)
   size_t stage_bytes = 0, halo_bytes = 0;  // halo_bytes: size of the tail
   int pipeline = 0;

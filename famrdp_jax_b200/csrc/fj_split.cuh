@@ -21,7 +21,10 @@ struct SplitBlock {
   const double* q0;      // step start state (stages 2, 3)
   double* out;           // RHS (stage 0) or stage result; may alias q0, never q
   const double* kxyz;    // (3, 3, ni, nj, nk)
-  const void* kaos;      // FP32-flux only: optional FP32 metric records (kRecK per cell), or nullptr
+  const void* kaos;      // FP32-flux only: optional FP32 metric records, or nullptr
+  int kstep;             // from one cell's metrics to the next's: kRecK (records) or 1 (FP64, in each field of
+                         // kxyz); 0 where all cells have the same (a uniform block: a Cartesian grid), which
+                         // are then read from L1
   const double* vol;     // (ni, nj, nk)
   void* prim;            // scratch: the primitives of the stage input (records in FP32)
   void* prim_next;       // where the assembly writes the next stage's primitives: a
@@ -43,6 +46,9 @@ struct SplitBlock {
 // field-major FP64 kxyz (3, 3, ni, nj, nk): the nine kxyz[l][m] and, in FP32
 // records, the three face-normal difference sums the pressure offset uses.
 int split_metric_records(const double* kxyz, void* out, int ni, int nj, int nk, int precision, cudaStream_t st);
+// *flag (device, cleared by the caller) := 1 where a block's FP32 records, or its
+// FP64 kxyz, are not the same bits in every cell.
+int split_metrics_differ(const void* records, const double* kxyz, int64_t N, int* flag, cudaStream_t st);
 // Mean pressure over all padded cells of the blocks, on stream st with
 // mean_pressure_scratch_bytes(nblocks) bytes of device scratch; waits for st.
 size_t mean_pressure_scratch_bytes(int nblocks);

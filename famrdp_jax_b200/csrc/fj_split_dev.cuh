@@ -149,9 +149,9 @@ __device__ __forceinline__ void prefetch_fluxes(const Dev& d, int cta, int cells
   const int64_t a1 = c0 + si, m1 = min(n, N - a1);
   if (m1 > 0) {
     if (K_AOS && !FIELD)
-      l2_prefetch((const T*)B.kaos + a1 * kRecK<T>, m1 * kRecK<T> * (int64_t)sizeof(T));
+      l2_prefetch((const T*)B.kaos + a1 * B.kstep, m1 * B.kstep * (int64_t)sizeof(T));
     else
-      for (int lm = 0; lm < 9; ++lm) l2_prefetch(B.kxyz + lm * N + a1, m1 * 8);
+      for (int lm = 0; lm < 9; ++lm) l2_prefetch(B.kxyz + lm * N + a1, FIELD ? m1 * B.kstep * 8 : m1 * 8);
   }
 }
 
@@ -181,7 +181,7 @@ __device__ __forceinline__ void prefetch_assembly(const Dev& d, int cta, int fla
   const bool inv = (flags & kRhsInvscd) != 0, vis = (flags & kRhsViscous) != 0;
   const int64_t a = c0 + (int64_t)B.nj * B.nk, m = min(n, N - a);
   if (FIELD) {
-    for (int lm = 6; lm < 9; ++lm) l2_prefetch(B.kxyz + lm * N + c0, n * 8);
+    for (int lm = 6; lm < 9; ++lm) l2_prefetch(B.kxyz + lm * N + c0, n * B.kstep * 8);
     if (inv) {
       l2_prefetch((const T*)B.prim + c0 * kRecP64, n * kRecP64 * (int64_t)sizeof(T));
       l2_prefetch(B.vol + c0, n * 8);
@@ -189,12 +189,12 @@ __device__ __forceinline__ void prefetch_assembly(const Dev& d, int cta, int fla
       for (int v = 0; v < 10; ++v) l2_prefetch((const T*)B.F + v * N + c0, n * (int64_t)sizeof(T));
     }
     if (vis) {
-      for (int lm = 0; lm < 6; ++lm) l2_prefetch(B.kxyz + lm * N + c0, n * 8);
+      for (int lm = 0; lm < 6; ++lm) l2_prefetch(B.kxyz + lm * N + c0, n * B.kstep * 8);
       if (m > 0)
         for (int v = 0; v < 9; ++v) l2_prefetch((const T*)B.G + v * N + a, m * (int64_t)sizeof(T));
     }
   } else {
-    if (K_AOS) l2_prefetch((const T*)B.kaos + c0 * kRecK<T>, n * kRecK<T> * (int64_t)sizeof(T));
+    if (K_AOS) l2_prefetch((const T*)B.kaos + c0 * B.kstep, n * B.kstep * (int64_t)sizeof(T));
     if (inv) {
       l2_prefetch((const T*)B.prim + c0 * kRecP, n * kRecP * (int64_t)sizeof(T));
       l2_prefetch(B.vol + c0, n * 8);
@@ -295,7 +295,7 @@ template <typename T, bool K_AOS>
 __device__ __forceinline__ void metric9(const SplitBlock& B, int32_t N, int32_t c, T kk[9], T* gcl = nullptr) {
   if constexpr (K_AOS) {
     T x[kRecK<T>];
-    ld_rec<T, kRecK<T>>((const T*)B.kaos + (size_t)c * kRecK<T>, x);
+    ld_rec<T, kRecK<T>>((const T*)B.kaos + (size_t)c * B.kstep, x);
 #pragma unroll
     for (int lm = 0; lm < 9; ++lm) kk[lm] = x[lm];
     if (gcl) {
@@ -313,7 +313,7 @@ __device__ __forceinline__ void metric9(const SplitBlock& B, int32_t N, int32_t 
 template <typename T, bool K_AOS>
 __device__ __forceinline__ void metric_row(const SplitBlock& B, int32_t N, int l, int32_t c, T k[3]) {
   if constexpr (K_AOS) {
-    const T* K = (const T*)B.kaos + (size_t)c * kRecK<T> + 3 * l;
+    const T* K = (const T*)B.kaos + (size_t)c * B.kstep + 3 * l;
     k[0] = __ldg(K);
     k[1] = __ldg(K + 1);
     k[2] = __ldg(K + 2);

@@ -134,10 +134,10 @@ __device__ __forceinline__ void face_from_cells(const Cell6<T>& a0, const Cell6<
 
 template <typename T>
 __device__ __forceinline__ void metric_row(const SplitBlock& B, int32_t N, int row, int32_t c, T k[3]) {
-  const double* K = B.kxyz + 3 * row * N;
-  k[0] = (T)__ldg(K + c);
-  k[1] = (T)__ldg(K + N + c);
-  k[2] = (T)__ldg(K + 2 * N + c);
+  const double* K = B.kxyz + 3 * row * N + c * B.kstep;
+  k[0] = (T)__ldg(K);
+  k[1] = (T)__ldg(K + N);
+  k[2] = (T)__ldg(K + 2 * N);
 }
 
 template <typename T, int OCC, int NT, class TB>
@@ -375,7 +375,7 @@ __device__ __forceinline__ void assemble_visc(const SplitBlock& B, const Cell& x
   const int n[3] = {x.ni, x.nj, x.nk};
   const int idx[3] = {x.i, x.j, x.k};
   const int32_t st[3] = {x.nj * x.nk, x.nk, 1};
-  const T* __restrict__ K = B.kxyz + c;
+  const T* __restrict__ K = B.kxyz + c * B.kstep;
 #pragma unroll
   for (int e = 0; e < 4; ++e) acc[e] = T(0);
 #pragma unroll
@@ -479,6 +479,22 @@ __global__ void k_metric_records(const double* __restrict__ kxyz, T* __restrict_
     }
   }
   st_rec<T, kRecK<T>>(out + c * kRecK<T>, rec);
+}
+
+// *flag := 1 where a word differs from word % period of the array (bits): n words
+// from m + blockIdx.y * n on, the grid's threads a multiple of `period`, so that
+// a thread compares with one word.  A block that is not uniform shows it in its
+// first cells, and the threads stop.
+__global__ void __launch_bounds__(192) k_words_differ(const unsigned long long* __restrict__ m, int64_t n, int period,
+                                                      int* flag) {
+  m += blockIdx.y * n;
+  const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+  const unsigned long long ref = m[t0 % period];
+  for (int64_t t = t0; t < n; t += step) {
+    if (m[t] == ref) continue;
+    *flag = 1;
+    return;
+  }
 }
 
 // Sum of (pressure) over a block, one partial per CTA (fixed grid, fixed
@@ -689,6 +705,19 @@ int split_metric_records(const double* kxyz, void* out, int ni, int nj, int nk, 
     k_metric_records<float><<<grid, 256, 0, st>>>(kxyz, (float*)out, ni, nj, nk);
   else
     k_metric_records<double><<<grid, 256, 0, st>>>(kxyz, (double*)out, ni, nj, nk);
+  return cudaGetLastError() == cudaSuccess ? FJ_OK : FJ_ERR_CUDA;
+}
+
+int split_metrics_differ(const void* records, const double* kxyz, int64_t N, int* flag, cudaStream_t st) {
+  if (N <= 0) return FJ_OK;
+  constexpr int nt = 192, per = kRecK<float> / 2;  // 8-byte words of an FP32 record
+  static_assert(nt % per == 0, "a thread's words all have the same place in their record");
+  if (records)
+    k_words_differ<<<(unsigned)std::min<int64_t>((N * per + nt - 1) / nt, 148 * 10), nt, 0, st>>>(
+        (const unsigned long long*)records, N * per, per, flag);
+  else
+    k_words_differ<<<dim3((unsigned)std::min<int64_t>((N + nt - 1) / nt, 148 * 2), 9), nt, 0, st>>>(
+        (const unsigned long long*)kxyz, N, 1, flag);
   return cudaGetLastError() == cudaSuccess ? FJ_OK : FJ_ERR_CUDA;
 }
 

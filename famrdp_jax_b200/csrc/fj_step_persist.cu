@@ -802,6 +802,7 @@ int persist_step(fj_ctx* ctx, const PersistPlan& pp, const fj_block* blocks, int
     e.out = nullptr;
     e.kxyz = blocks[b].kxyz;
     e.kaos = kmet[b];
+    e.kstep = kRecK<float>;
     e.vol = blocks[b].vol;
     e.mu0 = mu0_b ? mu0_b[b] : p->mu0;
     e.mu0_f = (float)e.mu0;

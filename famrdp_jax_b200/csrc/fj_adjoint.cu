@@ -614,9 +614,8 @@ int rhs_vjp_impl(fj_ctx* ctx, const double* q, const double* kxyz, const double*
   if constexpr (sizeof(T) == 4) {
     if (ctx->adj_variant == 0 && (flags & kRhsInvscd) && (flags & kRhsViscous)) {
       // FP32 default: both VJPs in one launch (96 registers, 5 CTAs of 128 per
-      // SM).  FP64 keeps two launches: its face VJP is bound by the FP64 pipe at
-      // the 128-register cap, and the fused form (128 x 4) measured 4 % slower
-      // on the reverse sweep
+      // SM).  FP64 keeps two launches, whose parts want different register caps
+      // (the fused form measured 4 % slower on the reverse sweep)
       constexpr int nt = 128;
       pdl_launch(k_adj_faces_visc<T, nt, 5>, 4 * (unsigned)((N + nt - 1) / nt), nt, 0, st, P, kxyz, lv, lamP, lam,
                  lamD, lamL, d, ph, dmu, mu_scale);
@@ -626,9 +625,9 @@ int rhs_vjp_impl(fj_ctx* ctx, const double* q, const double* kxyz, const double*
   }
   if (rest & kRhsInvscd) {
     // register caps (threads per CTA, minimum CTAs per SM): the FP64 face VJP
-    // needs ~180 registers uncapped.  Variant 0 is the fastest measured on
-    // B200 (TGV 96^3 adjoint sweep): FP64 128 x 4 (128 registers), FP32
-    // 256 x 3 (80 registers, a few spilled values)
+    // needs ~180 registers uncapped.  Variant 0 is the fastest measured: FP64 128
+    // x 3 (168 registers, few spills; 9.85 ms for the gradient of 6 steps on 96^3
+    // against 10.1 at 128 x 4), FP32 256 x 3 (80 registers, a few spilled values)
     auto launch = [&](auto kern, int nt) {
       pdl_launch(kern, dim3((unsigned)((N + nt - 1) / nt), 3), nt, 0, st, P, kxyz, lv, lamP, d, ph);
     };
@@ -637,19 +636,20 @@ int rhs_vjp_impl(fj_ctx* ctx, const double* q, const double* kxyz, const double*
       case 1: launch(k_adj_faces<T, 256, 1>, 256); break;
       case 2:
       case 4:
-        if (f64) launch(k_adj_faces<T, 128, 3>, 128);
+        if (f64) launch(k_adj_faces<T, 128, 4>, 128);
         else launch(k_adj_faces<T, 256, 2>, 256);
         break;
       default:
-        if (f64) launch(k_adj_faces<T, 128, 4>, 128);
+        if (f64) launch(k_adj_faces<T, 128, 3>, 128);
         else launch(k_adj_faces<T, 256, 3>, 256);
     }
     ctx->launches += 1;
   }
   if (rest & kRhsViscous) {
-    // variants 0 and 2 cap the viscous VJP at 64 registers (4 CTAs per SM)
+    // variants 0 and 2 cap the viscous VJP at 128 registers (FP64; 64 spill 230
+    // bytes a thread: 5.79 -> 5.60 ms for 20 steps on 48^3) or 64 (FP32)
     if (ctx->adj_variant == 0 || ctx->adj_variant == 2)
-      pdl_launch(k_adj_visc<T, 4>, grid, kAT, 0, st, P, kxyz, lam, lamD, lamL, d, ph, dmu, mu_scale);
+      pdl_launch(k_adj_visc<T, sizeof(T) == 8 ? 2 : 4>, grid, kAT, 0, st, P, kxyz, lam, lamD, lamL, d, ph, dmu, mu_scale);
     else
       pdl_launch(k_adj_visc<T, 1>, grid, kAT, 0, st, P, kxyz, lam, lamD, lamL, d, ph, dmu, mu_scale);
     ctx->launches += 1;

@@ -335,6 +335,125 @@ __device__ __forceinline__ void roe_prim_vjp(const Prim<T>& L, const Prim<T>& R,
   lR.p = lpR;
 }
 
+// Reverse of roe_face_f64, statement by statement from its grouped sums: lamF (5,
+// on the |n|-scaled flux) -> lL, lR.  G is the adjoint of the face's flux sum,
+// B = -G that of |A| dU.
+__device__ __forceinline__ void roe_face_f64_vjp(const Prim<double>& L, const Prim<double>& R, double nx, double ny,
+                                                 double nz, double gm1, double ig, double eps_e, const double lamF[5],
+                                                 Prim<double>& lL, Prim<double>& lR) {
+  // ---- forward (roe_face_f64)
+  const double nn = nx * nx + ny * ny + nz * nz;
+  const bool face = nn > 2.3e-308;
+  const double rn = face ? rsqrt_normal(nn) : 0.0;
+  const double hn = 0.5 * (face ? nn * rn : Tiny<double>::nmag());
+  const double n0 = nx * rn, n1 = ny * rn, n2 = nz * rn;
+  const bool clL = L.rho > Tiny<double>::rho(), clR = R.rho > Tiny<double>::rho();
+  const double rhoL = clL ? L.rho : Tiny<double>::rho(), rhoR = clR ? R.rho : Tiny<double>::rho();
+  const double kL = 0.5 * (L.u * L.u + L.v * L.v + L.w * L.w), kR = 0.5 * (R.u * R.u + R.v * R.v + R.w * R.w);
+  const double eL = L.p * ig + L.rho * kL, eR = R.p * ig + R.rho * kR;
+  const double epL = eL + L.p, epR = eR + R.p;
+  const double irL = rcp_normal(rhoL);
+  const double t2 = fj_max(rhoR * irL, Tiny<double>::rho());
+  const double t = t2 * rsqrt_normal(t2);
+  const double ix = rcp_normal((1.0 + t) * rhoR);
+  const double irR = ix * (1.0 + t), wl = ix * rhoR, wr = t * wl;
+  const double u = wl * L.u + wr * R.u, v = wl * L.v + wr * R.v, w = wl * L.w + wr * R.w;
+  const double HL = epL * irL, HR = epR * irR, H = wl * HL + wr * HR;
+  const double hq = 0.5 * (u * u + v * v + w * w);
+  const double c2r = gm1 * (H - hq);
+  const bool cc2 = c2r > Tiny<double>::c2();
+  const double c2 = cc2 ? c2r : Tiny<double>::c2();
+  const double ic = rsqrt_normal(c2);
+  const double c = c2 * ic, ic2 = ic * ic;
+  const double un = u * n0 + v * n1 + w * n2;
+  const double a2 = fabs(un), su = dsign(un);
+  const double eps = eps_e * (a2 + c);
+  const double e1 = un - c, e5 = un + c;
+  const bool f1 = fabs(e1) < eps, f5 = fabs(e5) < eps;
+  const double ie = f1 || f5 ? __drcp_rn(eps) : 0.0;
+  const double al1 = f1 ? 0.5 * (e1 * e1 * ie + eps) : fabs(e1), al5 = f5 ? 0.5 * (e5 * e5 * ie + eps) : fabs(e5);
+  const double d0 = R.rho - L.rho;
+  const double d1 = R.rho * R.u - L.rho * L.u, d2 = R.rho * R.v - L.rho * L.v, d3 = R.rho * R.w - L.rho * L.w;
+  const double ud = u * d1 + v * d2 + w * d3;
+  const double dp = gm1 * ((eR - eL) - ud + hq * d0);
+  const double dun = (d1 * n0 + d2 * n1 + d3 * n2) - un * d0;
+  const double rhoh = rhoL * t, rc = rhoh * c, rcd = rc * dun, hc2 = 0.5 * ic2;
+  const double m1 = dp - rcd, m5 = dp + rcd, A1 = m1 * hc2, A5 = m5 * hc2;
+  const double s1 = al1 * A1, s5 = al5 * A5, dpc = dp * ic2, sp = s1 + s5, qd = s5 - s1;
+  const double h = sp - a2 * dpc, g = c * qd - a2 * dun;
+  const double unL = L.u * n0 + L.v * n1 + L.w * n2, unR = R.u * n0 + R.v * n1 + R.w * n2;
+  const double mL = rhoL * unL, mR = rhoR * unR;
+
+  // ---- reverse of A_0 = h + a2 d0, A_m = h u_m + g n_m + a2 d_m,
+  //      A_4 = sp H + g un + a2 (ud - hq (d0 + dpc))
+  const double G0 = hn * lamF[0], G1 = hn * lamF[1], G2 = hn * lamF[2], G3 = hn * lamF[3], G4 = hn * lamF[4];
+  const double Gn = G1 * n0 + G2 * n1 + G3 * n2;
+  const double lh = -(G0 + G1 * u + G2 * v + G3 * w);
+  const double lg = -(Gn + G4 * un);
+  double la2 = -(G0 * d0 + G1 * d1 + G2 * d2 + G3 * d3 + G4 * (ud - hq * (d0 + dpc)));
+  double ld0 = -a2 * G0, ld1 = -a2 * G1, ld2 = -a2 * G2, ld3 = -a2 * G3;
+  double lu = -h * G1, lv = -h * G2, lw = -h * G3;
+  const double lsp = lh - G4 * H, lw4 = -a2 * G4;
+  double lH = -G4 * sp, lun = -G4 * g, lud = lw4, lhq = -lw4 * (d0 + dpc);
+  ld0 -= lw4 * hq;
+  const double ldpc = -(lw4 * hq + lh * a2);
+  la2 -= lh * dpc + lg * dun;
+  double lc = lg * qd, ldun = -lg * a2;
+  const double lq = lg * c, ls1 = lsp - lq, ls5 = lsp + lq;
+  const double lal1 = ls1 * A1, lal5 = ls5 * A5, lA1 = ls1 * al1, lA5 = ls5 * al5;
+  const double ldp = hc2 * (lA1 + lA5) + ldpc * ic2, lrcd = hc2 * (lA5 - lA1);
+  const double lic2 = ldpc * dp + 0.5 * (lA1 * m1 + lA5 * m5);
+  ldun += lrcd * rc;
+  const double lrc = lrcd * dun, lrhoh = lrc * c;
+  lc += lrc * rhoh;
+  lun -= ldun * d0;
+  ld0 -= ldun * un;
+  const double ld4 = gm1 * ldp;  // dp = gm1 (d4 - ud + hq d0)
+  lud -= ld4;
+  lhq += ld4 * d0;
+  ld0 += ld4 * hq;
+  ld1 += ldun * n0 + lud * u;
+  ld2 += ldun * n1 + lud * v;
+  ld3 += ldun * n2 + lud * w;
+  lu += lud * d1;
+  lv += lud * d2;
+  lw += lud * d3;
+  // the eigenvalues (Harten's fix where f1, f5)
+  const double l1 = f1 ? lal1 * e1 * ie : lal1 * dsign(e1), l5 = f5 ? lal5 * e5 * ie : lal5 * dsign(e5);
+  const double leps = eps_e * ((f1 ? 0.5 * lal1 * (1.0 - (e1 * ie) * (e1 * ie)) : 0.0) +
+                               (f5 ? 0.5 * lal5 * (1.0 - (e5 * ie) * (e5 * ie)) : 0.0));
+  lun += (l1 + l5) + (la2 + leps) * su;
+  lc += (l5 - l1) + leps;
+  // c, 1/c2 from c2 = gm1 (H - hq); un, hq, u, H from the Roe weights
+  const double tq = cc2 ? gm1 * (0.5 * lc * ic - lic2 * ic2 * ic2) : 0.0;
+  lH += tq;
+  lhq -= tq;
+  lu += lun * n0 + lhq * u;
+  lv += lun * n1 + lhq * v;
+  lw += lun * n2 + lhq * w;
+  const double lwl = lH * HL + lu * L.u + lv * L.v + lw * L.w, lwr = lH * HR + lu * R.u + lv * R.v + lw * R.w;
+  // wl = 1 / (1 + t), wr = 1 - wl, rhoh = rhoL t, t = sqrt(rhoR / rhoL)
+  const double ht = 0.5 * t * ((lwr - lwl) * wl * wl + lrhoh * rhoL);
+  const double lHL = wl * lH, lHR = wr * lH;
+  // the flux sum
+  const double lmL = G0 + G1 * L.u + G2 * L.v + G3 * L.w, lmR = G0 + G1 * R.u + G2 * R.v + G3 * R.w;
+  const double lunL = G4 * epL + lmL * rhoL, lunR = G4 * epR + lmR * rhoR;
+  const double lepL = G4 * unL + lHL * irL, lepR = G4 * unR + lHR * irR;
+  const double leL = lepL - ld4, leR = lepR + ld4;
+  const double lcL = lrhoh * t - ht * irL + lmL * unL - lHL * HL * irL;  // through the clamped densities
+  const double lcR = ht * irR + lmR * unR - lHR * HR * irR;
+  lL.rho = leL * kL - (ld0 + ld1 * L.u + ld2 * L.v + ld3 * L.w) + (clL ? lcL : 0.0);
+  lR.rho = leR * kR + (ld0 + ld1 * R.u + ld2 * R.v + ld3 * R.w) + (clR ? lcR : 0.0);
+  lL.u = mL * G1 + lunL * n0 + wl * lu + L.rho * (leL * L.u - ld1);
+  lL.v = mL * G2 + lunL * n1 + wl * lv + L.rho * (leL * L.v - ld2);
+  lL.w = mL * G3 + lunL * n2 + wl * lw + L.rho * (leL * L.w - ld3);
+  lR.u = mR * G1 + lunR * n0 + wr * lu + R.rho * (leR * R.u + ld1);
+  lR.v = mR * G2 + lunR * n1 + wr * lv + R.rho * (leR * R.v + ld2);
+  lR.w = mR * G3 + lunR * n2 + wr * lw + R.rho * (leR * R.w + ld3);
+  lL.p = Gn + lepL + leL * ig;
+  lR.p = Gn + lepR + leR * ig;
+}
+
 // Reverse of invscd_face_fast: lamF (5, on the |n|-scaled flux) -> lc[s][v], the
 // adjoint of the primitive v (rho, u, v, w, p) of cell s of the four (set).
 template <typename T>
@@ -344,13 +463,17 @@ __device__ __forceinline__ void invscd_face_vjp(const Prim<T> c[4], T kl0, T kl1
   Prim<T> L, R;
   muscl2_fast(c, limiter, L, R);
   const T nf0 = T(0.5) * (kl0 + kr0), nf1 = T(0.5) * (kl1 + kr1), nf2 = T(0.5) * (kl2 + kr2);
-  const T nmag = FastMath<T>::sqrt_nn(nf0 * nf0 + nf1 * nf1 + nf2 * nf2) + Tiny<T>::nmag();
-  const T inv = FastMath<T>::rcp_n(nmag);
-  T g[5];
-#pragma unroll
-  for (int v = 0; v < 5; ++v) g[v] = lamF[v] * nmag;  // F_out = nmag F
   Prim<T> lL, lR;
-  roe_prim_vjp(L, R, nf0 * inv, nf1 * inv, nf2 * inv, gm1, ig, eps_e, g, lL, lR);
+  if constexpr (sizeof(T) == 8) {
+    roe_face_f64_vjp(L, R, nf0, nf1, nf2, gm1, ig, eps_e, lamF, lL, lR);
+  } else {
+    const T nmag = FastMath<T>::sqrt_nn(nf0 * nf0 + nf1 * nf1 + nf2 * nf2) + Tiny<T>::nmag();
+    const T inv = FastMath<T>::rcp_n(nmag);
+    T g[5];
+#pragma unroll
+    for (int v = 0; v < 5; ++v) g[v] = lamF[v] * nmag;  // F_out = nmag F
+    roe_prim_vjp(L, R, nf0 * inv, nf1 * inv, nf2 * inv, gm1, ig, eps_e, g, lL, lR);
+  }
   T o[4];
 #define FJ_MUSCL_VJP(K, field, v)                                                                \
   muscl2_vjp<T, K>(c[0].field, c[1].field, c[2].field, c[3].field, lL.field, lR.field, o);       \

@@ -140,9 +140,14 @@ __device__ __forceinline__ void metric_row(const SplitBlock& B, int32_t N, int r
   k[2] = (T)__ldg(K + 2 * N);
 }
 
-template <typename T, int OCC, int NT, class TB>
-__global__ void __launch_bounds__(NT, OCC) k_fm_fluxes(const TB tab, const Phys ph,
-                                                                 const int flags) {
+// FL: the one kind of term that the kernel is compiled for, or 0: `flags_` at run
+// time.  (A step's kernels test the flags as the small tables' kernel does: without
+// the branches the compiler fuses a multiplication of the viscous terms into their
+// addition to the inviscid ones, and a block of a small table would differ from the
+// same block of a large one in the last bit.  On 4.0 M cells the time is the same.)
+template <typename T, int OCC, int NT, class TB, int FL>
+__global__ void __launch_bounds__(NT, OCC) k_fm_fluxes(const TB tab, const Phys ph, const int flags_) {
+  const int flags = FL ? FL : flags_;
   using M = FastMath<T>;
   const int b = find_block(tab, blockIdx.x);
   if (threadIdx.x == 0) prefetch_fluxes<T, false, true>(tab.b[b], blockIdx.x, NT);
@@ -410,11 +415,11 @@ __device__ __forceinline__ void assemble_cell(const SplitBlock& B, const Cell& x
 // left of its cell and takes the one on its right from lane l+1 by shuffle
 // (lane 31's cell is the next warp's first, for which it only supplies the
 // face), as in the FP32 assembly.
-template <typename T, int OCC, int NW, class TB>
-__global__ void __launch_bounds__(32 * NW, OCC) k_fm_assemble(const TB tab, const int flags,
-                                                                 const int stage, const int next_prims,
-                                                                 const double gm1, const double R,
-                                                                 const double iR, const Phys ph) {
+template <typename T, int OCC, int NW, class TB, int FL>
+__global__ void __launch_bounds__(32 * NW, OCC) k_fm_assemble(const TB tab, const int flags_, const int stage,
+                                                              const int next_prims, const double gm1, const double R,
+                                                              const double iR, const Phys ph) {
+  const int flags = FL ? FL : flags_;
   const int b = find_block_asm(tab, blockIdx.x);
   const Dev& dv = tab.b[b];
   const SplitBlock& B = dv.blk;
@@ -554,15 +559,30 @@ constexpr int kWarps64 = 4;
 constexpr SplitShape kSplitVariants64[] = {{4, 5}, {4, 6}, {4, 4}, {5, 5}, {5, 6}, {3, 5}};
 static_assert(sizeof(kSplitVariants64) / sizeof(kSplitVariants64[0]) == FJ_NUM_SPLIT_VARIANTS, "variant table");
 
-template <int V, class TB>
-void launch_pair64(const TB& tab, int ctas, int asm_ctas, const Phys& ph, int flags, int stage, int np,
-                   cudaStream_t st, cudaEvent_t after_fluxes) {
-  constexpr SplitShape sh = kSplitVariants64[V];
+// Shapes of the right-hand sides with one kind of term only.  Kernels compiled for
+// both and branching on the flags kept the registers of both (128 and 96 a thread):
+// too few warps to cover the viscous terms' loads.  Compiled for their own terms
+// they need 118 / 92 (inviscid) and 80 / 64 (viscous): on 127 x 66 x 51 cells the
+// inviscid call went from 58.0 to 57.1 us, the viscous one from 49.4 to 44.6.
+// (Viscous at {5, 8}, {8, 6}, {6, 10} and inviscid at {5, 6}, {5, 8}, {6, 6}:
+// 0.5 to 4 us slower.)
+constexpr SplitShape kShape64Inv{4, 5}, kShape64Vis{6, 8};
+
+template <int FLUX_OCC, int ASM_OCC, int FL, class TB>
+void launch_pair64(const TB& tab, int ctas, int asm_ctas, const Phys& ph, int stage, int np, cudaStream_t st,
+                   cudaEvent_t after_fluxes) {
   constexpr int nt = 32 * kWarps64;
-  pdl_launch(fm::k_fm_fluxes<double, sh.flux_occ, nt, TB>, ctas, nt, 0, st, tab, ph, flags);
+  pdl_launch(fm::k_fm_fluxes<double, FLUX_OCC, nt, TB, FL>, ctas, nt, 0, st, tab, ph, kRhsInvscd | kRhsViscous);
   if (after_fluxes) cudaEventRecord(after_fluxes, st);
-  pdl_launch(fm::k_fm_assemble<double, sh.asm_occ, kWarps64, TB>, asm_ctas, nt, 0, st, tab, flags, stage, np, ph.gm1,
-             ph.R, 1.0 / ph.R, ph);
+  pdl_launch(fm::k_fm_assemble<double, ASM_OCC, kWarps64, TB, FL>, asm_ctas, nt, 0, st, tab, kRhsInvscd | kRhsViscous,
+             stage, np, ph.gm1, ph.R, 1.0 / ph.R, ph);
+}
+
+template <int V, class TB>
+void launch_both64(const TB& tab, int ctas, int asm_ctas, const Phys& ph, int stage, int np, cudaStream_t st,
+                   cudaEvent_t after_fluxes) {
+  constexpr SplitShape sh = kSplitVariants64[V];
+  launch_pair64<sh.flux_occ, sh.asm_occ, 0>(tab, ctas, asm_ctas, ph, stage, np, st, after_fluxes);
 }
 
 template <typename T, bool K_AOS, int V, class TB>
@@ -583,13 +603,23 @@ int launch_tab(const TB& tab, int ctas, int asm_ctas, const Phys& ph, int flags,
   if constexpr (sizeof(T) == 8) {
     if (!prims_ready)
       pdl_launch(fm::k_fm_prims<double, kWarps64, TB>, ctas, 32 * kWarps64, 0, st, tab, ph.gm1, ph.R, 1.0 / ph.R);
+    if (flags == kRhsInvscd) {
+      launch_pair64<kShape64Inv.flux_occ, kShape64Inv.asm_occ, kRhsInvscd>(tab, ctas, asm_ctas, ph, stage, np, st,
+                                                                           after_fluxes);
+      return prims_ready ? 2 : 3;
+    }
+    if (flags == kRhsViscous) {
+      launch_pair64<kShape64Vis.flux_occ, kShape64Vis.asm_occ, kRhsViscous>(tab, ctas, asm_ctas, ph, stage, np, st,
+                                                                            after_fluxes);
+      return prims_ready ? 2 : 3;
+    }
     switch (variant) {
-      case 1: launch_pair64<1>(tab, ctas, asm_ctas, ph, flags, stage, np, st, after_fluxes); break;
-      case 2: launch_pair64<2>(tab, ctas, asm_ctas, ph, flags, stage, np, st, after_fluxes); break;
-      case 3: launch_pair64<3>(tab, ctas, asm_ctas, ph, flags, stage, np, st, after_fluxes); break;
-      case 4: launch_pair64<4>(tab, ctas, asm_ctas, ph, flags, stage, np, st, after_fluxes); break;
-      case 5: launch_pair64<5>(tab, ctas, asm_ctas, ph, flags, stage, np, st, after_fluxes); break;
-      default: launch_pair64<0>(tab, ctas, asm_ctas, ph, flags, stage, np, st, after_fluxes);
+      case 1: launch_both64<1>(tab, ctas, asm_ctas, ph, stage, np, st, after_fluxes); break;
+      case 2: launch_both64<2>(tab, ctas, asm_ctas, ph, stage, np, st, after_fluxes); break;
+      case 3: launch_both64<3>(tab, ctas, asm_ctas, ph, stage, np, st, after_fluxes); break;
+      case 4: launch_both64<4>(tab, ctas, asm_ctas, ph, stage, np, st, after_fluxes); break;
+      case 5: launch_both64<5>(tab, ctas, asm_ctas, ph, stage, np, st, after_fluxes); break;
+      default: launch_both64<0>(tab, ctas, asm_ctas, ph, stage, np, st, after_fluxes);
     }
   } else {
     if (!prims_ready)

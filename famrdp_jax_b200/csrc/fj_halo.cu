@@ -335,9 +335,9 @@ struct CopyFillTableN {
   short order[NL];
 };
 using CopyFillTable = CopyFillTableN<kMaxFillBlocks, kMaxLinksPerLaunch>;
-// one block with a link on each face at most: 1.5 KB of parameters instead of 28
-using HaloTable1 = HaloTableN<6>;
-using CopyFillTable1 = CopyFillTableN<1, 6>;
+// The parameters that a launch uploads are cut to the number of blocks: 1 or
+// sd::kFewBlocks blocks with a link on each face at most, else kMaxFillBlocks and
+// kMaxLinksPerLaunch (1.5, 9 and 28 KB).
 static_assert(sizeof(HaloTable) + sizeof(CopyFillTable) <= 32764, "kernel parameter space");
 
 // dst[b] := src[b] cell by cell, except the ghost cells a link of block b
@@ -527,26 +527,29 @@ int copy_fill(fj_ctx* ctx, const fj_block* blocks, double* const* dst, int nbloc
                           : (wide ? k_copy_fill<0, W, NB, NL> : k_copy_fill<0, 1, NB, NL>);
     pdl_launch(kern, dim3((unsigned)ctas), kThreads, 0, st, ht, ft);
   };
-  if (nblocks == 1 && tab.n <= 6) {
-    HaloTable1 h1;
-    h1.n = tab.n;
-    CopyFillTable1 f1;
-    f1.nb = 1;
-    f1.ghost = ct.ghost;
-    f1.cells = ct.cells;
-    f1.gm1 = ct.gm1;
-    f1.R = ct.R;
-    f1.p_ref = ct.p_ref;
-    std::copy(&ct.set[0][0], &ct.set[0][0] + 5 * kMaxBcSets, &f1.set[0][0]);
-    f1.b[0] = ct.b[0];
-    for (int L = 0; L < tab.n; ++L) {
-      h1.d[L] = tab.d[L];
-      f1.order[L] = ct.order[L];
-    }
-    launch(std::integral_constant<int, 1>(), std::integral_constant<int, 6>(), h1, f1);
-  } else {
+  auto launch_few = [&](auto nb) {
+    constexpr int NB = decltype(nb)::value, NL = 6 * NB;
+    HaloTableN<NL> h;
+    CopyFillTableN<NB, NL> f;
+    h.n = tab.n;
+    f.nb = ct.nb;
+    f.ghost = ct.ghost;
+    f.cells = ct.cells;
+    f.gm1 = ct.gm1;
+    f.R = ct.R;
+    f.p_ref = ct.p_ref;
+    std::memcpy(f.set, ct.set, sizeof(ct.set));
+    std::copy(ct.b, ct.b + nblocks, f.b);
+    std::copy(tab.d, tab.d + tab.n, h.d);
+    std::copy(ct.order, ct.order + tab.n, f.order);
+    launch(nb, std::integral_constant<int, NL>(), h, f);
+  };
+  if (nblocks == 1 && tab.n <= 6)
+    launch_few(std::integral_constant<int, 1>());
+  else if (nblocks <= sd::kFewBlocks && tab.n <= 6 * sd::kFewBlocks)
+    launch_few(std::integral_constant<int, sd::kFewBlocks>());
+  else
     launch(std::integral_constant<int, kMaxFillBlocks>(), std::integral_constant<int, kMaxLinksPerLaunch>(), tab, ct);
-  }
   ctx->launches += 1;
   s = launch_status(ctx, "copy-fill launch");
   if (s == FJ_OK) *done = true;
@@ -724,7 +727,7 @@ int halo_transpose(fj_ctx* ctx, const fj_block* lam, int nblocks, const fj_link*
     pdl_launch(give, grid, kThreads, 0, st, t, scratch);
   };
   if (tab.n <= 6) {  // a block's own faces: 0.7 KB of parameters instead of 21
-    HaloTable1 t;
+    HaloTableN<6> t;
     t.n = tab.n;
     for (int L = 0; L < tab.n; ++L) t.d[L] = tab.d[L];
     launch(t, k_halo_transpose<true, 6>, k_halo_transpose<false, 6>);

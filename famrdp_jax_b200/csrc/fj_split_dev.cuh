@@ -43,16 +43,24 @@ struct Tile {
 struct Dev {
   SplitBlock blk;
   FastDiv dk, dj;  // n / nk, n / nj
-  Tile tile;       // k_small_stage's boxes of this block
 };
 
-// The blocks of a launch, a kernel parameter.  TableN<1> serves launches of one
-// block: the kernels then read its fields at fixed parameter offsets, without
-// the block search, and 200 bytes of parameters are uploaded instead of 13 KB.
+// The blocks of a launch, a kernel parameter, which each launch uploads: in tables
+// of 1, kFewBlocks or kMaxSplitBlocks blocks (0.2, 1.4 and 11 KB).  TableN<1> serves
+// launches of one block: the kernels then read its fields at fixed parameter
+// offsets, without the block search.  (One step() of four 20^3 blocks, where the
+// host sets the pace: 60.4 us with tables of 1 and 64 blocks only, 46.6 with this.)
 template <int NB>
 struct TableN {
   int n;
   Dev b[NB];
+};
+constexpr int kFewBlocks = 8;
+
+// k_small_stage's table: each block's boxes as well.
+template <int NB>
+struct SmallTableN : TableN<NB> {
+  Tile tile[NB];
 };
 using Table = TableN<kMaxSplitBlocks>;
 static_assert(sizeof(Table) <= 32764, "kernel parameter space (sm_70+, CUDA 12.1+)");

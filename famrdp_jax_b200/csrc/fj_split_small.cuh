@@ -93,15 +93,15 @@ struct BoxSrc {
   }
 };
 
-template <typename T, bool K_AOS, class TB>
+template <typename T, bool K_AOS, int NB>
 __global__ void __launch_bounds__(32 * kWarpsOf<T>, 1)
-    k_small_stage(const TB tab, const int flags, const int stage, const int next_prims, const double gm1,
+    k_small_stage(const SmallTableN<NB> tab, const int flags, const int stage, const int next_prims, const double gm1,
                   const double R, const double iR, const Phys ph) {
   constexpr int kWarps = kWarpsOf<T>;
   extern __shared__ __align__(16) unsigned char smem[];
-  const Dev& d = tab.b[find_block_asm(tab, blockIdx.x)];
-  const SplitBlock& B = d.blk;
-  const Tile& S = d.tile;
+  const int blk = find_block_asm(static_cast<const TableN<NB>&>(tab), blockIdx.x);
+  const SplitBlock& B = tab.b[blk].blk;
+  const Tile& S = tab.tile[blk];
   const int ti = S.t[0], tj = S.t[1], tk = S.t[2];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int ni = B.ni, nj = B.nj, nk = B.nk;

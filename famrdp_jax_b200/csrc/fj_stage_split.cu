@@ -8,22 +8,26 @@
 //                    fill a step's start state)
 //   k_split_fluxes   per cell c: the viscous flux components G(c)
 //                    (rhs/viscous.py:36-105, neighbours wrap around the padded
-//                    block like jnp.roll) and the three Roe faces c | c+e_a
-//                    (rhs/invscd.py:53-100) for c_a in [1, n_a-3]
-//   k_split_assemble per cell: -(F_a(c) - F_a(c-e_a)) / (vol + 1e-300) over
+//                    block like jnp.roll) and the Roe faces c | c+e_a of the
+//                    axes i and j (rhs/invscd.py:53-100) for c_a in [1, n_a-3]
+//   k_split_assemble per cell: the Roe faces along k (a lane's right face by
+//                    shuffle), -(F_a(c) - F_a(c-e_a)) / (vol + 1e-300) over
 //                    the axes where c_a in [2, n_a-3] (rhs/invscd.py:119-131),
 //                    the viscous divergence of G with the cell's own kxyz
 //                    (rhs/viscous.py:86-117) and the TVD-RK3 combine
 //                    (solver/step.py:45-53)
 //
-// Intermediates live in scratch in the flux type T (float on the FP32-flux
-// path, double on the FP64 path) as per-cell RECORDS, so that a cell's fields
-// sit at compile-time offsets from one address and move with 16-byte vector
-// loads and stores:
-//   P  8 T per cell: rho u v w p T (2 pad)
-//   F 16 T per cell: the faces c | c+e_i, c | c+e_j, c | c+e_k, 5 T each (1 pad)
-//   G 12 T per cell: tau_00 tau_01 tau_02 tau_11 tau_12 tau_22, the energy
-//     flux components 0..2 (3 pad)
+// (fm:: for the FP64 path, whose face and viscous fluxes are field-major).  Small
+// tables run a whole stage in one launch (fj_split_small.cuh).
+//
+// Intermediates live in scratch in the flux type.  On the FP32-flux path they are
+// per-cell RECORDS, so that a cell's fields sit at compile-time offsets from one
+// address and move with 16- and 32-byte vector loads and stores:
+//   P  8 floats per cell: rho u v w p' T (2 pad)
+//   F  8 floats per cell: the face c | c+e_i (5) and the first three of
+//      c | c+e_j; the other two of c | c+e_j as a pair in an array of their own
+//   G  8 floats per cell: tau_00 tau_01 tau_02 tau_11 tau_12 tau_22, the energy
+//      flux components 0 and 1; component 2 in an array of its own
 // A plan also keeps the metrics as records (kRecK<T> T per cell: the nine
 // kxyz[l][m], l-major, then pad), converted once from the caller's FP64
 // field-major kxyz; without one the kernels read kxyz field by field.
@@ -640,9 +644,11 @@ int launch_tab(const TB& tab, int ctas, int asm_ctas, const Phys& ph, int flags,
 // A small table: the primitives (unless the producer of q left them), then the
 // whole stage in one launch.  ctas: boxes (numbered by cta_begin_asm); prim_ctas:
 // 128-cell ranges (by cta_begin).
-template <typename T, bool K_AOS, class TB>
-int launch_small(const TB& tab, int ctas, int prim_ctas, size_t smem, const Phys& ph, int flags, int stage,
+template <typename T, bool K_AOS, int NB>
+int launch_small(const SmallTableN<NB>& small_tab, int ctas, int prim_ctas, size_t smem, const Phys& ph, int flags, int stage,
                  bool prims_ready, bool next_prims, cudaStream_t st, cudaEvent_t after_fluxes) {
+  using TB = TableN<NB>;
+  const TB& tab = small_tab;
   if (!prims_ready) {
     if constexpr (sizeof(T) == 8)
       pdl_launch(fm::k_fm_prims<double, kWarps64, TB>, prim_ctas, 32 * kWarps64, 0, st, tab, ph.gm1, ph.R, 1.0 / ph.R);
@@ -650,9 +656,9 @@ int launch_small(const TB& tab, int ctas, int prim_ctas, size_t smem, const Phys
       pdl_launch(k_split_prims<T, kWarps32, TB>, prim_ctas, 32 * kWarps32, 0, st, tab, ph.gm1, ph.R, 1.0 / ph.R,
                  K_AOS ? ph.p_ref : 0.0);
   }
-  auto kern = small::k_small_stage<T, K_AOS, TB>;
+  auto kern = small::k_small_stage<T, K_AOS, NB>;
   if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  pdl_launch(kern, ctas, 32 * small::kWarpsOf<T>, smem, st, tab, flags, stage, next_prims ? 1 : 0, ph.gm1, ph.R,
+  pdl_launch(kern, ctas, 32 * small::kWarpsOf<T>, smem, st, small_tab, flags, stage, next_prims ? 1 : 0, ph.gm1, ph.R,
              1.0 / ph.R, ph);
   if (after_fluxes) cudaEventRecord(after_fluxes, st);
   return prims_ready ? 1 : 2;
@@ -671,6 +677,7 @@ int launch_split(fj_ctx* ctx, const SplitBlock* blocks, int nblocks, const Phys&
     int64_t cells = 0;
     for (int t = 0; t < tab.n; ++t) cells += (int64_t)blocks[base + t].ni * blocks[base + t].nj * blocks[base + t].nk;
     // a small table runs in one launch if its boxes fit the SMs once
+    Tile tiles[kMaxSplitBlocks];
     bool small_tab = cells <= small::kMaxCellsPerSm * (int64_t)sms;
     int boxes = 0;
     size_t smem = 0;
@@ -678,8 +685,8 @@ int launch_split(fj_ctx* ctx, const SplitBlock* blocks, int nblocks, const Phys&
       const SplitBlock& sb = blocks[base + t];
       const int64_t N = (int64_t)sb.ni * sb.nj * sb.nk;
       tab.b[t].blk.cta_begin_asm = boxes;
-      boxes += small::cut(sb.ni, sb.nj, sb.nk, std::max(1, (int)(sms * N / cells)), tab.b[t].tile);
-      smem = std::max(smem, small::values(tab.b[t].tile) * sizeof(T));
+      boxes += small::cut(sb.ni, sb.nj, sb.nk, std::max(1, (int)(sms * N / cells)), tiles[t]);
+      smem = std::max(smem, small::values(tiles[t]) * sizeof(T));
       small_tab = boxes <= sms;
     }
     constexpr int nw = sizeof(T) == 8 ? kWarps64 : kWarps32, fcells = 32 * nw, acells = 31 * nw;
@@ -706,19 +713,34 @@ int launch_split(fj_ctx* ctx, const SplitBlock* blocks, int nblocks, const Phys&
       return set_err(ctx, FJ_ERR_INVALID_ARGUMENT, "the FP64 split path reads kxyz directly");
     // the event marks the first chunk's flux launch
     cudaEvent_t ev = base == 0 ? after_fluxes : nullptr;
-    auto launch = [&](const auto& t, auto aos) {
+    auto launch = [&](auto nb, auto aos) {
+      constexpr int NB = decltype(nb)::value;
       constexpr bool AOS = decltype(aos)::value;
-      if (small_tab)
-        return launch_small<T, AOS>(t, boxes, ctas, smem, ph, flags, stage, prims_ready, next_prims, st, ev);
-      return launch_tab<T, AOS>(t, ctas, asm_ctas, ph, flags, stage, prims_ready, next_prims, variant, st, ev);
-    };
-    auto pick = [&](const auto& t) {
-      if constexpr (sizeof(T) == 4) {
-        if (k_aos) return launch(t, std::true_type());
+      if (small_tab) {
+        SmallTableN<NB> t;
+        t.n = tab.n;
+        std::copy(tab.b, tab.b + tab.n, t.b);
+        std::copy(tiles, tiles + tab.n, t.tile);
+        return launch_small<T, AOS, NB>(t, boxes, ctas, smem, ph, flags, stage, prims_ready, next_prims, st, ev);
       }
-      return launch(t, std::false_type());
+      if constexpr (NB == kMaxSplitBlocks) {
+        return launch_tab<T, AOS>(tab, ctas, asm_ctas, ph, flags, stage, prims_ready, next_prims, variant, st, ev);
+      } else {
+        TableN<NB> t;
+        t.n = tab.n;
+        std::copy(tab.b, tab.b + tab.n, t.b);
+        return launch_tab<T, AOS>(t, ctas, asm_ctas, ph, flags, stage, prims_ready, next_prims, variant, st, ev);
+      }
     };
-    ctx->launches += tab.n == 1 ? pick(TableN<1>{1, {tab.b[0]}}) : pick(tab);
+    auto pick = [&](auto nb) {
+      if constexpr (sizeof(T) == 4) {
+        if (k_aos) return launch(nb, std::true_type());
+      }
+      return launch(nb, std::false_type());
+    };
+    ctx->launches += tab.n == 1             ? pick(std::integral_constant<int, 1>())
+                     : tab.n <= kFewBlocks  ? pick(std::integral_constant<int, kFewBlocks>())
+                                            : pick(std::integral_constant<int, kMaxSplitBlocks>());
     int s = launch_status(ctx, "split stage launch");
     if (s != FJ_OK) return s;
   }

@@ -141,7 +141,7 @@ int fj_ctx_set_pipeline(fj_ctx* ctx, int pipeline, int seg, int tile);
 /* Launch shape of the RHS adjoint's face and viscous kernels (a tuning knob;
  * results agree to the rounding of atomic accumulation order): 0 = the
  * fastest measured (default; face kernel register-capped per precision,
- * viscous kernel capped at 64 registers; with FP32 fluxes both VJPs in one
+ * viscous kernel at 64 registers, FP64 128; with FP32 fluxes both VJPs in one
  * launch of interleaved CTAs), 1 = face kernel uncapped, 2 = the
  * other face cap, 3 = 0 and 4 = 2 with the viscous kernel uncapped.  The
  * reference has no counterpart. */
@@ -401,7 +401,7 @@ int fj_plan_destroy(fj_plan* plan);
 /* One TVD-RK3 stage (1..3) of every block of the plan, without the halo fill
  * (solver/step.py:45-53): out[b] from q[b] (stage input) and q0[b] (step start
  * state); out[b] may alias q0[b], never q[b].  With the split pipeline this is
- * three launches over all blocks. */
+ * three launches over all blocks (two for small tables). */
 int fj_plan_stage(fj_plan* plan, double* const* q, double* const* q0, double* const* out,
                   double dt, int stage, void* stream);
 

@@ -60,3 +60,21 @@ def test_small_tables_match_large(cuda_device, shapes, precision, limiter):
             assert torch.equal(a, b)
         else:
             assert rel_l2(host(a), host(b)) <= 1e-14
+
+
+@pytest.mark.parametrize("precision", ["f32", "f64"])
+@pytest.mark.parametrize("shape", [(5, 6, 9), (20, 33, 40)])
+@pytest.mark.parametrize("n", [2, 8, 9, 65])
+def test_tables_of_every_size_agree(cuda_device, n, shape, precision):
+    """n independent blocks, all the same: tables of few, many and more blocks than a
+    launch takes; every block must come out with the bits of the first."""
+    one = tuple(dev(x) for x in random_block(shape, 60))
+    qs = [one[0].clone() for _ in range(n)]
+    outs = _step(_plan([one] * n, "minmod", precision), qs)
+    ref = _step(_plan([one] * (n + 1), "minmod", precision), qs + [one[0]])
+    assert torch.isfinite(ref[0]).all()
+    for a in outs + ref:
+        if precision == "f32":
+            assert torch.equal(a, ref[0])
+        else:
+            assert rel_l2(host(a), host(ref[0])) <= 1e-14

@@ -74,10 +74,11 @@ STEP_BYTES = {"f64": 560.0, "f32": 452.0}
 # DRAM bytes per padded cell of one stage-2 launch group (dram__bytes_read +
 # dram__bytes_write summed over its kernels), measured by ncu on
 # `bench.py --stage-only --n 96` (4 blocks of 100^3 padded cells, 4.0 M) and
-# scaled per cell: split FP32 59 + 147 + 283 B (primitives, fluxes, assembly),
-# split FP64 75 + 259 + 406 B; the fused tile kernel 220 B (its primitive
+# scaled per cell: split FP32 60 + 147 + 282 B (primitives, fluxes, assembly),
+# split FP64 74 + 259 + 399 B, of which blocks with uniform metrics read up to 96
+# and 144 B less; the fused tile kernel 220 B (its primitive
 # launch not included)
-STAGE_TRAFFIC = {("f32", "split"): 489.0, ("f64", "split"): 740.0, ("f32", "tile"): 220.0}
+STAGE_TRAFFIC = {("f32", "split"): 488.0, ("f64", "split"): 733.0, ("f32", "tile"): 220.0}
 
 
 def _peaks():
@@ -473,7 +474,8 @@ def _stage_roofline(plan, q0s, dt, prec, padded_cells):
     return {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
             "traffic": traffic * padded_cells * (3 if whole_step else 1) if traffic else None,
             "traffic_note": f"{traffic:.0f} B per padded cell (ncu dram__bytes_read+write of the stage-2 group on "
-                            f"4 x 100^3 padded cells) x the cells of one launch" if traffic else None,
+                            f"4 x 100^3 padded curvilinear cells; less where metrics are uniform) x the cells of one "
+                            f"launch" if traffic else None,
             "kernel": what, "stage_kernel": kern,
             "alg_bytes_per_cell": STAGE_BYTES[prec], "alg_bytes_per_launch": alg, "launch_ms": stage_ms,
             "peak_kind": peak_kind}

@@ -470,7 +470,8 @@ def _stage_roofline(plan, q0s, dt, prec, padded_cells):
             "that fills the padded primitive planes)" if kern == "tile" else
             "one whole TVD-RK3 step of all blocks (persistent kernel: halo, boundary faces, primitives and the "
             "three stages in one launch after a counter reset; algorithmic bytes of three stages)" if whole_step
-            else "one TVD-RK3 stage of all blocks (split pipeline: prims, fluxes, assembly; 3 launches)")
+            else "one TVD-RK3 stage of all blocks (split pipeline: prims, fluxes, assembly; 3 launches, 2 for small "
+            "tables)")
     return {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
             "traffic": traffic * padded_cells * (3 if whole_step else 1) if traffic else None,
             "traffic_note": f"{traffic:.0f} B per padded cell (ncu dram__bytes_read+write of the stage-2 group on "

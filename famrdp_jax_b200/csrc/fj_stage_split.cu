@@ -368,12 +368,14 @@ __device__ __forceinline__ void assemble_inv(const SplitBlock& B, const Cell& x,
   // every face value in one batch of loads: a face that does not count is read
   // at the cell itself and left out of the sum, not branched around
   const bool on_i = x.i >= 2 && x.i <= x.ni - 3, on_j = x.j >= 2 && x.j <= x.nj - 3, on_k = x.k >= 2 && x.k <= x.nk - 3;
-  const double ivd = rcp_normal(__ldg(B.vol + x.c) + 1e-300);
+  // (the caller's volumes may be anything: the general reciprocal, 0 of an infinite
+  // volume; a cell with no face that counts keeps 0 whatever its volume is)
+  const double neg_ivd = on_i || on_j || on_k ? -__drcp_rn(__ldg(B.vol + x.c) + 1e-300) : 0.0;
   T di[5], dj[5], dk[5];
   src.faces(on_i, on_j, di, dj, dk);
 #pragma unroll
   for (int v = 0; v < 5; ++v)  // axis by axis like the reference
-    r[v] = -((on_i ? di[v] : 0.0) + (on_j ? dj[v] : 0.0) + (on_k ? dk[v] : 0.0)) * ivd;
+    r[v] = ((on_i ? di[v] : 0.0) + (on_j ? dj[v] : 0.0) + (on_k ? dk[v] : 0.0)) * neg_ivd;
 }
 
 // sum over l of 0.5 kxyz[l][jj] (G(c+e_l) - G(c-e_l)): the 18 components of an axis

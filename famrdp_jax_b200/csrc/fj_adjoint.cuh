@@ -14,16 +14,26 @@ template <typename T> __device__ __forceinline__ T dsign(T x) {
   return x > T(0) ? T(1) : (x < T(0) ? T(-1) : T(0));
 }
 
+// Both nonzero and of one sign, whatever their size (the product of two small
+// numbers underflows to 0).
+__device__ __forceinline__ bool same_sign(float a, float b) {
+  return (__float_as_int(a) ^ __float_as_int(b)) >= 0 && a != 0.0f && b != 0.0f;
+}
+__device__ __forceinline__ bool same_sign(double a, double b) {
+  return (__double2hiint(a) ^ __double2hiint(b)) >= 0 && a != 0.0 && b != 0.0;
+}
+
 // Reverse of muscl2_fast for one variable: lamL, lamR -> lamc[0..3] (set).
 template <typename T, bool MINMOD>
 __device__ __forceinline__ void muscl2_vjp(T c0, T c1, T c2, T c3, T lamL, T lamR, T lamc[4]) {
   const T d0 = c1 - c0, d1 = c2 - c1, d2 = c3 - c2;
   // L = c1 + 0.5 sL(d0, d1); R = c2 - 0.5 sR(d1, d2)
   const T lsL = T(0.5) * lamL, lsR = T(-0.5) * lamR;
-  const bool s0 = d0 * d1 > T(0), s1 = d1 * d2 > T(0);
   if constexpr (MINMOD) {
     // minmod is its smaller argument where the signs agree: the slope's adjoint
-    // goes to that one (selections, no 0/1 weights to multiply by)
+    // goes to that one (selections, no 0/1 weights to multiply by).  The signs are
+    // compared as muscl2_one does: slopes too small to multiply keep their adjoint
+    const bool s0 = same_sign(d0, d1), s1 = same_sign(d1, d2);
     const bool a0 = fj_abs(d0) < fj_abs(d1), a1 = fj_abs(d1) < fj_abs(d2);
     const T ld0 = s0 && a0 ? lsL : T(0);
     const T ld1 = (s0 && !a0 ? lsL : T(0)) + (s1 && a1 ? lsR : T(0));
@@ -33,6 +43,7 @@ __device__ __forceinline__ void muscl2_vjp(T c0, T c1, T c2, T c3, T lamL, T lam
     lamc[2] = lamR + ld1 - ld2;
     lamc[3] = ld2;
   } else {  // van Leer 2ab/(a+b) where ab > 0
+    const bool s0 = d0 * d1 > T(0), s1 = d1 * d2 > T(0);
     const T e0 = d0 + d1, e1 = d1 + d2;
     const T pa0 = s0 ? T(2) * d1 * d1 / (e0 * e0) : T(0);
     const T pb0 = s0 ? T(2) * d0 * d0 / (e0 * e0) : T(0);

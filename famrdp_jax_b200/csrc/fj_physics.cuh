@@ -444,6 +444,14 @@ __device__ __forceinline__ double rcp_normal(double x) {
   const double e = fma(-x, y, 1.0);
   return fma(y, fma(e, e, e), y);
 }
+// 1/x of any x: where the seed is no start for the step (0, infinities, NaN, a
+// result below the normal range), the seed itself: inf, 0, NaN, 0.
+__device__ __forceinline__ double rcp_any(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y, 1.0);
+  return fabs(e) < 0.5 ? fma(y, fma(e, e, e), y) : y;
+}
 __device__ __forceinline__ double rsqrt_normal(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));

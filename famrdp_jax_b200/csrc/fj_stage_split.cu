@@ -370,7 +370,7 @@ __device__ __forceinline__ void assemble_inv(const SplitBlock& B, const Cell& x,
   const bool on_i = x.i >= 2 && x.i <= x.ni - 3, on_j = x.j >= 2 && x.j <= x.nj - 3, on_k = x.k >= 2 && x.k <= x.nk - 3;
   // (the caller's volumes may be anything: the general reciprocal, 0 of an infinite
   // volume; a cell with no face that counts keeps 0 whatever its volume is)
-  const double neg_ivd = on_i || on_j || on_k ? -__drcp_rn(__ldg(B.vol + x.c) + 1e-300) : 0.0;
+  const double neg_ivd = on_i || on_j || on_k ? -rcp_any(__ldg(B.vol + x.c) + 1e-300) : 0.0;
   T di[5], dj[5], dk[5];
   src.faces(on_i, on_j, di, dj, dk);
 #pragma unroll

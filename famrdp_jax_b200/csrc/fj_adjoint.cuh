@@ -348,7 +348,12 @@ __device__ __forceinline__ void roe_prim_vjp(const Prim<T>& L, const Prim<T>& R,
 
 // Reverse of roe_face_f64, statement by statement from its grouped sums: lamF (5,
 // on the |n|-scaled flux) -> lL, lR.  G is the adjoint of the face's flux sum,
-// B = -G that of |A| dU.
+// -G that of |A| dU.  The forward's dissipation is small (jumps), its adjoint is
+// not: what enters it, c, 1/c^2 and the Roe averages, is rounded about once here
+// (c and 1/c^2 corrected by their residuals, averages as L + wr (R - L)).  The
+// error of a right-hand side's gradient against extended precision is 2.7e-16 so,
+// 3.1e-16 with the forward's own forms, 2.8e-16 in the ungrouped reverse; the
+// gradient of 20 steps on 48^3 takes 5.51 ms instead of 5.46.
 __device__ __forceinline__ void roe_face_f64_vjp(const Prim<double>& L, const Prim<double>& R, double nx, double ny,
                                                  double nz, double gm1, double ig, double eps_e, const double lamF[5],
                                                  Prim<double>& lL, Prim<double>& lR) {
@@ -356,7 +361,7 @@ __device__ __forceinline__ void roe_face_f64_vjp(const Prim<double>& L, const Pr
   const double nn = nx * nx + ny * ny + nz * nz;
   const bool face = nn > 2.3e-308;
   const double rn = face ? rsqrt_normal(nn) : 0.0;
-  const double hn = 0.5 * (face ? nn * rn : Tiny<double>::nmag());
+  const double hn = 0.5 * (face ? sqrt_normal(nn, rn) : Tiny<double>::nmag());
   const double n0 = nx * rn, n1 = ny * rn, n2 = nz * rn;
   const bool clL = L.rho > Tiny<double>::rho(), clR = R.rho > Tiny<double>::rho();
   const double rhoL = clL ? L.rho : Tiny<double>::rho(), rhoR = clR ? R.rho : Tiny<double>::rho();
@@ -368,14 +373,14 @@ __device__ __forceinline__ void roe_face_f64_vjp(const Prim<double>& L, const Pr
   const double t = t2 * rsqrt_normal(t2);
   const double ix = rcp_normal((1.0 + t) * rhoR);
   const double irR = ix * (1.0 + t), wl = ix * rhoR, wr = t * wl;
-  const double u = wl * L.u + wr * R.u, v = wl * L.v + wr * R.v, w = wl * L.w + wr * R.w;
-  const double HL = epL * irL, HR = epR * irR, H = wl * HL + wr * HR;
+  const double u = fma(wr, R.u - L.u, L.u), v = fma(wr, R.v - L.v, L.v), w = fma(wr, R.w - L.w, L.w);
+  const double HL = epL * irL, HR = epR * irR, H = fma(wr, HR - HL, HL);
   const double hq = 0.5 * (u * u + v * v + w * w);
   const double c2r = gm1 * (H - hq);
   const bool cc2 = c2r > Tiny<double>::c2();
   const double c2 = cc2 ? c2r : Tiny<double>::c2();
   const double ic = rsqrt_normal(c2);
-  const double c = c2 * ic, ic2 = ic * ic;
+  const double c = sqrt_normal(c2, ic), i2 = ic * ic, ic2 = fma(i2, fma(-c2, i2, 1.0), i2);
   const double un = u * n0 + v * n1 + w * n2;
   const double a2 = fabs(un), su = dsign(un);
   const double eps = eps_e * (a2 + c);

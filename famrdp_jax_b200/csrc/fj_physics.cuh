@@ -434,8 +434,14 @@ __device__ __forceinline__ void roe_prim(const Prim<T>& L, const Prim<T>& R, T n
 
 // 1/x, 1/sqrt(x) and sqrt(x) in FP64 for a normal, finite x (whose result is normal
 // too), without the special cases of the general functions: the hardware's seed
-// (relative error 1e-6, measured) and one third-order step, y (1 + e + e^2) with
-// e = 1 - x y, and y (1 + e/2 + 3 e^2/8) with e = 1 - x y^2.
+// (relative error 1e-6, measured) and one step of Householder's iteration of the
+// second order (A. S. Householder, The Numerical Treatment of a Single Nonlinear
+// Equation, 1970): the series of 1/(1 - e) and 1/sqrt(1 - e) up to e^2, e the
+// seed's residual, which the FMA gives without rounding (P. Markstein, IBM J. Res.
+// Dev. 34(1), 1990).  The root takes one more such step from x times the reciprocal
+// root.  Largest relative errors over 2^-1020 .. 2^1000 (4 million arguments), in
+// units of 2^-53 (half a unit in the last place): rcp_normal 1.00, rsqrt_normal
+// 1.25, sqrt_normal 1.00, held to 1.02, 2.05 and 1.02 by tests/test_gpu_f64_roots.py.
 __device__ __forceinline__ double rcp_normal(double x) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));

@@ -438,6 +438,11 @@ int fj_ctx_create(fj_ctx** out) {
     delete c;
     return FJ_ERR_CUDA;
   }
+  if (cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess || c->sms <= 0) {
+    cudaGetLastError();
+    delete c;
+    return FJ_ERR_CUDA;
+  }
   *out = c;
   return FJ_OK;
 }

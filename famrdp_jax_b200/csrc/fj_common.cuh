@@ -14,6 +14,9 @@
 
 struct fj_ctx {
   int device = 0;
+  int sms = 148;             // SMs of the device
+  unsigned small_ready = 0;  // instances of k_small_stage whose shared-memory limit is set (fj_stage_split.cu)
+  int small_device = -1;     // on this device
   void* ws = nullptr;        // scratch owned by the context (stage buffers, fluxes)
   size_t ws_bytes = 0;
   void* red = nullptr;       // small reduction scratch (partials + counters)

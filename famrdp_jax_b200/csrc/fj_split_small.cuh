@@ -54,6 +54,11 @@ inline size_t values(const sd::Tile& T) {
   return 9 * (size_t)((a + 2) * (b + 2) * (c + 2)) + 5 * (size_t)((a + 1) * b * c + a * (b + 1) * c + a * b * (c + 1));
 }
 
+// The same for the largest box: every launch may use this much.
+constexpr int kMaxValues = 9 * (kMaxI + 2) * (kMaxJ + 2) * (kMaxK + 2) +
+                           5 * ((kMaxI + 1) * kMaxJ * kMaxK + kMaxI * (kMaxJ + 1) * kMaxK + kMaxI * kMaxJ * (kMaxK + 1));
+static_assert(kMaxValues * sizeof(double) <= 227 * 1024, "shared memory of a CTA");
+
 // The assembly's view of the shared memory: the slots of one cell.
 template <typename T>
 struct BoxSrc {

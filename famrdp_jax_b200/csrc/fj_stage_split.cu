@@ -643,6 +643,28 @@ int launch_tab(const TB& tab, int ctas, int asm_ctas, const Phys& ph, int flags,
   return prims_ready ? 2 : 3;
 }
 
+// Raises the shared-memory limit of one instance of k_small_stage on the current
+// device.  The limit belongs to the function on the device, which other contexts
+// launch from other threads: it is always the largest box's, never this table's,
+// so that nobody's setting refuses another's launch.  Once per context, device and
+// instance (a call for each launch is host time in steps whose pace the host sets).
+template <typename T, bool K_AOS, int NB>
+int small_ready(fj_ctx* ctx) {
+  constexpr unsigned bit = 1u << ((sizeof(T) == 4 ? 0 : 1) + (K_AOS ? 2 : 0) + (NB == 1 ? 0 : NB == kFewBlocks ? 4 : 8));
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess && dev != ctx->small_device) {
+    ctx->small_device = dev;
+    ctx->small_ready = 0;
+  }
+  if (e == cudaSuccess && !(ctx->small_ready & bit)) {
+    e = cudaFuncSetAttribute(small::k_small_stage<T, K_AOS, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             small::kMaxValues * (int)sizeof(T));
+    if (e == cudaSuccess) ctx->small_ready |= bit;
+  }
+  return e == cudaSuccess ? FJ_OK : cuda_status(ctx, e, "small stage: shared memory attribute");
+}
+
 // A small table: the primitives (unless the producer of q left them), then the
 // whole stage in one launch.  ctas: boxes (numbered by cta_begin_asm); prim_ctas:
 // 128-cell ranges (by cta_begin).
@@ -658,9 +680,7 @@ int launch_small(const SmallTableN<NB>& small_tab, int ctas, int prim_ctas, size
       pdl_launch(k_split_prims<T, kWarps32, TB>, prim_ctas, 32 * kWarps32, 0, st, tab, ph.gm1, ph.R, 1.0 / ph.R,
                  K_AOS ? ph.p_ref : 0.0);
   }
-  auto kern = small::k_small_stage<T, K_AOS, NB>;
-  if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  pdl_launch(kern, ctas, 32 * small::kWarpsOf<T>, smem, st, small_tab, flags, stage, next_prims ? 1 : 0, ph.gm1, ph.R,
+  pdl_launch(small::k_small_stage<T, K_AOS, NB>, ctas, 32 * small::kWarpsOf<T>, smem, st, small_tab, flags, stage, next_prims ? 1 : 0, ph.gm1, ph.R,
              1.0 / ph.R, ph);
   if (after_fluxes) cudaEventRecord(after_fluxes, st);
   return prims_ready ? 1 : 2;
@@ -670,9 +690,7 @@ template <typename T>
 int launch_split(fj_ctx* ctx, const SplitBlock* blocks, int nblocks, const Phys& ph, int flags,
                  int stage, bool prims_ready, bool next_prims, int variant, cudaStream_t st,
                  cudaEvent_t after_fluxes) {
-  static int sms = 0;  // SMs of the device (B200: 148)
-  if (sms == 0 && (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device) != cudaSuccess || sms <= 0))
-    sms = 148;
+  const int sms = ctx->sms;
   for (int base = 0; base < nblocks; base += kMaxSplitBlocks) {
     Table tab;
     tab.n = std::min(kMaxSplitBlocks, nblocks - base);
@@ -715,10 +733,11 @@ int launch_split(fj_ctx* ctx, const SplitBlock* blocks, int nblocks, const Phys&
       return set_err(ctx, FJ_ERR_INVALID_ARGUMENT, "the FP64 split path reads kxyz directly");
     // the event marks the first chunk's flux launch
     cudaEvent_t ev = base == 0 ? after_fluxes : nullptr;
-    auto launch = [&](auto nb, auto aos) {
+    auto launch = [&](auto nb, auto aos) {  // kernels launched, or -1 (the error is set)
       constexpr int NB = decltype(nb)::value;
       constexpr bool AOS = decltype(aos)::value;
       if (small_tab) {
+        if (small_ready<T, AOS, NB>(ctx) != FJ_OK) return -1;
         SmallTableN<NB> t;
         t.n = tab.n;
         std::copy(tab.b, tab.b + tab.n, t.b);
@@ -740,9 +759,11 @@ int launch_split(fj_ctx* ctx, const SplitBlock* blocks, int nblocks, const Phys&
       }
       return launch(nb, std::false_type());
     };
-    ctx->launches += tab.n == 1             ? pick(std::integral_constant<int, 1>())
-                     : tab.n <= kFewBlocks  ? pick(std::integral_constant<int, kFewBlocks>())
-                                            : pick(std::integral_constant<int, kMaxSplitBlocks>());
+    const int launched = tab.n == 1             ? pick(std::integral_constant<int, 1>())
+                         : tab.n <= kFewBlocks  ? pick(std::integral_constant<int, kFewBlocks>())
+                                                : pick(std::integral_constant<int, kMaxSplitBlocks>());
+    if (launched < 0) return FJ_ERR_CUDA;
+    ctx->launches += launched;
     int s = launch_status(ctx, "split stage launch");
     if (s != FJ_OK) return s;
   }

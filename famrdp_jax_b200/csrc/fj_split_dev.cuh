@@ -545,8 +545,11 @@ __device__ __forceinline__ void assemble_cell(const SplitBlock& B, const SP& sp,
   if (flags & kRhsViscous) {
     T acc[4];
     assemble_visc<T>(x, src, kk, acc);
+    // an addition of its own in every kernel: fused with a product where a kernel's
+    // branches allow it, a block of a small table would differ from the same block
+    // of a large one in the last bit
 #pragma unroll
-    for (int e = 0; e < 4; ++e) r[e + 1] += (double)acc[e];
+    for (int e = 0; e < 4; ++e) r[e + 1] = __dadd_rn(r[e + 1], (double)acc[e]);
   }
   assemble_out<T>(B, sp, x, stage, next_prims, gm1, R, iR, ph_p_ref, r);
 }

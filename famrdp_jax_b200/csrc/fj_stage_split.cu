@@ -145,10 +145,8 @@ __device__ __forceinline__ void metric_row(const SplitBlock& B, int32_t N, int r
 }
 
 // FL: the one kind of term that the kernel is compiled for, or 0: `flags_` at run
-// time.  (A step's kernels test the flags as the small tables' kernel does: without
-// the branches the compiler fuses a multiplication of the viscous terms into their
-// addition to the inviscid ones, and a block of a small table would differ from the
-// same block of a large one in the last bit.  On 4.0 M cells the time is the same.)
+// time (a step's kernels; compiled for both terms they take the same time on 4.0 M
+// cells).
 template <typename T, int OCC, int NT, class TB, int FL>
 __global__ void __launch_bounds__(NT, OCC) k_fm_fluxes(const TB tab, const Phys ph, const int flags_) {
   const int flags = FL ? FL : flags_;
@@ -412,7 +410,7 @@ __device__ __forceinline__ void assemble_cell(const SplitBlock& B, const Cell& x
     T acc[4];
     assemble_visc<T>(B, x, src, acc);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) r[e + 1] += acc[e];
+    for (int e = 0; e < 4; ++e) r[e + 1] = __dadd_rn(r[e + 1], acc[e]);  // (as in sd::assemble_cell)
   }
   sd::assemble_out<T>(B, TablePtrs{B}, x, stage, next_prims, gm1, R, iR, 0.0, r);
 }

@@ -133,7 +133,9 @@ class StepPlan:
         NUM_SPLIT_VARIANTS * (streams - 1), 2 * NUM_SPLIT_VARIANTS for the
         tile kernel, 2 * NUM_SPLIT_VARIANTS + 1 + k for the persistent step
         in shape k, or 2 * NUM_SPLIT_VARIANTS + 1 + NUM_PERSIST_SHAPES for the
-        split kernels behind the fused ghost fill ("split_fill")."""
+        split kernels behind the fused ghost fill ("split_fill").  (Tables
+        small enough for one launch a stage have one launch shape: their split
+        candidates differ by noise.)"""
         n = _capi.AUTOTUNE_CANDIDATES
         ms = (ctypes.c_double * n)()
         ch = ctypes.c_int()

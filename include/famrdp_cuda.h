@@ -391,7 +391,8 @@ int fj_plan_set_streams(fj_plan* plan, int n);
  * more candidates) (and,
  * if ms_out is non-NULL, the FJ_AUTOTUNE_CANDIDATES mean step times at those
  * indices; 0 where not timed).  q_out is overwritten; q_in is not changed.
- * Synchronises the stream. */
+ * Tables small enough for one launch a stage have one launch shape: their
+ * split shapes are timed alike and differ by noise.  Synchronises the stream. */
 #define FJ_AUTOTUNE_CANDIDATES (2 * FJ_NUM_SPLIT_VARIANTS + 2 + FJ_NUM_PERSIST_SHAPES)
 int fj_plan_autotune(fj_plan* plan, double* const* q_in, double* const* q_out, double dt, int reps,
                      int* chosen, double* ms_out, void* stream);

@@ -53,3 +53,19 @@ def test_same_bits(cuda_device, shapes, limiter, law, precision):
     for a, b in zip(alone, among):
         assert torch.isfinite(a).all()
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("precision", ["f64", "f32"])
+def test_launch_shapes_of_large_tables(cuda_device, precision):
+    """Every launch shape at one and two streams on a table too large for one launch a
+    stage (small ones have one shape): the same bits."""
+    blocks = [tuple(dev(x) for x in random_block(s, 95 + n)) for n, s in enumerate([(40, 37, 45), (52, 48, 40)])]
+    plan, qs = _plan(blocks, "minmod", precision, "sutherland"), [b[0] for b in blocks]
+    ref, n = _step(plan, qs)
+    assert n == 1 + 3 * 2
+    for streams in (1, 2):
+        plan.set_streams(streams)
+        for v in range(_capi.NUM_SPLIT_VARIANTS):
+            plan.set_variant(v)
+            for a, b in zip(_step(plan, qs)[0], ref):
+                assert torch.equal(a, b)

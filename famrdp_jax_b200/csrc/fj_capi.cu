@@ -739,11 +739,9 @@ int fj_plan_create(fj_ctx* ctx, const fj_block* blocks, int nblocks, const fj_li
     int* flags = (int*)pl->scratch;  // no step has used it yet
     e = total >= nblocks * sizeof(int) ? cudaMemsetAsync(flags, 0, nblocks * sizeof(int), pl->capture_stream)
                                        : cudaErrorMemoryAllocation;
-    for (int b = 0; b < nblocks && e == cudaSuccess; ++b)
-      if (split_metrics_differ(pl->kmet.empty() ? nullptr : pl->kmet[b], blocks[b].kxyz,
-                               (int64_t)blocks[b].ni * blocks[b].nj * blocks[b].nk, flags + b,
-                               pl->capture_stream) != FJ_OK)
-        e = cudaErrorUnknown;
+    if (e == cudaSuccess && split_metrics_differ(pl->kmet.empty() ? nullptr : pl->kmet.data(), blocks, nblocks, flags,
+                                                 pl->capture_stream) != FJ_OK)
+      e = cudaErrorUnknown;
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(differ.data(), flags, nblocks * sizeof(int), cudaMemcpyDeviceToHost, pl->capture_stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(pl->capture_stream);

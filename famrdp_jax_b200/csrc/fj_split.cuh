@@ -46,9 +46,9 @@ struct SplitBlock {
 // field-major FP64 kxyz (3, 3, ni, nj, nk): the nine kxyz[l][m] and, in FP32
 // records, the three face-normal difference sums the pressure offset uses.
 int split_metric_records(const double* kxyz, void* out, int ni, int nj, int nk, int precision, cudaStream_t st);
-// *flag (device, cleared by the caller) := 1 where a block's FP32 records, or its
-// FP64 kxyz, are not the same bits in every cell.
-int split_metrics_differ(const void* records, const double* kxyz, int64_t N, int* flag, cudaStream_t st);
+// flags[b] (device, cleared by the caller) := 1 where block b's FP32 records, or
+// (records null) its FP64 kxyz, are not the same bits in every cell.
+int split_metrics_differ(const void* const* records, const fj_block* blocks, int nblocks, int* flags, cudaStream_t st);
 // Mean pressure over all padded cells of the blocks, on stream st with
 // mean_pressure_scratch_bytes(nblocks) bytes of device scratch; waits for st.
 size_t mean_pressure_scratch_bytes(int nblocks);

@@ -490,19 +490,38 @@ __global__ void k_metric_records(const double* __restrict__ kxyz, T* __restrict_
   st_rec<T, kRecK<T>>(out + c * kRecK<T>, rec);
 }
 
-// *flag := 1 where a word differs from word % period of the array (bits): n words
-// from m + blockIdx.y * n on, the grid's threads a multiple of `period`, so that
-// a thread compares with one word.  A block that is not uniform shows it in its
-// first cells, and the threads stop.
-__global__ void __launch_bounds__(192) k_words_differ(const unsigned long long* __restrict__ m, int64_t n, int period,
-                                                      int* flag) {
-  m += blockIdx.y * n;
-  const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+// flags[b] := 1 where a word of a field of block b differs from word % period of it
+// (bits): n[b] words a field, fields blockIdx.y, strides a multiple of `period`, so
+// that a thread compares with one word.  CTAs of a block whose flag is set have
+// nothing to do.  A block that is not uniform mostly shows it anywhere: a first launch
+// (`sample`) of one CTA a field looks at 32 places spread over the block, and the
+// second, at all words, then ends at once.  (In one launch the CTAs of the first wave
+// all store the flag, 4 ns each: 0.15 ms for the four 128^3 blocks of a wavy grid
+// instead of 0.02; polling the flag as they go takes longer still.)
+struct WordsTable {
+  const unsigned long long* m[kMaxSplitBlocks];
+  int64_t n[kMaxSplitBlocks];
+};
+constexpr int kWordThreads = 192;
+__global__ void __launch_bounds__(kWordThreads) k_words_differ(const WordsTable tab, int sample, int period,
+                                                               int* flags) {
+  const int64_t n = tab.n[blockIdx.z];
+  const unsigned long long* m = tab.m[blockIdx.z] + blockIdx.y * n;
+  int* flag = flags + blockIdx.z;
+  if (__syncthreads_or(threadIdx.x == 0 && *(volatile int*)flag)) return;
+  const int lane = threadIdx.x & 31;
+  const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int64_t step = sample ? max((int64_t)1, n / (32 * kWordThreads)) * kWordThreads : (int64_t)gridDim.x * blockDim.x;
   const unsigned long long ref = m[t0 % period];
-  for (int64_t t = t0; t < n; t += step) {
-    if (m[t] == ref) continue;
-    *flag = 1;
-    return;
+  constexpr int kU = 4;  // words in flight
+  for (int64_t t = t0; t - lane < n; t += kU * step) {
+    bool differ = false;
+#pragma unroll
+    for (int u = 0; u < kU; ++u) differ |= t + u * step < n && m[t + u * step] != ref;
+    if (__any_sync(0xffffffffu, differ)) {
+      if (lane == 0) *flag = 1;
+      return;
+    }
   }
 }
 
@@ -781,16 +800,25 @@ int split_metric_records(const double* kxyz, void* out, int ni, int nj, int nk, 
   return cudaGetLastError() == cudaSuccess ? FJ_OK : FJ_ERR_CUDA;
 }
 
-int split_metrics_differ(const void* records, const double* kxyz, int64_t N, int* flag, cudaStream_t st) {
-  if (N <= 0) return FJ_OK;
-  constexpr int nt = 192, per = kRecK<float> / 2;  // 8-byte words of an FP32 record
+int split_metrics_differ(const void* const* records, const fj_block* blocks, int nblocks, int* flags, cudaStream_t st) {
+  constexpr int nt = kWordThreads, per = kRecK<float> / 2;  // 8-byte words of an FP32 record
   static_assert(nt % per == 0, "a thread's words all have the same place in their record");
-  if (records)
-    k_words_differ<<<(unsigned)std::min<int64_t>((N * per + nt - 1) / nt, 148 * 10), nt, 0, st>>>(
-        (const unsigned long long*)records, N * per, per, flag);
-  else
-    k_words_differ<<<dim3((unsigned)std::min<int64_t>((N + nt - 1) / nt, 148 * 2), 9), nt, 0, st>>>(
-        (const unsigned long long*)kxyz, N, 1, flag);
+  for (int base = 0; base < nblocks; base += kMaxSplitBlocks) {
+    WordsTable tab;
+    const int nb = std::min(kMaxSplitBlocks, nblocks - base);
+    int64_t most = 0;
+    for (int b = 0; b < nb; ++b) {
+      const fj_block& B = blocks[base + b];
+      const int64_t N = (int64_t)B.ni * B.nj * B.nk;
+      tab.m[b] = (const unsigned long long*)(records ? records[base + b] : B.kxyz);
+      tab.n[b] = records ? N * per : N;
+      most = std::max(most, tab.n[b]);
+    }
+    const unsigned ctas = (unsigned)std::min<int64_t>((most + nt - 1) / nt, records ? 148 * 10 : 148 * 2);
+    const unsigned fields = records ? 1 : 9, step = records ? per : 1;
+    k_words_differ<<<dim3(1, fields, nb), nt, 0, st>>>(tab, 1, step, flags + base);
+    k_words_differ<<<dim3(ctas, fields, nb), nt, 0, st>>>(tab, 0, step, flags + base);
+  }
   return cudaGetLastError() == cudaSuccess ? FJ_OK : FJ_ERR_CUDA;
 }
 

@@ -59,11 +59,12 @@ __device__ __forceinline__ void muscl2_vjp(T c0, T c1, T c2, T c3, T lamL, T lam
   }
 }
 
-// Reverse of roe_prim: lamF (5) -> lamL, lamR (primitive face states, set).
+// Reverse of roe_prim (FP32): lamF (5) -> lamL, lamR (primitive face states, set).
 template <typename T>
 __device__ __forceinline__ void roe_prim_vjp(const Prim<T>& L, const Prim<T>& R, T n0, T n1, T n2,
                                              T gm1, T ig, T eps_e, const T g[5], Prim<T>& lL,
                                              Prim<T>& lR) {
+  static_assert(sizeof(T) == 4, "FP64 faces: roe_face_f64_vjp");
   using M = FastMath<T>;
   // ---- forward recomputation (same statements as roe_prim) ----
   const bool clL = L.rho > Tiny<T>::rho(), clR = R.rho > Tiny<T>::rho();

@@ -22,9 +22,11 @@
 // first / second target tangential axis runs backwards on the source.  Each
 // link is reduced on the host to an affine map from the target slab's
 // coordinates to a source cell index (base + signed stride per axis).
-// Boundary conditions run after the halo, one launch per face in Face enum
-// order (physics/bc/dispatch.py:15), each launch covering that face of every
-// block (blocks are independent).
+// Boundary conditions run after the halo, in Face enum order
+// (physics/bc/dispatch.py:15): one launch per face, each covering that face of
+// every block (blocks are independent).  A step that is not in place copies its
+// start state, fills its ghost cells and applies its boundary conditions in one
+// kernel (k_copy_fill).
 #include <algorithm>
 #include <cstring>
 #include <vector>

@@ -222,9 +222,6 @@ template <> struct FastMath<double> {
   // __drcp_rn: the IEEE round-to-nearest reciprocal, the same value as 1.0 / x
   static __device__ __forceinline__ double rcp(double x) { return __drcp_rn(x); }
   static __device__ __forceinline__ double sqrt_pos(double x) { return sqrt(x); }
-  static __device__ __forceinline__ double sqrt_nn(double x) { return sqrt(x); }
-  static __device__ __forceinline__ double rcp_n(double x) { return rcp(x); }
-  static __device__ __forceinline__ double sqrt_n(double x) { return sqrt(x); }
 };
 template <> struct FastMath<float> {
   static __device__ __forceinline__ float rcp(float x) { return __fdividef(1.0f, x); }
@@ -316,8 +313,8 @@ __device__ __forceinline__ void muscl2_fast(const Prim<T> c[4], int limiter, Pri
 #undef FJ_MUSCL
 }
 
-// Roe flux (flux/roe.py:21-85) of the primitive face states L, R along the unit
-// normal n; inv_gm1 = 1/(gamma-1).
+// Roe flux (flux/roe.py:21-85) in FP32 of the primitive face states L, R along the
+// unit normal n; inv_gm1 = 1/(gamma-1).  (FP64: roe_face_f64.)
 //
 // POFF (the FP32-flux split path): the states carry the pressure OFFSET
 // p' = p - p_ref instead of p.  The energies and enthalpies add p_ref back as
@@ -330,6 +327,7 @@ __device__ __forceinline__ void muscl2_fast(const Prim<T> c[4], int limiter, Pri
 template <typename T, bool POFF = false>
 __device__ __forceinline__ void roe_prim(const Prim<T>& L, const Prim<T>& R, T n0, T n1, T n2,
                                          T gm1, T inv_gm1, T eps_entropy, T F[5], T p_ref = T(0)) {
+  static_assert(sizeof(T) == 4, "FP64 faces: roe_face_f64");
   using M = FastMath<T>;
   // arguments of rcp_n / sqrt_n are clamped above the subnormal range (eps is
   // used only where it exceeds an eigenvalue)
@@ -344,58 +342,25 @@ __device__ __forceinline__ void roe_prim(const Prim<T>& L, const Prim<T>& R, T n
   const T irL = M::rcp_n(rhoL), irR = M::rcp_n(rhoR);
   const T HL = (POFF ? (eL + L.p) + Hc : EL + L.p) * irL;
   const T HR = (POFF ? (eR + R.p) + Hc : ER + R.p) * irR;
-  // Roe weights sqL / (sqL + sqR), sqR / (sqL + sqR) and rho_h = sqL sqR.  In
-  // FP64 from one square root, t = sqrt(rhoR / rhoL): wl = 1 / (1 + t),
-  // wr = t / (1 + t), rho_h = rhoL t (the same values; the reference's clamp
-  // of sqL + sqR at 1e-150 cannot bind once rho >= 1e-300).  FP32 keeps the
-  // two MUFU square roots.
-  T wl, wr, rho_h;
-  if constexpr (sizeof(T) == 8) {
-    const T t = sqrt(rhoR * irL);
-    wl = M::rcp_n(T(1) + t);
-    wr = t * wl;
-    rho_h = rhoL * t;
-  } else {
-    const T sqL = M::sqrt_n(rhoL), sqR = M::sqrt_n(rhoR);
-    const T inv_ss = M::rcp_n(fj_max(sqL + sqR, Tiny<T>::ss()));
-    wl = sqL * inv_ss;
-    wr = sqR * inv_ss;
-    rho_h = sqL * sqR;
-  }
+  // Roe weights sqL / (sqL + sqR), sqR / (sqL + sqR) and rho_h = sqL sqR
+  const T sqL = M::sqrt_n(rhoL), sqR = M::sqrt_n(rhoR);
+  const T inv_ss = M::rcp_n(fj_max(sqL + sqR, Tiny<T>::ss()));
+  const T wl = sqL * inv_ss, wr = sqR * inv_ss, rho_h = sqL * sqR;
   const T u_h = wl * L.u + wr * R.u;
   const T v_h = wl * L.v + wr * R.v;
   const T w_h = wl * L.w + wr * R.w;
   const T H_h = wl * HL + wr * HR;
   const T q2 = u_h * u_h + v_h * v_h + w_h * w_h;
   const T c2 = fj_max(gm1 * (H_h - T(0.5) * q2), Tiny<T>::c2());
-  T c_h, inv_c2;
-  if constexpr (sizeof(T) == 8) {
-    // one reciprocal square root for c and 1/c^2 (c2 >= 1e-30 > 0)
-    const T ic = rsqrt(c2);
-    c_h = c2 * ic;
-    inv_c2 = ic * ic;
-  } else {
-    c_h = M::sqrt_n(c2);
-    inv_c2 = M::rcp_n(c2);
-  }
+  const T c_h = M::sqrt_n(c2), inv_c2 = M::rcp_n(c2);
   const T un_h = u_h * n0 + v_h * n1 + w_h * n2;
 
   const T eps = eps_entropy * (fj_abs(un_h) + c_h);
   const T lam1 = un_h - c_h, lam5 = un_h + c_h;
   T al1 = fj_abs(lam1), al5 = fj_abs(lam5);
-  if constexpr (sizeof(T) == 8) {
-    // Harten's fix (flux/roe.py:45-52) only where |lambda| < eps: the FP64
-    // reciprocal of eps is taken only then
-    if (al1 < eps || al5 < eps) {
-      const T inv_eps = M::rcp_n(eps);
-      if (al1 < eps) al1 = T(0.5) * (lam1 * lam1 * inv_eps + eps);
-      if (al5 < eps) al5 = T(0.5) * (lam5 * lam5 * inv_eps + eps);
-    }
-  } else {
-    const T inv_eps = M::rcp_n(eps);
-    al1 = al1 >= eps ? al1 : T(0.5) * (lam1 * lam1 * inv_eps + eps);
-    al5 = al5 >= eps ? al5 : T(0.5) * (lam5 * lam5 * inv_eps + eps);
-  }
+  const T inv_eps = M::rcp_n(eps);  // Harten's fix (flux/roe.py:45-52)
+  al1 = al1 >= eps ? al1 : T(0.5) * (lam1 * lam1 * inv_eps + eps);
+  al5 = al5 >= eps ? al5 : T(0.5) * (lam5 * lam5 * inv_eps + eps);
   const T al2 = fj_abs(un_h);
 
   const T d0 = R.rho - L.rho;
@@ -557,16 +522,16 @@ __device__ __forceinline__ void invscd_face_fast(const Prim<T> c[4], T kl0, T kl
                                                  int limiter, T F[5], T p_ref = T(0)) {
   Prim<T> L, R;
   muscl2_fast(c, limiter, L, R);
-  if constexpr (sizeof(T) == 8 && !POFF) {
+  if constexpr (sizeof(T) == 8) {
     roe_face_f64(L, R, 0.5 * (kl0 + kr0), 0.5 * (kl1 + kr1), 0.5 * (kl2 + kr2), gm1, inv_gm1, eps_entropy, F);
-    return;
-  }
-  const T nf0 = T(0.5) * (kl0 + kr0), nf1 = T(0.5) * (kl1 + kr1), nf2 = T(0.5) * (kl2 + kr2);
-  const T nmag = FastMath<T>::sqrt_nn(nf0 * nf0 + nf1 * nf1 + nf2 * nf2) + Tiny<T>::nmag();
-  const T inv = FastMath<T>::rcp_n(nmag);
-  roe_prim<T, POFF>(L, R, nf0 * inv, nf1 * inv, nf2 * inv, gm1, inv_gm1, eps_entropy, F, p_ref);
+  } else {
+    const T nf0 = T(0.5) * (kl0 + kr0), nf1 = T(0.5) * (kl1 + kr1), nf2 = T(0.5) * (kl2 + kr2);
+    const T nmag = FastMath<T>::sqrt_nn(nf0 * nf0 + nf1 * nf1 + nf2 * nf2) + Tiny<T>::nmag();
+    const T inv = FastMath<T>::rcp_n(nmag);
+    roe_prim<T, POFF>(L, R, nf0 * inv, nf1 * inv, nf2 * inv, gm1, inv_gm1, eps_entropy, F, p_ref);
 #pragma unroll
-  for (int v = 0; v < 5; ++v) F[v] = F[v] * nmag;
+    for (int v = 0; v < 5; ++v) F[v] = F[v] * nmag;
+  }
 }
 
 // physics/eos.py:24-25 (or the constant law)

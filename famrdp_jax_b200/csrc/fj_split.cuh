@@ -1,4 +1,5 @@
-// fj_split.cuh -- the three-kernel stage pipeline over a table of blocks
+// fj_split.cuh -- the split stage pipeline (primitives, fluxes, assembly; one kernel
+// for all three where the table is small) over a table of blocks
 // (fj_stage_split.cu).
 #pragma once
 
@@ -39,7 +40,7 @@ struct SplitBlock {
   double dt;             // time step of this block (stages 1..3)
   int ni, nj, nk;
   int cta_begin;         // filled by the launcher
-  int cta_begin_asm;     // the same for the FP32 assembly's 248-cell CTAs
+  int cta_begin_asm;     // the same for the assembly's CTAs, or the small kernel's boxes
 };
 
 // Metric records (kRecK values of the flux type per cell) from the caller's
@@ -60,7 +61,8 @@ size_t split_scratch_bytes(int precision, int64_t cells);
 // Points prim/F/G of every block into one scratch region of
 // split_scratch_bytes(precision, sum of the blocks' cells) bytes.
 void split_assign_scratch(int precision, SplitBlock* blocks, int nblocks, void* scratch);
-// One RHS (stage 0) or TVD-RK3 stage (1..3) of all blocks: three launches
+// One RHS (stage 0) or TVD-RK3 stage (1..3) of all blocks: the primitives, the
+// fluxes and the assembly, or the primitives and one launch for both in small tables
 // (per chunk of kMaxSplitBlocks blocks).  ph supplies everything but mu0,
 // which comes per block like dt.
 // prims_ready: the blocks' primitives were already written (by the previous

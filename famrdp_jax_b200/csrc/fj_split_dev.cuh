@@ -379,8 +379,6 @@ __device__ __forceinline__ void face_from_cells(const Cell6<T>& a0, const Cell6<
                             num<T>(ph).eps_entropy, ph.limiter, F, p_ref);
 }
 
-// With next_prims, also writes the primitives of the stage result (the next
-// stage's input) in place of a separate k_split_prims launch.
 // Where the assembly reads the intermediates of a cell from: the scratch
 // arrays through L1/L2 (the interface lets another source, e.g. a
 // shared-memory copy, feed the same arithmetic).
@@ -429,6 +427,7 @@ struct GlobalSrc {
 template <typename T, bool K_AOS, class Src>
 __device__ __forceinline__ void assemble_inv(const SplitBlock& B, const Cell& x, const Src& src, double ph_p_ref,
                                              const T fk_m[5], const T fk_p[5], const T gcl[3], double r[5]) {
+  static_assert(sizeof(T) == 4, "the FP32 path (FP64: fm::assemble_inv)");
   const int32_t c = (int32_t)x.c;
   const int n[3] = {x.ni, x.nj, x.nk};
   const int idx[3] = {x.i, x.j, x.k};
@@ -460,20 +459,12 @@ __device__ __forceinline__ void assemble_inv(const SplitBlock& B, const Cell& x,
     }
 #pragma unroll
     for (int v = 0; v < 5; ++v) {
-      double dsum;
-      if (sizeof(T) == sizeof(double)) {
-        dsum = 0.0;  // axis by axis like the reference
+      T s = T(0);
 #pragma unroll
-        for (int a = 0; a < 3; ++a)
-          if (on[a]) dsum += (double)(Fc[5 * a + v] - Fm[a][v]);
-      } else {
-        T s = T(0);
-#pragma unroll
-        for (int a = 0; a < 3; ++a)
-          if (on[a]) s += Fc[5 * a + v] - Fm[a][v];
-        dsum = (double)s;
-        if (K_AOS && v >= 1 && v <= 3) dsum += pg[v - 1];
-      }
+      for (int a = 0; a < 3; ++a)
+        if (on[a]) s += Fc[5 * a + v] - Fm[a][v];
+      double dsum = (double)s;
+      if (K_AOS && v >= 1 && v <= 3) dsum += pg[v - 1];
       r[v] = -dsum * ivd;
     }
   }
@@ -554,8 +545,6 @@ __device__ __forceinline__ void assemble_cell(const SplitBlock& B, const SP& sp,
   assemble_out<T>(B, sp, x, stage, next_prims, gm1, R, iR, ph_p_ref, r);
 }
 
-// With next_prims, also writes the primitives of the stage result (the next
-// stage's input) in place of a separate k_split_prims launch.
 // The k face c-1 | c (rhs/invscd.py:62-100) from the stage input's primitive
 // records of c-2 .. c+1, the k row of the metrics of c-1 and kr, that of c.
 template <typename T, bool K_AOS, bool NC = true>
@@ -568,10 +557,6 @@ __device__ __forceinline__ void k_face_left(const SplitBlock& B, const void* pri
   metric_row<T, K_AOS>(B, N, 2, c - 1, kl);
   face_from_cells<T, K_AOS>(a0, a1, a2, a3, kl, kr, ph, F, K_AOS ? num<T>(ph).p_ref : T(0));
 }
-
-// Cells per assembly CTA: each warp assembles 31 consecutive cells; its 32nd
-// lane only evaluates the k face its 31st cell needs on the right.
-constexpr int kAsmCells = kSplitThreads / 32 * 31;
 
 // The last b with cta_begin_asm <= cta (the assembly's CTA ranges).
 template <int NB>
@@ -599,6 +584,48 @@ __device__ __forceinline__ void prims_cell(const SplitBlock& B, int32_t c, doubl
   store_prim_record<T>(B.prim, (size_t)c, qc, gm1, R, iR, p_ref);
 }
 
+// The viscous flux components G(c) (rhs/viscous.py:36-105) from the primitives of c
+// and its six neighbours and the metrics of c.
+template <typename T>
+__device__ __forceinline__ void visc_components(const SplitBlock& B, const Cell6<T>& C0, const Cell6<T>& Im,
+                                                const Cell6<T>& Ip, const Cell6<T>& Jm, const Cell6<T>& Jp,
+                                                const Cell6<T>& Km, const Cell6<T>& Kp, const T kk[9], const Phys& ph,
+                                                T G[9]) {
+  const T h = T(0.5);
+  const T d[4][3] = {{h * (Ip.u - Im.u), h * (Jp.u - Jm.u), h * (Kp.u - Km.u)},
+                     {h * (Ip.v - Im.v), h * (Jp.v - Jm.v), h * (Kp.v - Km.v)},
+                     {h * (Ip.w - Im.w), h * (Jp.w - Jm.w), h * (Kp.w - Km.w)},
+                     {h * (Ip.t - Im.t), h * (Jp.t - Jm.t), h * (Kp.t - Km.t)}};
+  T g[4][3];
+#pragma unroll
+  for (int s = 0; s < 4; ++s)
+#pragma unroll
+    for (int m = 0; m < 3; ++m) g[s][m] = d[s][0] * kk[m] + d[s][1] * kk[3 + m] + d[s][2] * kk[6 + m];
+  T mu = block_mu0<T>(B);
+  if (ph.visc_law == 0) {  // Sutherland (physics/eos.py:24-25)
+    const T r = C0.t * num<T>(ph).inv_T0;
+    mu = block_mu0<T>(B) * (r * FastMath<T>::sqrt_pos(r)) * num<T>(ph).sfac * FastMath<T>::rcp(C0.t + num<T>(ph).Ts);
+  }
+  const T kappa = num<T>(ph).kap_fac * mu;
+  const T third = (T)(1.0 / 3.0);
+  const T div_u = g[0][0] + g[1][1] + g[2][2];
+  const T t00 = T(2) * mu * (g[0][0] - div_u * third);
+  const T t01 = mu * (g[0][1] + g[1][0]);
+  const T t02 = mu * (g[0][2] + g[2][0]);
+  const T t11 = T(2) * mu * (g[1][1] - div_u * third);
+  const T t12 = mu * (g[1][2] + g[2][1]);
+  const T t22 = T(2) * mu * (g[2][2] - div_u * third);
+  G[0] = t00;
+  G[1] = t01;
+  G[2] = t02;
+  G[3] = t11;
+  G[4] = t12;
+  G[5] = t22;
+  G[6] = C0.u * t00 + C0.v * t01 + C0.w * t02 + kappa * g[3][0];
+  G[7] = C0.u * t01 + C0.v * t11 + C0.w * t12 + kappa * g[3][1];
+  G[8] = C0.u * t02 + C0.v * t12 + C0.w * t22 + kappa * g[3][2];
+}
+
 // Flux work of cell x of B (k_split_fluxes): the viscous flux components G(c)
 // (rhs/viscous.py:36-105, neighbours wrap around the padded block like
 // jnp.roll) and the Roe faces c | c+e_i and c | c+e_j (rhs/invscd.py:53-100)
@@ -606,7 +633,6 @@ __device__ __forceinline__ void prims_cell(const SplitBlock& B, int32_t c, doubl
 template <typename T, bool K_AOS, bool NC>
 __device__ __forceinline__ void flux_cell(const SplitBlock& B, const void* prim, const Cell& x, const Phys& ph,
                                           int flags) {
-  using M = FastMath<T>;
   // 32-bit cell indices: kRecF N < 2^31 is checked on the host
   const int32_t N = (int32_t)x.N, c = (int32_t)x.c;
   const int32_t si = x.nj * x.nk, sj = x.nk;
@@ -630,36 +656,10 @@ __device__ __forceinline__ void flux_cell(const SplitBlock& B, const void* prim,
   metric9<T, K_AOS>(B, N, c, kk);
 
   if (vis) {
-    // viscous flux components at c (rhs/viscous.py:36-105)
-    const T h = T(0.5);
-    const T d[4][3] = {{h * (Ip.u - Im.u), h * (Jp.u - Jm.u), h * (Kp.u - Km.u)},
-                       {h * (Ip.v - Im.v), h * (Jp.v - Jm.v), h * (Kp.v - Km.v)},
-                       {h * (Ip.w - Im.w), h * (Jp.w - Jm.w), h * (Kp.w - Km.w)},
-                       {h * (Ip.t - Im.t), h * (Jp.t - Jm.t), h * (Kp.t - Km.t)}};
-    T g[4][3];
-#pragma unroll
-    for (int s = 0; s < 4; ++s)
-#pragma unroll
-      for (int m = 0; m < 3; ++m) g[s][m] = d[s][0] * kk[m] + d[s][1] * kk[3 + m] + d[s][2] * kk[6 + m];
-    T mu = block_mu0<T>(B);
-    if (ph.visc_law == 0) {  // Sutherland (physics/eos.py:24-25)
-      const T r = C0.t * num<T>(ph).inv_T0;
-      mu = block_mu0<T>(B) * (r * M::sqrt_pos(r)) * num<T>(ph).sfac * M::rcp(C0.t + num<T>(ph).Ts);
-    }
-    const T kappa = num<T>(ph).kap_fac * mu;
-    const T third = (T)(1.0 / 3.0);
-    const T div_u = g[0][0] + g[1][1] + g[2][2];
-    const T t00 = T(2) * mu * (g[0][0] - div_u * third);
-    const T t01 = mu * (g[0][1] + g[1][0]);
-    const T t02 = mu * (g[0][2] + g[2][0]);
-    const T t11 = T(2) * mu * (g[1][1] - div_u * third);
-    const T t12 = mu * (g[1][2] + g[2][1]);
-    const T t22 = T(2) * mu * (g[2][2] - div_u * third);
-    const T rec[kRecG] = {t00, t01, t02, t11, t12, t22,
-                          C0.u * t00 + C0.v * t01 + C0.w * t02 + kappa * g[3][0],
-                          C0.u * t01 + C0.v * t11 + C0.w * t12 + kappa * g[3][1]};
-    st_rec<T, kRecG>((T*)B.G + (size_t)c * kRecG, rec);
-    ((T*)B.Gz)[c] = C0.u * t02 + C0.v * t12 + C0.w * t22 + kappa * g[3][2];
+    T g[9];
+    visc_components(B, C0, Im, Ip, Jm, Jp, Km, Kp, kk, ph, g);
+    st_rec<T, kRecG>((T*)B.G + (size_t)c * kRecG, g);
+    ((T*)B.Gz)[c] = g[8];
   }
   if (inv) {
     // the faces c | c+e_i and c | c+e_j for c_a in [1, n_a - 3]; invalid faces
@@ -695,7 +695,6 @@ template <typename T, bool K_AOS>
 __device__ __forceinline__ void visc_value(const SplitBlock& B, const void* prim, const Cell& x, const Phys& ph,
                                            T G[9]) {
   static_assert(sizeof(T) == 4, "the FP32 records path");
-  using M = FastMath<T>;
   const int32_t N = (int32_t)x.N, c = (int32_t)x.c;
   const int32_t si = x.nj * x.nk, sj = x.nk;
   const T* __restrict__ P = (const T*)prim;
@@ -711,39 +710,7 @@ __device__ __forceinline__ void visc_value(const SplitBlock& B, const void* prim
   const Cell6<T> Km = load_cell<T, true>(P, km), Kp = load_cell<T, true>(P, kp);
   T kk[9];
   metric9<T, K_AOS>(B, N, c, kk);
-  const T h = T(0.5);
-  const T d[4][3] = {{h * (Ip.u - Im.u), h * (Jp.u - Jm.u), h * (Kp.u - Km.u)},
-                     {h * (Ip.v - Im.v), h * (Jp.v - Jm.v), h * (Kp.v - Km.v)},
-                     {h * (Ip.w - Im.w), h * (Jp.w - Jm.w), h * (Kp.w - Km.w)},
-                     {h * (Ip.t - Im.t), h * (Jp.t - Jm.t), h * (Kp.t - Km.t)}};
-  T g[4][3];
-#pragma unroll
-  for (int s = 0; s < 4; ++s)
-#pragma unroll
-    for (int m = 0; m < 3; ++m) g[s][m] = d[s][0] * kk[m] + d[s][1] * kk[3 + m] + d[s][2] * kk[6 + m];
-  T mu = block_mu0<T>(B);
-  if (ph.visc_law == 0) {  // Sutherland (physics/eos.py:24-25)
-    const T r = C0.t * num<T>(ph).inv_T0;
-    mu = block_mu0<T>(B) * (r * M::sqrt_pos(r)) * num<T>(ph).sfac * M::rcp(C0.t + num<T>(ph).Ts);
-  }
-  const T kappa = num<T>(ph).kap_fac * mu;
-  const T third = (T)(1.0 / 3.0);
-  const T div_u = g[0][0] + g[1][1] + g[2][2];
-  const T t00 = T(2) * mu * (g[0][0] - div_u * third);
-  const T t01 = mu * (g[0][1] + g[1][0]);
-  const T t02 = mu * (g[0][2] + g[2][0]);
-  const T t11 = T(2) * mu * (g[1][1] - div_u * third);
-  const T t12 = mu * (g[1][2] + g[2][1]);
-  const T t22 = T(2) * mu * (g[2][2] - div_u * third);
-  G[0] = t00;
-  G[1] = t01;
-  G[2] = t02;
-  G[3] = t11;
-  G[4] = t12;
-  G[5] = t22;
-  G[6] = C0.u * t00 + C0.v * t01 + C0.w * t02 + kappa * g[3][0];
-  G[7] = C0.u * t01 + C0.v * t11 + C0.w * t12 + kappa * g[3][1];
-  G[8] = C0.u * t02 + C0.v * t12 + C0.w * t22 + kappa * g[3][2];
+  visc_components(B, C0, Im, Ip, Jm, Jp, Km, Kp, kk, ph, G);
 }
 
 // The Roe face c | c+e_a (stride sa) for c_a = ia in [1, na-3], zeros elsewhere.
@@ -764,8 +731,8 @@ __device__ __forceinline__ void face_value(const SplitBlock& B, const void* prim
   }
 }
 
-// Assembly of the kAsmCells cells from c0 of B (k_split_assemble; all 256
-// threads of the CTA call it).  The k faces are evaluated here: lane l of a
+// Assembly of 31 consecutive cells a warp from c0 of B on (k_split_assemble and the
+// persistent step; every thread of the CTA calls it).  The k faces are evaluated here: lane l of a
 // warp evaluates the face on the left of its cell (c-1 | c) and takes the one
 // on its right from lane l+1 by shuffle, so no face is evaluated twice and no
 // barrier is needed; lane 31's cell is the next warp's first, for which it

@@ -144,13 +144,54 @@ __device__ __forceinline__ void metric_row(const SplitBlock& B, int32_t N, int r
   k[2] = (T)__ldg(K + 2 * N);
 }
 
+// The viscous flux components G(c) (rhs/viscous.py:36-105) from the primitives of c
+// and its six neighbours and the metrics of c.
+template <typename T>
+__device__ __forceinline__ void visc_components(const SplitBlock& B, const Cell6<T>& C0, const Cell6<T>& Im,
+                                                const Cell6<T>& Ip, const Cell6<T>& Jm, const Cell6<T>& Jp,
+                                                const Cell6<T>& Km, const Cell6<T>& Kp, const T kk[9], const Phys& ph,
+                                                T G[9]) {
+  // the central differences' factor 1/2 is carried by mu and kappa (exact)
+  const T d[4][3] = {{Ip.u - Im.u, Jp.u - Jm.u, Kp.u - Km.u},
+                     {Ip.v - Im.v, Jp.v - Jm.v, Kp.v - Km.v},
+                     {Ip.w - Im.w, Jp.w - Jm.w, Kp.w - Km.w},
+                     {Ip.t - Im.t, Jp.t - Jm.t, Kp.t - Km.t}};
+  T g[4][3];
+#pragma unroll
+  for (int s = 0; s < 4; ++s)
+#pragma unroll
+    for (int m = 0; m < 3; ++m) g[s][m] = d[s][0] * kk[m] + d[s][1] * kk[3 + m] + d[s][2] * kk[6 + m];
+  T mu = (T)B.mu0;
+  if (ph.visc_law == 0) {  // Sutherland (physics/eos.py:24-25)
+    const T r = C0.t * (T)ph.inv_T0;
+    mu = (T)B.mu0 * (r * FastMath<T>::sqrt_pos(r)) * (T)ph.sfac * FastMath<T>::rcp(C0.t + (T)ph.Ts);
+  }
+  const T muh = T(0.5) * mu, kappa = (T)ph.kap_fac * muh;
+  const T third = (T)(1.0 / 3.0);
+  const T div_u = g[0][0] + g[1][1] + g[2][2];
+  const T t00 = mu * (g[0][0] - div_u * third);
+  const T t01 = muh * (g[0][1] + g[1][0]);
+  const T t02 = muh * (g[0][2] + g[2][0]);
+  const T t11 = mu * (g[1][1] - div_u * third);
+  const T t12 = muh * (g[1][2] + g[2][1]);
+  const T t22 = mu * (g[2][2] - div_u * third);
+  G[0] = t00;
+  G[1] = t01;
+  G[2] = t02;
+  G[3] = t11;
+  G[4] = t12;
+  G[5] = t22;
+  G[6] = C0.u * t00 + C0.v * t01 + C0.w * t02 + kappa * g[3][0];
+  G[7] = C0.u * t01 + C0.v * t11 + C0.w * t12 + kappa * g[3][1];
+  G[8] = C0.u * t02 + C0.v * t12 + C0.w * t22 + kappa * g[3][2];
+}
+
 // FL: the one kind of term that the kernel is compiled for, or 0: `flags_` at run
 // time (a step's kernels; compiled for both terms they take the same time on 4.0 M
 // cells).
 template <typename T, int OCC, int NT, class TB, int FL>
 __global__ void __launch_bounds__(NT, OCC) k_fm_fluxes(const TB tab, const Phys ph, const int flags_) {
   const int flags = FL ? FL : flags_;
-  using M = FastMath<T>;
   const int b = find_block(tab, blockIdx.x);
   if (threadIdx.x == 0) prefetch_fluxes<T, false, true>(tab.b[b], blockIdx.x, NT);
   grid_dep_wait();
@@ -178,45 +219,14 @@ __global__ void __launch_bounds__(NT, OCC) k_fm_fluxes(const TB tab, const Phys 
   const Cell6<T> Km = load_cell<T>(P, km), Kp = load_cell<T>(P, kp);
 
   if (vis) {
-    // viscous flux components at c (rhs/viscous.py:36-105)
-    // the central differences' factor 1/2 is carried by mu and kappa (exact)
-    const T d[4][3] = {{Ip.u - Im.u, Jp.u - Jm.u, Kp.u - Km.u},
-                       {Ip.v - Im.v, Jp.v - Jm.v, Kp.v - Km.v},
-                       {Ip.w - Im.w, Jp.w - Jm.w, Kp.w - Km.w},
-                       {Ip.t - Im.t, Jp.t - Jm.t, Kp.t - Km.t}};
-    T kk[9];
+    T kk[9], g[9];
     metric_row<T>(B, N, 0, c, kk);
     metric_row<T>(B, N, 1, c, kk + 3);
     metric_row<T>(B, N, 2, c, kk + 6);
-    T g[4][3];
-#pragma unroll
-    for (int s = 0; s < 4; ++s)
-#pragma unroll
-      for (int m = 0; m < 3; ++m) g[s][m] = d[s][0] * kk[m] + d[s][1] * kk[3 + m] + d[s][2] * kk[6 + m];
-    T mu = (T)B.mu0;
-    if (ph.visc_law == 0) {  // Sutherland (physics/eos.py:24-25)
-      const T r = C0.t * (T)ph.inv_T0;
-      mu = (T)B.mu0 * (r * M::sqrt_pos(r)) * (T)ph.sfac * M::rcp(C0.t + (T)ph.Ts);
-    }
-    const T muh = T(0.5) * mu, kappa = (T)ph.kap_fac * muh;
-    const T third = (T)(1.0 / 3.0);
-    const T div_u = g[0][0] + g[1][1] + g[2][2];
-    const T t00 = mu * (g[0][0] - div_u * third);
-    const T t01 = muh * (g[0][1] + g[1][0]);
-    const T t02 = muh * (g[0][2] + g[2][0]);
-    const T t11 = mu * (g[1][1] - div_u * third);
-    const T t12 = muh * (g[1][2] + g[2][1]);
-    const T t22 = mu * (g[2][2] - div_u * third);
+    visc_components(B, C0, Im, Ip, Jm, Jp, Km, Kp, kk, ph, g);
     T* __restrict__ G = (T*)B.G;
-    G[c] = t00;
-    G[N + c] = t01;
-    G[2 * N + c] = t02;
-    G[3 * N + c] = t11;
-    G[4 * N + c] = t12;
-    G[5 * N + c] = t22;
-    G[6 * N + c] = C0.u * t00 + C0.v * t01 + C0.w * t02 + kappa * g[3][0];
-    G[7 * N + c] = C0.u * t01 + C0.v * t11 + C0.w * t12 + kappa * g[3][1];
-    G[8 * N + c] = C0.u * t02 + C0.v * t12 + C0.w * t22 + kappa * g[3][2];
+#pragma unroll
+    for (int m = 0; m < 9; ++m) G[m * N + c] = g[m];
   }
   if (inv) {
     // the three faces c | c+e_a with face index c_a - 1 in [0, n_a - 4]
@@ -262,7 +272,6 @@ __device__ __forceinline__ void face_value(const SplitBlock& B, int32_t N, int a
 
 template <typename T>
 __device__ __forceinline__ void visc_value(const SplitBlock& B, const Cell& x, const Phys& ph, T G[9]) {
-  using M = FastMath<T>;
   const int32_t N = (int32_t)x.N, c = (int32_t)x.c;
   const int32_t si = x.nj * x.nk, sj = x.nk;
   const T* __restrict__ P = (const T*)B.prim;
@@ -276,43 +285,11 @@ __device__ __forceinline__ void visc_value(const SplitBlock& B, const Cell& x, c
   const Cell6<T> Im = load_cell<T>(P, im), Ip = load_cell<T>(P, ip);
   const Cell6<T> Jm = load_cell<T>(P, jm), Jp = load_cell<T>(P, jp);
   const Cell6<T> Km = load_cell<T>(P, km), Kp = load_cell<T>(P, kp);
-  // the central differences' factor 1/2 is carried by mu and kappa (exact)
-  const T d[4][3] = {{Ip.u - Im.u, Jp.u - Jm.u, Kp.u - Km.u},
-                     {Ip.v - Im.v, Jp.v - Jm.v, Kp.v - Km.v},
-                     {Ip.w - Im.w, Jp.w - Jm.w, Kp.w - Km.w},
-                     {Ip.t - Im.t, Jp.t - Jm.t, Kp.t - Km.t}};
   T kk[9];
   metric_row<T>(B, N, 0, c, kk);
   metric_row<T>(B, N, 1, c, kk + 3);
   metric_row<T>(B, N, 2, c, kk + 6);
-  T g[4][3];
-#pragma unroll
-  for (int s = 0; s < 4; ++s)
-#pragma unroll
-    for (int m = 0; m < 3; ++m) g[s][m] = d[s][0] * kk[m] + d[s][1] * kk[3 + m] + d[s][2] * kk[6 + m];
-  T mu = (T)B.mu0;
-  if (ph.visc_law == 0) {  // Sutherland (physics/eos.py:24-25)
-    const T r = C0.t * (T)ph.inv_T0;
-    mu = (T)B.mu0 * (r * M::sqrt_pos(r)) * (T)ph.sfac * M::rcp(C0.t + (T)ph.Ts);
-  }
-  const T muh = T(0.5) * mu, kappa = (T)ph.kap_fac * muh;
-  const T third = (T)(1.0 / 3.0);
-  const T div_u = g[0][0] + g[1][1] + g[2][2];
-  const T t00 = mu * (g[0][0] - div_u * third);
-  const T t01 = muh * (g[0][1] + g[1][0]);
-  const T t02 = muh * (g[0][2] + g[2][0]);
-  const T t11 = mu * (g[1][1] - div_u * third);
-  const T t12 = muh * (g[1][2] + g[2][1]);
-  const T t22 = mu * (g[2][2] - div_u * third);
-  G[0] = t00;
-  G[1] = t01;
-  G[2] = t02;
-  G[3] = t11;
-  G[4] = t12;
-  G[5] = t22;
-  G[6] = C0.u * t00 + C0.v * t01 + C0.w * t02 + kappa * g[3][0];
-  G[7] = C0.u * t01 + C0.v * t11 + C0.w * t12 + kappa * g[3][1];
-  G[8] = C0.u * t02 + C0.v * t12 + C0.w * t22 + kappa * g[3][2];
+  visc_components(B, C0, Im, Ip, Jm, Jp, Km, Kp, kk, ph, G);
 }
 
 // The k face c-1 | c (rhs/invscd.py:62-100) of the FP64 path from the

@@ -562,10 +562,12 @@ static_assert(sizeof(kSplitVariants64) / sizeof(kSplitVariants64[0]) == FJ_NUM_S
 // Shapes of the right-hand sides with one kind of term only.  Kernels compiled for
 // both and branching on the flags kept the registers of both (128 and 96 a thread):
 // too few warps to cover the viscous terms' loads.  Compiled for their own terms
-// they need 118 / 92 (inviscid) and 80 / 64 (viscous): on 127 x 66 x 51 cells the
-// inviscid call went from 58.0 to 57.1 us, the viscous one from 49.4 to 44.6.
-// (Viscous at {5, 8}, {8, 6}, {6, 10} and inviscid at {5, 6}, {5, 8}, {6, 6}:
-// 0.5 to 4 us slower.)
+// they need 118 / 92 (inviscid) and 80 / 64 (viscous).  Viscous calls at {6, 8} and,
+// in brackets, at the steps' {4, 5}, at {5, 8}, {6, 6} and {7, 8}: 70 x 50 x 40 cells
+// 16.4 us (16.6, 16.6, 16.8, 16.9), 96^3 86.6 (90.6, 87.8, 91.2, 89.1), 160 x 97 x 61
+// 95.5 (99.8, 97.9, 100.7, 98.0).  Inviscid calls at {4, 5} and at {5, 5}, {4, 4} and
+// {4, 6}: 21.5 (22.6, 21.5, 22.0), 102.7 (104.9, 102.4, 103.1), 115.6 (118.9, 115.7,
+// 115.4).
 constexpr SplitShape kShape64Inv{4, 5}, kShape64Vis{6, 8};
 
 template <int FLUX_OCC, int ASM_OCC, int FL, class TB>
@@ -625,7 +627,10 @@ int launch_tab(const TB& tab, int ctas, int asm_ctas, const Phys& ph, int flags,
     if (!prims_ready)
       pdl_launch(k_split_prims<T, kWarps32, TB>, ctas, 32 * kWarps32, 0, st, tab, ph.gm1, ph.R, 1.0 / ph.R,
                  K_AOS ? ph.p_ref : 0.0);
-    switch (K_AOS ? variant : 0) {
+    // without records (no plan) the kernels convert FP64 metrics and want the registers
+    // of shape 1: a viscous right-hand side of 127 x 66 x 51 cells takes 30.4 us (shape
+    // 0: 30.9), of 160 x 97 x 61 64.1 (66.0), the inviscid ones the same in both
+    switch (K_AOS ? variant : 1) {
       case 1: launch_pair<T, K_AOS, 1>(tab, ctas, asm_ctas, ph, flags, stage, np, st, after_fluxes); break;
       case 2: launch_pair<T, K_AOS, 2>(tab, ctas, asm_ctas, ph, flags, stage, np, st, after_fluxes); break;
       case 3: launch_pair<T, K_AOS, 3>(tab, ctas, asm_ctas, ph, flags, stage, np, st, after_fluxes); break;

@@ -246,13 +246,11 @@ template <> struct FastMath<float> {
   }
 };
 
-// minmod(a, b) of muscl2.py:5-7 without sign products: the smaller-magnitude
-// argument when both have the same strict sign (a*b > 0), else 0.  (For
-// |a*b| below the smallest normal the product rounds to 0 and the result is
-// 0 where the reference returns the tiny min(|a|, |b|).)
+// minmod(a, b) of muscl2.py:5-7 in four min/max: the smaller-magnitude argument when
+// both have the same sign, else 0 (one of the two terms is 0).  No product of the
+// arguments, which would underflow where both are small.
 template <typename T> __device__ __forceinline__ T minmod_sel(T a, T b) {
-  const T m = fj_abs(a) < fj_abs(b) ? a : b;
-  return a * b > T(0) ? m : T(0);
+  return fj_max(fj_min(a, b), T(0)) + fj_min(fj_max(a, b), T(0));
 }
 
 // MINMOD: the limiter, else van Leer.

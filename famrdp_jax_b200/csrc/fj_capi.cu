@@ -731,8 +731,9 @@ int fj_plan_create(fj_ctx* ctx, const fj_block* blocks, int nblocks, const fj_li
       }
     }
   }
-  // blocks whose cells all have the same metrics (uniform Cartesian grids; the
-  // metrics stay unchanged while the plan lives): the split kernels then read one
+  // blocks whose cells all have the same metrics, bit for bit (filled with constants;
+  // the rounding noise of metrics differenced from coordinates is enough to differ;
+  // the metrics stay unchanged while the plan lives): the split kernels then read one
   // cell's for all
   if (split) {
     std::vector<int> differ(nblocks, 1);

@@ -24,7 +24,7 @@ struct SplitBlock {
   const double* kxyz;    // (3, 3, ni, nj, nk)
   const void* kaos;      // FP32-flux only: optional FP32 metric records, or nullptr
   int kstep;             // from one cell's metrics to the next's: kRecK (records) or 1 (FP64, in each field of
-                         // kxyz); 0 where all cells have the same (a uniform block: a Cartesian grid), which
+                         // kxyz); 0 where all cells have the same bits (a uniform block), which
                          // are then read from L1
   const double* vol;     // (ni, nj, nk)
   void* prim;            // scratch: the primitives of the stage input (records in FP32)

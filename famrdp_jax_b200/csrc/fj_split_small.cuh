@@ -10,10 +10,11 @@
 // work of the two-kernel stage at 36^3 cells), which costs less than the second
 // launch and the trip through L2.  The arithmetic is the split kernels' (the same
 // bits).
-// Steps (graph replays; FP32, FP64) against the two-kernel stages: 16^3 block 28.7
-// -> 24.3 us, 30.8 -> 26.7; 24^3 31.1 -> 26.7, 36.9 -> 32.8; 32^3 35.5 -> 32.8, 42.8
-// -> 41.7; from 36^3 on (432 cells an SM) the two kernels are faster (36.9 against
-// 41.0, 45.1 against 57.4).  Submitting a step takes 4 launches instead of 7.
+// Steps (graph replays; FP32, FP64) against the two-kernel stages, of blocks of
+// 20^3 interior cells 30.8 -> 22.6 us, 31.6 -> 26.7; 28^3 31.4 -> 28.8, 37.0 -> 34.9;
+// 32^3 32.9 -> 30.8, 41.0 -> 39.0; from 36^3 on (432 padded cells an SM) the two
+// kernels are faster (34.9 against 39.0, 43.3 against 51.5).  Submitting a step takes
+// 4 launches instead of 7.
 #pragma once
 
 namespace small {

@@ -562,7 +562,7 @@ static_assert(sizeof(kSplitVariants64) / sizeof(kSplitVariants64[0]) == FJ_NUM_S
 // Shapes of the right-hand sides with one kind of term only.  Kernels compiled for
 // both and branching on the flags kept the registers of both (128 and 96 a thread):
 // too few warps to cover the viscous terms' loads.  Compiled for their own terms
-// they need 118 / 92 (inviscid) and 80 / 64 (viscous).  Viscous calls at {6, 8} and,
+// the viscous ones need 80 / 64 (inviscid 128 / 96, at the caps).  Viscous calls at {6, 8} and,
 // in brackets, at the steps' {4, 5}, at {5, 8}, {6, 6} and {7, 8}: 70 x 50 x 40 cells
 // 16.4 us (16.6, 16.6, 16.8, 16.9), 96^3 86.6 (90.6, 87.8, 91.2, 89.1), 160 x 97 x 61
 // 95.5 (99.8, 97.9, 100.7, 98.0).  Inviscid calls at {4, 5} and at {5, 5}, {4, 4} and
